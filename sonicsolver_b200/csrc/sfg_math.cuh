@@ -424,80 +424,123 @@ template <> struct Teno<float> {
     }
 };
 
-// FP64 left / right core pairs sharing one division: with x/a and y/b needed,
-// r = 1/(a b) gives x b r and y a r.  The WENO5 denominators lie in
-// [6e-25, ~1e33] and the TENO5 products e0 e1 e2 in [1e-120, ~1e24] for any
-// state the reference accepts, so a b stays inside FP64 range.
-__device__ __forceinline__ void weno5_pair64(const double* l, const double* r, double& wl, double& wr,
-                                             unsigned& flags) {
-    double num[2], den[2];
-    const double* v2[2] = {l, r};
+// ---------------------------------------------------------------------------
+// FP64 WENO5 / TENO5 on a face's six points in differences.  With the
+// characteristic first differences W_i = c_{i+1} - c_i (i = 0..4) and second
+// differences t_i = W_{i+1} - W_i (centred on the points 1..4), and the
+// reconstructions taken relative to the midpoint (c_2 + c_3) / 2:
+//   4 b_k = 13/3 t^2 + r^2   left:  (t0, t0 + 2 W1), (t1, W1 + W2), (t2, t2 - 2 W2)
+//                            right: (t3, t3 - 2 W3), (t2, W2 + W3), (t1, t1 + 2 W2)
+//   6 (p_k - mid)            left:  2 t0 - 3 t1, -t1, -t2;   right: 2 t3 - 3 t2, -t2, -t1
+// so both sides share the differences and the t^2 terms, no projected point
+// is needed (only the five projected differences), and the face states are
+// q-bar + R (deltas).  FP64 pipe operations of a field, both sides: WENO5
+// about 65 (about 115 from the points), TENO5 on smooth stencils 32 (84).
+// The FP64 kernels are bound by that pipe and by issue (FP64 tile, 1024^2,
+// before: pipe 65 % busy on TENO5 with 1430 instructions a face, 79 % on
+// WENO5 with 1210).  Whole runs, before -> after: TENO5 vortex 1024^2 0.537 ->
+// 0.432 ms a step, WENO5 Taylor-Green 256^3 sweeps 15.2 -> 14.0 ms a step,
+// WENO5 + Roe tube 257 x 193 1.10x, WENO5 Sod 1000 (one cluster) 1.12x.
+// Every rounding is fixed (fma or an _rn intrinsic), so the same inputs round
+// alike in every kernel.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// Second differences and eps + 4 b_k of both sides.
+__device__ __forceinline__ void indicators64(const double (&W)[5], double eps, double (&t)[4], double (&el)[3],
+                                             double (&er)[3]) {
+    double b[4];
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        const double* v = v2[side];
-        const double p0 = 2.0 * v[0] - 7.0 * v[1] + 11.0 * v[2];
-        const double p1 = -v[1] + 5.0 * v[2] + 2.0 * v[3];
-        const double p2 = 2.0 * v[2] + 5.0 * v[3] - v[4];
-        const double t0 = v[0] - 2.0 * v[1] + v[2], r0 = v[0] - 4.0 * v[1] + 3.0 * v[2];
-        const double t1 = v[1] - 2.0 * v[2] + v[3], r1 = v[1] - v[3];
-        const double t2 = v[2] - 2.0 * v[3] + v[4], r2 = 3.0 * v[2] - 4.0 * v[3] + v[4];
-        const double c13 = 13.0 / 12.0;
-        const double b0 = c13 * (t0 * t0) + 0.25 * (r0 * r0);
-        const double b1 = c13 * (t1 * t1) + 0.25 * (r1 * r1);
-        const double b2 = c13 * (t2 * t2) + 0.25 * (r2 * r2);
-        const double s0 = (1e-6 + b0) * (1e-6 + b0), s1 = (1e-6 + b1) * (1e-6 + b1), s2 = (1e-6 + b2) * (1e-6 + b2);
-        const double w0 = 0.1 * (s1 * s2), w1 = 0.6 * (s0 * s2), w2 = 0.3 * (s0 * s1);
-        den[side] = 6.0 * (w0 + w1 + w2);
-        num[side] = w0 * p0 + w1 * p1 + w2 * p2;
+    for (int i = 0; i < 4; ++i) {
+        t[i] = add_rn(W[i + 1], -W[i]);
+        b[i] = fma(mul_rn(13.0 / 3.0, t[i]), t[i], eps);
     }
-    const double inv = 1.0 / (den[0] * den[1]);
-    if (!(inv > 0.0) || !isfinite(inv)) flags |= FLAG_NONFINITE;
-    wl = num[0] * den[1] * inv;
-    wr = num[1] * den[0] * inv;
+    const double l0 = fma(2.0, W[1], t[0]), l1 = add_rn(W[1], W[2]), l2 = fma(-2.0, W[2], t[2]);
+    const double r0 = fma(-2.0, W[3], t[3]), r1 = add_rn(W[2], W[3]), r2 = fma(2.0, W[2], t[1]);
+    el[0] = fma(l0, l0, b[0]);
+    el[1] = fma(l1, l1, b[1]);
+    el[2] = fma(l2, l2, b[2]);
+    er[0] = fma(r0, r0, b[3]);
+    er[1] = fma(r1, r1, b[2]);
+    er[2] = fma(r2, r2, b[1]);
 }
 
-__device__ __forceinline__ void teno5_pair64(const double* l, const double* r, double& wl, double& wr,
-                                             unsigned& flags, unsigned& cut) {
-    double b[2][3], p[2][3], e[2][3], tau[2], prod[2];
-    const double* v2[2] = {l, r};
+// WENO5-JS: the folding of weno5_core on both sides, one division for the
+// two: with x/a and y/b needed, r = 1/(a b) gives x b r and y a r.  The
+// denominators lie in [1e-19, ~1e37] for any state the reference accepts, so
+// a b stays inside FP64 range.
+__device__ __forceinline__ void weno5_pair64(const double (&W)[5], double& dl, double& dr, unsigned& flags) {
+    double t[4], el[3], er[3];
+    indicators64(W, 4e-6, t, el, er);
+    const double u1 = mul_rn(3.0, t[1]), u2 = mul_rn(3.0, t[2]);
+    const double v1 = mul_rn(6.0, t[1]), v2 = mul_rn(6.0, t[2]);
+    double num[2], den[2];
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-        const double* v = v2[side];
-        teno_polys<double>(v, p[side][0], p[side][1], p[side][2]);
-        teno_betas<double>(v, b[side][0], b[side][1], b[side][2]);
-        tau[side] = fabs(b[side][0] - b[side][2]);
-        for (int k = 0; k < 3; ++k) e[side][k] = b[side][k] + 1e-40;
-        prod[side] = e[side][0] * (e[side][1] * e[side][2]);
+        const double* e = side ? er : el;
+        const double s0 = mul_rn(e[0], e[0]), s1 = mul_rn(e[1], e[1]), s2 = mul_rn(e[2], e[2]);
+        const double a = mul_rn(s1, s2), b = mul_rn(s0, s2), c = mul_rn(s0, s1);  // weights 1 : 6 : 3
+        den[side] = fma(3.0, c, fma(6.0, b, a));
+        const double m0 = side ? fma(2.0, t[3], -u2) : fma(2.0, t[0], -u1);
+        num[side] = side ? fma(a, m0, fma(-b, v2, mul_rn(-c, u1))) : fma(a, m0, fma(-b, v1, mul_rn(-c, u2)));
     }
-    if (warp_all(teno_smooth64(b[0], tau[0]) && teno_smooth64(b[1], tau[1]))) {
-        // every sub-stencil kept on both sides: the m = 7 weights below
-        wl = teno_sum64(0.1, 0.6, 0.3, p[0][0], p[0][1], p[0][2]) * (1.0 / 6.0);
-        wr = teno_sum64(0.1, 0.6, 0.3, p[1][0], p[1][1], p[1][2]) * (1.0 / 6.0);
-        return;
-    }
-    const double inv = 1.0 / (prod[0] * prod[1]);
-    double out[2];
+    const double inv = 1.0 / mul_rn(den[0], den[1]);
+    // positive and finite: 0 < high word < 0x7ff00000
+    if ((unsigned)(__double2hiint(inv) - 1) >= 0x7fefffffu) flags |= FLAG_NONFINITE;
+    const double r = mul_rn(inv, 1.0 / 6.0);
+    dl = mul_rn(mul_rn(num[0], den[1]), r);
+    dr = mul_rn(mul_rn(num[1], den[0]), r);
+}
+
+// The smooth-stencil test on the indicators e_k = 4 b_k + eps of one side:
+// tau <= 4 e_min and e_max < 1e30, taken on the high words (order and factor
+// 4 of positive doubles to 2^-20), which keeps it off the FP64 pipe.  The
+// proof at teno_smooth64 leaves far more room than 2^-20.
+__device__ __forceinline__ bool teno_smooth_hi(const double (&e)[3], double tau) {
+    const int h0 = __double2hiint(e[0]), h1 = __double2hiint(e[1]), h2 = __double2hiint(e[2]);
+    return hi_abs(tau) <= min(h0, min(h1, h2)) + 0x00200000 && max(h0, max(h1, h2)) < 0x46293E59;
+}
+
+__device__ __forceinline__ void teno5_pair64(const double (&W)[5], double& dl, double& dr, unsigned& flags,
+                                             unsigned& cut) {
+    double t[4], e[2][3];
+    indicators64(W, 4e-40, t, e[0], e[1]);
+    const double tau[2] = {fabs(add_rn(e[0][0], -e[0][2])), fabs(add_rn(e[1][0], -e[1][2]))};
+    // all sub-stencils: (0.1 (2 t0 - 3 t1) - 0.6 t1 - 0.3 t2) / 6
+    dl = fma(1.0 / 30.0, t[0], fma(-0.15, t[1], mul_rn(-0.05, t[2])));
+    dr = fma(1.0 / 30.0, t[3], fma(-0.15, t[2], mul_rn(-0.05, t[1])));
+    if (warp_all(teno_smooth_hi(e[0], tau[0]) && teno_smooth_hi(e[1], tau[1]))) return;
+    // tau / (e0 e1 e2) of both sides from one reciprocal; the products are >= 6e-119
+    double prod[2];
+#pragma unroll
+    for (int side = 0; side < 2; ++side) prod[side] = mul_rn(e[side][0], mul_rn(e[side][1], e[side][2]));
+    const double inv = 1.0 / mul_rn(prod[0], prod[1]);
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-        // tau / (e0 e1 e2) from the shared reciprocal
-        const double ti = tau[side] * prod[1 - side] * inv;
-        const double g0 = 1.0 + ti * (e[side][1] * e[side][2]);
-        const double g1 = 1.0 + ti * (e[side][0] * e[side][2]);
-        const double g2 = 1.0 + ti * (e[side][0] * e[side][1]);
-        const double q0 = g0 * g0 * g0, q1 = g1 * g1 * g1, q2 = g2 * g2 * g2;
-        const double G0 = q0 * q0, G1 = q1 * q1, G2 = q2 * q2;
-        const double lim = 1e-5 * (G0 + G1 + G2);
+        const double ti = mul_rn(mul_rn(tau[side], prod[1 - side]), inv);
+        const double g0 = fma(ti, mul_rn(e[side][1], e[side][2]), 1.0);
+        const double g1 = fma(ti, mul_rn(e[side][0], e[side][2]), 1.0);
+        const double g2 = fma(ti, mul_rn(e[side][0], e[side][1]), 1.0);
+        const double q0 = mul_rn(mul_rn(g0, g0), g0), q1 = mul_rn(mul_rn(g1, g1), g1),
+                     q2 = mul_rn(mul_rn(g2, g2), g2);
+        const double G0 = mul_rn(q0, q0), G1 = mul_rn(q1, q1), G2 = mul_rn(q2, q2);
+        const double lim = mul_rn(1e-5, add_rn(add_rn(G0, G1), G2));
         if (!isfinite(lim)) flags |= FLAG_NONFINITE;
         const int m = int(!(G0 < lim)) | (int(!(G1 < lim)) << 1) | (int(!(G2 < lim)) << 2);
         cut += 3 - __popc(m);
         if (m == 0) flags |= FLAG_TENO_CUTOFF;
-        const double inv6act = m == 7 ? 1.0 / 6.0 : m == 6 ? 1.0 / 5.4 : m == 5 ? 1.0 / 2.4 : m == 4 ? 1.0 / 1.8
-                             : m == 3 ? 1.0 / 4.2 : m == 2 ? 1.0 / 3.6 : m == 1 ? 1.0 / 0.6 : 0.0;
-        const double d0 = (m & 1) ? 0.1 : 0.0, d1 = (m & 2) ? 0.6 : 0.0, d2 = (m & 4) ? 0.3 : 0.0;
-        out[side] = teno_sum64(d0, d1, d2, p[side][0], p[side][1], p[side][2]) * inv6act;
+        if (m != 7) {
+            // 1 / (6 x the sum of the kept linear weights), by kept set
+            const double inv6act = m == 6 ? 1.0 / 5.4 : m == 5 ? 1.0 / 2.4 : m == 4 ? 1.0 / 1.8
+                                 : m == 3 ? 1.0 / 4.2 : m == 2 ? 1.0 / 3.6 : m == 1 ? 1.0 / 0.6 : 0.0;
+            const double d0 = (m & 1) ? 0.1 : 0.0, d1 = (m & 2) ? 0.6 : 0.0, d2 = (m & 4) ? 0.3 : 0.0;
+            const double ta = side ? t[3] : t[0], tb = side ? t[2] : t[1], tc = side ? t[1] : t[2];
+            const double m0 = fma(2.0, ta, mul_rn(-3.0, tb));
+            const double x = mul_rn(fma(d0, m0, fma(-d1, tb, mul_rn(-d2, tc))), inv6act);
+            if (side) dr = x;
+            else dl = x;
+        }
     }
-    wl = out[0];
-    wr = out[1];
 }
 
 template <int SCHEME, typename T>
@@ -521,22 +564,23 @@ __device__ __forceinline__ void rusanov(const T qL[5], const T qR[5], T gamma, T
     const T iL = rcp<T>(qL[0]), iR = rcp<T>(qR[0]);
     const T uL[3] = {qL[1] * iL, qL[2] * iL, qL[3] * iL};
     const T uR[3] = {qR[1] * iR, qR[2] * iR, qR[3] * iR};
-    const T kL = T(0.5) * qL[0] * (uL[0] * uL[0] + uL[1] * uL[1] + uL[2] * uL[2]);
-    const T kR = T(0.5) * qR[0] * (uR[0] * uR[0] + uR[1] * uR[1] + uR[2] * uR[2]);
-    const T pL = (gamma - T(1)) * (qL[4] - kL);
-    const T pR = (gamma - T(1)) * (qR[4] - kR);
+    const T kL = fma(qL[1], uL[0], fma(qL[2], uL[1], mul_rn(qL[3], uL[2])));  // 2 x kinetic energy
+    const T kR = fma(qR[1], uR[0], fma(qR[2], uR[1], mul_rn(qR[3], uR[2])));
+    const T pL = (gamma - T(1)) * fma(T(-0.5), kL, qL[4]);
+    const T pR = (gamma - T(1)) * fma(T(-0.5), kR, qR[4]);
     if (!(qL[0] > T(0)) || !(qR[0] > T(0))) flags |= FLAG_DENSITY;
     if (!(pL > T(0)) || !(pR > T(0))) flags |= FLAG_PRESSURE;
     const T cL = sqrt_<T>(gamma * pL * iL), cR = sqrt_<T>(gamma * pR * iR);
     const T unL = uL[N - 1], unR = uR[N - 1];
-    const T lam = fmax(fabs(unL) + cL, fabs(unR) + cR);
-    const T hl = T(0.5) * lam;
+    const T lam = fmax(add_rn(fabs(unL), cL), add_rn(fabs(unR), cR));
+    // F = (f_L + f_R) / 2 - lam / 2 (q_R - q_L), the halves on u_n and lam
+    const T hl = mul_rn(T(0.5), lam), hL = mul_rn(T(0.5), unL), hR = mul_rn(T(0.5), unR);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        T fl = qL[v] * unL, fr = qR[v] * unR;
-        if (v == N) { fl += pL; fr += pR; }
-        if (v == 4) { fl += pL * unL; fr += pR * unR; }
-        F[v] = T(0.5) * (fl + fr) - hl * (qR[v] - qL[v]);
+        T f = fma(qL[v], hL, mul_rn(qR[v], hR));
+        if (v == N) f = fma(T(0.5), add_rn(pL, pR), f);
+        if (v == 4) f = fma(pL, hL, fma(pR, hR, f));
+        F[v] = fma(-hl, add_rn(qR[v], -qL[v]), f);
     }
 }
 
@@ -709,10 +753,93 @@ __device__ __forceinline__ void laxw(const T qL[5], const T qR[5], T gamma, T la
     euler_flux<AX, T>(qh, gamma, F, flags);
 }
 
+// Characteristic projection of a state difference and the back-projection of
+// characteristic deltas, FP64, every rounding fixed.  The tangential variables
+// take the raw Cartesian components (a sign common to a projection and its
+// back-projection cancels).
+template <int AX>
+__device__ __forceinline__ void project64(const Eigen<double>& e, const double (&q)[5], double (&w)[5]) {
+    using B = AxisBasis<AX>;
+    const double vel[3] = {e.u, e.v, e.w};
+    const double nA = fma(-e.u, q[1], fma(-e.v, q[2], fma(-e.w, q[3], fma(e.h, q[0], q[4]))));  // -A
+    const double nB = fma(-vel[B::N - 1], q[0], q[B::N]);                                       // -B
+    const double y = mul_rn(e.b2, nA);
+    w[0] = fma(-e.b1, nA, q[0]);
+    w[1] = fma(-vel[B::L - 1], q[0], q[B::L]);
+    w[2] = fma(-vel[B::M - 1], q[0], q[B::M]);
+    w[3] = fma(-e.x1, nB, y);
+    w[4] = fma(e.x1, nB, y);
+}
+
+// q = qbar + R w.
+template <int AX>
+__device__ __forceinline__ void back_project64(const Eigen<double>& e, const double (&qbar)[5], const double (&w)[5],
+                                               double (&q)[5]) {
+    using B = AxisBasis<AX>;
+    const double vel[3] = {e.u, e.v, e.w};
+    const double P = add_rn(w[3], w[4]);
+    const double S = add_rn(w[0], P);
+    const double cD = mul_rn(e.c, add_rn(w[4], -w[3]));
+    q[0] = add_rn(qbar[0], S);
+    q[B::N] = add_rn(qbar[B::N], fma(vel[B::N - 1], S, cD));
+    q[B::L] = add_rn(qbar[B::L], fma(vel[B::L - 1], S, w[1]));
+    q[B::M] = add_rn(qbar[B::M], fma(vel[B::M - 1], S, w[2]));
+    q[4] = add_rn(qbar[4], fma(e.h, w[0], fma(vel[B::L - 1], w[1], fma(vel[B::M - 1], w[2],
+                           fma(e.H, P, mul_rn(vel[B::N - 1], cD))))));
+}
+
+template <int AX, int FLUX, typename T>
+__device__ __forceinline__ void flux_of(const T (&ql)[5], const T (&qr)[5], T gamma, T lam, T F[5], unsigned& flags) {
+    if constexpr (FLUX == RUSANOV) rusanov<AX, T>(ql, qr, gamma, F, flags);
+    else if constexpr (FLUX == ROE) roe<AX, T>(ql, qr, gamma, F, flags);
+    else if constexpr (FLUX == STEGER) steger<AX, T>(ql, qr, gamma, F, flags);
+    else if constexpr (FLUX == LAXF) laxf<AX, T>(ql, qr, gamma, F, flags);
+    else laxw<AX, T>(ql, qr, gamma, lam, F, flags);
+}
+
+// FP64 WENO5 / TENO5 face: the five state differences are projected, not the
+// six points, and the face states are q-bar + R (deltas).
+template <int AX, int SCHEME, int FLUX>
+__device__ __forceinline__ void face_flux64(const double (&st)[6][5], double gamma, double F[5], unsigned& flags,
+                                            unsigned& cut, double lam) {
+    double qbar[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) qbar[v] = 0.5 * (st[2][v] + st[3][v]);
+    Eigen<double> e;
+    if (!eigen_at<AX, double>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
+    double W[5][5];
+#pragma unroll
+    for (int s = 0; s < 5; ++s) {
+        double d[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) d[v] = add_rn(st[s + 1][v], -st[s][v]);
+        project64<AX>(e, d, W[s]);
+    }
+    double wl[5], wr[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        const double w[5] = {W[0][v], W[1][v], W[2][v], W[3][v], W[4][v]};
+        if constexpr (SCHEME == WENO5) weno5_pair64(w, wl[v], wr[v], flags);
+        else teno5_pair64(w, wl[v], wr[v], flags, cut);
+    }
+    double ql[5], qr[5];
+    back_project64<AX>(e, qbar, wl, ql);
+    back_project64<AX>(e, qbar, wr, qr);
+    flux_of<AX, FLUX, double>(ql, qr, gamma, lam, F, flags);
+    int top = 0;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) top = max(top, hi_abs(F[v]));
+    if (top >= 0x7ff00000) flags |= FLAG_NONFINITE;
+}
+
 // `lam` = dt / h along AX, used by the Lax-Wendroff flux only.
 template <int AX, int SCHEME, int FLUX, typename T>
 __device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>::NST][5], T gamma, T F[5],
                                           unsigned& flags, unsigned& cut, T lam = T(0)) {
+    if constexpr (sizeof(T) == sizeof(double) && (SCHEME == WENO5 || SCHEME == TENO5)) {
+        face_flux64<AX, SCHEME, FLUX>(st, gamma, F, flags, cut, lam);
+        return;
+    }
     constexpr int NST = SchemeInfo<SCHEME>::NST;
     constexpr int W = SchemeInfo<SCHEME>::W;
     constexpr int CL = NST / 2 - 1;
@@ -742,14 +869,8 @@ __device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>:
             sl[s] = ch[s][v];
             sr[s] = ch[NST - 1 - s][v];
         }
-        if constexpr (sizeof(T) == sizeof(double) && SCHEME == WENO5) {
-            weno5_pair64(sl, sr, wl[v], wr[v], flags);
-        } else if constexpr (sizeof(T) == sizeof(double) && SCHEME == TENO5) {
-            teno5_pair64(sl, sr, wl[v], wr[v], flags, cut);
-        } else {
-            wl[v] = recon_core<SCHEME, T>(sl, flags, cut);
-            wr[v] = recon_core<SCHEME, T>(sr, flags, cut);
-        }
+        wl[v] = recon_core<SCHEME, T>(sl, flags, cut);
+        wr[v] = recon_core<SCHEME, T>(sr, flags, cut);
     }
     T dl[5], dr[5], ql[5], qr[5];
     from_characteristic<AX, T>(e, wl, dl);
@@ -759,11 +880,7 @@ __device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>:
         ql[v] = DEV ? T(qbar64[v] + double(dl[v])) : dl[v];
         qr[v] = DEV ? T(qbar64[v] + double(dr[v])) : dr[v];
     }
-    if constexpr (FLUX == RUSANOV) rusanov<AX, T>(ql, qr, gamma, F, flags);
-    else if constexpr (FLUX == ROE) roe<AX, T>(ql, qr, gamma, F, flags);
-    else if constexpr (FLUX == STEGER) steger<AX, T>(ql, qr, gamma, F, flags);
-    else if constexpr (FLUX == LAXF) laxf<AX, T>(ql, qr, gamma, F, flags);
-    else laxw<AX, T>(ql, qr, gamma, lam, F, flags);
+    flux_of<AX, FLUX, T>(ql, qr, gamma, lam, F, flags);
 #pragma unroll
     for (int v = 0; v < 5; ++v)
         if (!finite_(F[v])) flags |= FLAG_NONFINITE;
