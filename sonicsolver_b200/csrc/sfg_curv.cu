@@ -826,6 +826,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) curv_tile2d_f32_kernel(GridVi
     }
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 // The FP64 form of the fused 2-D tile: the state staged as is, full face
@@ -943,6 +944,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
     }
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 // Divergence and stage update of the solved nodes.
@@ -974,6 +976,7 @@ __global__ void __launch_bounds__(256) curv_stage_kernel(GridView g, StageView s
     }
     if (flags) atomicOr(sv.flags, flags);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 // ---------------------------------------------------------------------------

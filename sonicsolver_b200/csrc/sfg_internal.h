@@ -50,6 +50,7 @@ struct Clock {
     int active;               // 1 while the current step runs
     int dt_ready;             // 1: dt_bits already holds the CFL minimum of the current
                               // state (reduced by the previous step's last stage)
+    unsigned blocks_done;     // blocks of a MODE_STEP launch that have finished (0 between launches)
 };
 
 // Geometry of one grid as the kernels see it (uniform Cartesian metrics).
@@ -108,6 +109,8 @@ struct StageView {
     double base, inc;     // SSPRK3: base*q0 + inc*(q - dt R);  RK4: inc = stage weight
     int mode;             // MODE_* bits
     int require_active;   // skip when clock->active == 0
+    double* dt_log;       // MODE_STEP: where the step's dt is logged
+    long long dt_cap;
 };
 
 constexpr int MODE_READ_R = 1;     // add the residual accumulated by earlier axes
@@ -115,6 +118,9 @@ constexpr int MODE_FINAL = 2;      // last axis: finish the node
 constexpr int MODE_RESIDUAL = 4;   // final output is R = Jac * div (no stage update)
 constexpr int MODE_CFL = 8;        // last stage of a step: also reduce the CFL minimum of
                                    // the new state into clock->dt_bits (the next step's dt)
+
+constexpr int MODE_STEP = 16;      // last stage of a step: the launch's last block commits the step
+                                   // and opens the next one (step_tail)
 
 // One launch of the 1-D whole-run cluster kernel (sfg_cluster1d.cu): the
 // stage views of a step, the clock it advances and where it logs.

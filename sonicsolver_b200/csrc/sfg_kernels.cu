@@ -289,48 +289,15 @@ __global__ void __launch_bounds__(256) dt_kernel(GridView g, const double* __res
     if (fl) atomicOr(flags, fl);
 }
 
-// FlowDtCompute's min(dt, maxDeltaT, limit) with the Time::Driver end / output
-// clipping and stop test (SF_time.cpp:56-72).  One thread.  A status word
-// with bits set stops the run (the reference exits on an invalid state): the
-// failing step is the last one counted, and the rest of a graph is no-ops.
-__global__ void finalize_dt_kernel(Clock* c, const unsigned* flags) {
-    if (*flags) {
-        c->active = 0;
-        return;
-    }
-    const double eps = 2.220446049250313e-16;
-    const double remaining = c->t_end - c->t;
-    double scale = fmax(fabs(c->t), fabs(c->t_end));
-    scale = scale < 1.0 ? 1.0 : scale;
-    if (!(remaining > 64.0 * eps * scale) || c->steps >= c->max_steps) {
-        c->active = 0;  // dt keeps the last step's size
-        return;
-    }
-    double limit = remaining;
-    if (c->write_interval > 0.0 && c->next_out - c->t < limit) limit = c->next_out - c->t;
-    if (c->limit < limit) limit = c->limit;
-    double dt = __longlong_as_double((long long)c->dt_bits);
-    if (c->max_dt < dt) dt = c->max_dt;
-    if (limit < dt) dt = limit;
-    c->dt = dt;
-    c->active = 1;
-    c->dt_bits = 0x7FEFFFFFFFFFFFFFull;  // consumed: re-armed for the next minimum
-    c->dt_ready = 0;
-}
+// Opens the first step of a run (clock_open_step).  One thread.
+__global__ void finalize_dt_kernel(Clock* c, const unsigned* flags) { clock_open_step(c, *flags); }
 
-// TimeCommit: t += dt, ++step, output-time bookkeeping.  `cfl_next`: the
-// step's last stage reduced the CFL minimum of the new state into dt_bits.
-__global__ void commit_kernel(Clock* c, double* dt_log, long long dt_cap, int cfl_next) {
-    if (c->active) {
-        if (dt_log && c->steps - c->log_base < dt_cap && c->steps >= c->log_base) dt_log[c->steps - c->log_base] = c->dt;
-        c->t += c->dt;
-        c->steps += 1;
-        double sc = fabs(c->t);
-        sc = sc < 1.0 ? 1.0 : sc;
-        if (c->write_interval > 0.0 && c->t >= c->next_out - 1.0e-11 * sc) c->next_out += c->write_interval;
-    }
-    c->dt_ready = c->active && cfl_next ? 1 : 0;
-    c->limit = __longlong_as_double(0x7FF0000000000000ll);
+// Commits a step; `open_next`: also opens the next one (the step's launches
+// that have no MODE_STEP tail of their own).  One thread.
+__global__ void commit_kernel(Clock* c, const unsigned* flags, double* dt_log, long long dt_cap, int cfl_next,
+                              int open_next) {
+    clock_commit_step(c, dt_log, dt_cap, cfl_next);
+    if (open_next) clock_open_step(c, *flags);
 }
 
 __global__ void set_dt_kernel(Clock* c, double dt) {
@@ -506,8 +473,9 @@ cudaError_t launch_finalize_dt(Clock* c, const unsigned* flags, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_commit(Clock* c, double* dt_log, long long dt_cap, int cfl_next, cudaStream_t st) {
-    commit_kernel<<<1, 1, 0, st>>>(c, dt_log, dt_cap, cfl_next);
+cudaError_t launch_commit(Clock* c, const unsigned* flags, double* dt_log, long long dt_cap, int cfl_next,
+                          int open_next, cudaStream_t st) {
+    commit_kernel<<<1, 1, 0, st>>>(c, flags, dt_log, dt_cap, cfl_next, open_next);
     return cudaGetLastError();
 }
 

@@ -11,6 +11,7 @@
 #include "../../include/sonicsolver_b200.h"
 #include "sfg_internal.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -26,7 +27,8 @@ cudaError_t launch_sweep(int scheme, int flux, int prec64, int axis, const GridV
 cudaError_t launch_dt(const GridView& g, const double* q, Clock* clock, unsigned* flags, int skip_if_ready,
                       cudaStream_t st);
 cudaError_t launch_finalize_dt(Clock* c, const unsigned* flags, cudaStream_t st);
-cudaError_t launch_commit(Clock* c, double* dt_log, long long dt_cap, int cfl_next, cudaStream_t st);
+cudaError_t launch_commit(Clock* c, const unsigned* flags, double* dt_log, long long dt_cap, int cfl_next,
+                          int open_next, cudaStream_t st);
 cudaError_t launch_set_dt(Clock* c, double dt, cudaStream_t st);
 cudaError_t launch_reset_min(Clock* c, cudaStream_t st);
 cudaError_t launch_stage_from_residual(const GridView& g, const StageView& sv, cudaStream_t st);
@@ -154,12 +156,24 @@ struct sfg_solver_s {
     // graph of `graph_steps` steps for sfg_advance
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
+    // graph of a run's last `rest_steps` steps (fewer than a graph holds), once
+    // a second run has left the same number
+    cudaGraphExec_t rest_graph = nullptr;
+    int rest_steps = 0;
     double* dt_log = nullptr;
     long long dt_log_cap = 0;
     Clock* host_clock = nullptr;  // pinned mirror
 };
 
 namespace {
+
+// The captured steps hold the launches' arguments: dropped when those change.
+void drop_graphs(sfg_solver_s* s) {
+    for (cudaGraphExec_t* g : {&s->graph, &s->rest_graph}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+}
 
 int validate(const sfg_grid_desc* g, const sfg_numerics_desc* n, const RecipeInfo** recipe) {
     if (!g || !n) return fail(SFG_ERR_ARG, "null descriptor");
@@ -425,11 +439,15 @@ StageView stage_view(sfg_solver_s* s, int stage, bool residual_only, bool requir
 
 // All axis sweeps of one stage (or of the residual alone).
 // `cfl`: the launch that finishes the nodes also reduces the CFL minimum of
-// the new state (the last stage of a step).
-int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_active, bool cfl = false) {
+// the new state (the last stage of a step).  `tail`: it also ends the step
+// (MODE_STEP; has_tail() grids only).
+int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_active, bool cfl = false,
+                  bool tail = false) {
     StageView sv = stage_view(s, stage, residual_only, require_active);
+    sv.dt_log = s->dt_log;
+    sv.dt_cap = s->dt_log_cap;
     const int dim = s->grid.dim;
-    const int cfl_bit_all = cfl && !residual_only ? MODE_CFL : 0;
+    const int cfl_bit_all = (cfl && !residual_only ? MODE_CFL : 0) | (tail ? MODE_STEP : 0);
     if (s->has_laws) {
         // prepareBoundaryState before the RHS: the laws on the stage's input;
         // the previous application's values sit in the previous stage's input
@@ -444,7 +462,7 @@ int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_a
                                    s->variant > 0, s->gv, sv, s->face_flux, s->stream));
         return SFG_OK;
     }
-    const int cfl_bit = cfl && !residual_only ? MODE_CFL : 0;
+    const int cfl_bit = cfl_bit_all;
     if (dim == 2 && s->variant > 0) {
         sv.mode = MODE_FINAL | (residual_only ? MODE_RESIDUAL : 0) | cfl_bit;
         CUDA_TRY(launch_tile2d(s->variant, s->recipe->scheme, s->recipe->flux, s->num.precision == SFG_PREC_FP64,
@@ -489,32 +507,39 @@ int enqueue_post_step(sfg_solver_s* s) {
     return SFG_OK;
 }
 
-// One full step with the CFL dt computed and clipped on device.  The CFL
-// minimum of the step's result is reduced by its last stage (MODE_CFL) and
-// marked ready by the commit, so the next step's dt_kernel returns at once;
-// dt_kernel reads the state only when nothing reduced it (first step after
-// an upload, a host-driven stage or the start of sfg_advance).
-int enqueue_cfl_step(sfg_solver_s* s, bool require_active) {
+// Whether a stage of this solver is one launch that can end a step itself
+// (step_tail): every tile and curvilinear stage.  The axis sweeps cannot (a
+// warp of sweep_x leaves early), and law ends have their commit fill after
+// the last stage: those steps end in a commit launch.
+bool has_tail(const sfg_solver_s* s) { return !s->has_laws && (s->gv.curv || s->variant > 0); }
+
+// Opens the first step of a run: its CFL minimum, then dt.  Each step opens
+// the next one (the CFL minimum of its result is reduced by its last stage,
+// MODE_CFL), so this runs once per sfg_advance.
+int enqueue_open_run(sfg_solver_s* s) {
     CUDA_TRY(launch_dt(s->gv, s->qn, s->clock, s->flags, 1, s->stream));
     CUDA_TRY(launch_finalize_dt(s->clock, s->flags, s->stream));
+    return SFG_OK;
+}
+
+// One full opened step; `open_next`: its end opens the next one.
+int enqueue_cfl_step(sfg_solver_s* s, bool require_active, bool open_next) {
     // FlowStepPrepare opens the step (before its dt in the reference; the dt
     // reads solved nodes only, which the laws never write)
     if (s->has_laws)
         CUDA_TRY(launch_law_fill(s->gv, s->lv, s->qn, s->qn, s->clock, require_active ? 1 : 0, s->flags, s->stream));
     const int ns = stage_count(s->num.time_recipe);
+    const bool tail = open_next && has_tail(s);
     for (int st = 0; st < ns; ++st) {
-        int rc = enqueue_stage(s, st, false, require_active, st == ns - 1);
+        int rc = enqueue_stage(s, st, false, require_active, st == ns - 1, tail && st == ns - 1);
         if (rc) return rc;
     }
     int rc = enqueue_commit_laws(s, require_active);
     if (rc) return rc;
-    if (s->num.time_recipe == T_EULER) {
-        // guarded copy: only when the step ran (graph-safe: copy unconditionally
-        // is wrong once the run has stopped), so Euler keeps its own kernel path
-        int rc = enqueue_post_step(s);
-        if (rc) return rc;
-    }
-    CUDA_TRY(launch_commit(s->clock, s->dt_log, s->dt_log_cap, 1, s->stream));
+    rc = enqueue_post_step(s);  // Euler
+    if (rc) return rc;
+    if (!tail)
+        CUDA_TRY(launch_commit(s->clock, s->flags, s->dt_log, s->dt_log_cap, 1, open_next ? 1 : 0, s->stream));
     return SFG_OK;
 }
 
@@ -730,7 +755,7 @@ int sfg_create(const sfg_grid_desc* grid, const sfg_numerics_desc* numerics, voi
 int sfg_destroy(sfg_solver s) {
     if (!s) return SFG_OK;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->graph) cudaGraphExecDestroy(s->graph);
+    drop_graphs(s);
     for (double* p : {s->qn, s->qa, s->qb, s->r, s->k, s->staging, s->totals, s->dt_log})
         if (p) cudaFree(p);
     if (s->clock) cudaFree(s->clock);
@@ -753,10 +778,7 @@ int sfg_set_boundary_law(sfg_solver s, int axis, int end, const sfg_boundary_law
     if (const char* why = sfg::law_problem(*law)) return fail(SFG_ERR_ARG, "%s", why);
     s->laws[2 * axis + end] = *law;
     build_law_view(s);
-    if (s->graph) {  // the captured launches hold the previous laws
-        cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
-    }
+    drop_graphs(s);  // the captured launches hold the previous laws
     return upload_law_codes(s);
 }
 
@@ -821,10 +843,7 @@ int sfg_set_metrics(sfg_solver s, const double* host, int layout) {
     s->gv.node_jac = s->node_metrics;
     s->gv.node_metric = s->node_metrics + s->gv.vs;
     for (int a = 0; a < 3; ++a) s->gv.geom[a] = geom[a];
-    if (s->graph) {  // the captured launches hold the previous grid view
-        cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
-    }
+    drop_graphs(s);  // the captured launches hold the previous grid view
     return SFG_OK;
 }
 
@@ -1005,7 +1024,7 @@ int sfg_stage(sfg_solver s, int stage, double dt) {
         if (rc) return rc;
         rc = enqueue_post_step(s);
         if (rc) return rc;
-        CUDA_TRY(launch_commit(s->clock, nullptr, 0, 0, s->stream));
+        CUDA_TRY(launch_commit(s->clock, s->flags, nullptr, 0, 0, 0, s->stream));
         s->next_stage = 0;
     } else {
         s->next_stage = stage + 1;
@@ -1044,49 +1063,93 @@ int sfg_step(sfg_solver s, double dt, double limit) {
     s->host_clock->next_out = kInf;
     rc = push_clock(s);
     if (rc) return rc;
-    rc = enqueue_cfl_step(s, false);
+    rc = enqueue_open_run(s);
+    if (rc) return rc;
+    rc = enqueue_cfl_step(s, false, false);
     if (rc) return rc;
     return sync_and_check(s);
 }
 
-// sfg_advance on the CUDA-graph path: graphs of `graph_steps` CFL steps,
-// relaunched until the clock stops.  `ms`: device time of the launches.
+// Captures `n` steps as one CUDA graph (kept until the solver's launches
+// change).
+static int capture_steps(sfg_solver_s* s, int n, cudaGraphExec_t* out) {
+    cudaGraph_t g;
+    CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    int crc = SFG_OK;
+    for (int i = 0; i < n && !crc; ++i) crc = enqueue_cfl_step(s, true, true);
+    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    if (crc) return crc;
+    if (e != cudaSuccess) return fail(SFG_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        *out = nullptr;
+        return fail(SFG_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
+    }
+    return SFG_OK;
+}
+
+// Enqueues `n` steps as a graph kept in (*graph, *steps), captured when the
+// slot holds another count.
+static int launch_steps_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* steps) {
+    if (!*graph || *steps != n) {
+        if (*graph) cudaGraphExecDestroy(*graph);
+        *graph = nullptr;
+        if (int rc = capture_steps(s, n, graph)) return rc;
+        *steps = n;
+    }
+    CUDA_TRY(cudaGraphLaunch(*graph, s->stream));
+    return SFG_OK;
+}
+
+// sfg_advance outside the cluster kernel: graphs of `graph_steps` CFL steps,
+// relaunched until the clock stops.  Fewer steps than a graph holds (max_steps,
+// or what t_end leaves at the last dt) are launched one by one, or by a graph
+// of their own once a run has left the same number before (5-7 us a step less
+// on small grids; capturing at once would cost a single run more than it
+// gains): a graph's steps past the end return at once but still cost their
+// launches, 3.9 ms of the 14 ms a three-step run of 256^3 sweeps took.
+// `ms`: device time of the launches.
 static int advance_graph(sfg_solver_s* s, int graph_steps, float* ms) {
     Clock* hc = s->host_clock;
-    if (!s->graph || s->graph_steps != graph_steps) {
-        if (s->graph) cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
-        cudaGraph_t g;
-        CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        int crc = SFG_OK;
-        for (int i = 0; i < graph_steps && !crc; ++i) crc = enqueue_cfl_step(s, true);
-        cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-        if (crc) return crc;
-        if (e != cudaSuccess) return fail(SFG_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&s->graph, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(SFG_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
-        s->graph_steps = graph_steps;
-    }
     cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
+    CUDA_TRY(cudaEventCreate(&e0));
+    CUDA_TRY(cudaEventCreate(&e1));
     cudaEventRecord(e0, s->stream);
-    for (;;) {
-        CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(hc, s->clock, sizeof(Clock), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaStreamSynchronize(s->stream));
+    int rc = enqueue_open_run(s);
+    for (bool first = true; !rc; first = false) {
+        // steps left at most; after the first launches also by time, with two
+        // to spare for a shrinking dt
+        double left = double(hc->max_steps - hc->steps);
+        if (!first && hc->dt > 0.0) left = std::min(left, std::ceil((hc->t_end - hc->t) / hc->dt) + 2.0);
+        if (left >= graph_steps) {
+            rc = launch_steps_graph(s, graph_steps, &s->graph, &s->graph_steps);
+        } else {
+            const int n = std::max(1, int(left));
+            if (s->rest_steps == n) {
+                rc = launch_steps_graph(s, n, &s->rest_graph, &s->rest_steps);
+            } else {
+                if (s->rest_graph) cudaGraphExecDestroy(s->rest_graph);
+                s->rest_graph = nullptr;
+                s->rest_steps = n;
+                for (int i = 0; i < n && !rc; ++i) rc = enqueue_cfl_step(s, true, true);
+            }
+        }
         unsigned bits = 0;
-        CUDA_TRY(cudaMemcpy(&bits, s->flags, sizeof bits, cudaMemcpyDeviceToHost));
-        if (bits) break;
-        if (!hc->active || hc->steps >= hc->max_steps) break;
+        if (!rc && (cudaMemcpyAsync(hc, s->clock, sizeof(Clock), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
+                    cudaStreamSynchronize(s->stream) != cudaSuccess ||
+                    cudaMemcpy(&bits, s->flags, sizeof bits, cudaMemcpyDeviceToHost) != cudaSuccess))
+            rc = fail(SFG_ERR_CUDA, "advance: %s", cudaGetErrorString(cudaGetLastError()));
+        if (bits || !hc->active || hc->steps >= hc->max_steps) break;
     }
-    cudaEventRecord(e1, s->stream);
-    cudaEventSynchronize(e1);
-    cudaEventElapsedTime(ms, e0, e1);
+    if (!rc) {
+        cudaEventRecord(e1, s->stream);
+        cudaEventSynchronize(e1);
+        cudaEventElapsedTime(ms, e0, e1);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    return SFG_OK;
+    return rc;
 }
 
 // sfg_advance of a small 1-D FP64 grid in the whole-run cluster kernel
@@ -1158,10 +1221,7 @@ int sfg_advance(sfg_solver s, double t_end, int64_t max_steps, double write_inte
         if (s->dt_log) cudaFree(s->dt_log);
         s->dt_log = nullptr;
         s->dt_log_cap = 0;
-        if (s->graph) {
-            cudaGraphExecDestroy(s->graph);
-            s->graph = nullptr;
-        }
+        drop_graphs(s);
         if (cudaMalloc((void**)&s->dt_log, sizeof(double) * want) != cudaSuccess)
             return fail(SFG_ERR_NOMEM, "dt log allocation failed");
         s->dt_log_cap = want;
@@ -1253,7 +1313,7 @@ int sfg_stage_with_residual(sfg_solver s, int stage, double dt, const double* ho
     if (stage == ns - 1) {
         int rc = enqueue_post_step(s);
         if (rc) return rc;
-        CUDA_TRY(launch_commit(s->clock, nullptr, 0, 0, s->stream));
+        CUDA_TRY(launch_commit(s->clock, s->flags, nullptr, 0, 0, 0, s->stream));
         s->next_stage = 0;
     } else {
         s->next_stage = stage + 1;
@@ -1296,10 +1356,7 @@ int sfg_status_word(sfg_solver s, uint32_t* bits, int clear) {
 
 int sfg_set_counting(sfg_solver s, int enable) {
     if (!s) return fail(SFG_ERR_ARG, "null solver");
-    if ((enable != 0) != s->counting && s->graph) {
-        cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
-    }
+    if ((enable != 0) != s->counting) drop_graphs(s);
     s->counting = enable != 0;
     CUDA_TRY(cudaMemsetAsync(s->counters, 0, 16, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -1405,10 +1462,7 @@ int sfg_set_kernel_variant(sfg_solver s, int variant) {
     if (variant < 0 || variant > 2) return fail(SFG_ERR_ARG, "unknown kernel variant %d", variant);
     if (variant > 1 && s->grid.dim == 3) return fail(SFG_ERR_ARG, "3-D grids have variants 0 (sweeps) and 1 (tiles)");
     // variant 2: the 22 x 22 tile (2-D), the whole-run cluster kernel (1-D)
-    if (variant != s->variant && s->graph) {
-        cudaGraphExecDestroy(s->graph);
-        s->graph = nullptr;
-    }
+    if (variant != s->variant) drop_graphs(s);
     s->variant = variant;
     return SFG_OK;
 }

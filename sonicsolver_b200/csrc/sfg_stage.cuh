@@ -191,4 +191,66 @@ __device__ __forceinline__ void flush_status(const StageView& sv, unsigned flags
     }
 }
 
+// FlowDtCompute's min(dt, maxDeltaT, limit) with the Time::Driver end / output
+// clipping and stop test (SF_time.cpp:56-72), by one thread.  A status word
+// with bits set stops the run (the reference exits on an invalid state): the
+// failing step is the last one counted, and the rest of a graph is no-ops.
+__device__ __forceinline__ void clock_open_step(Clock* c, unsigned flags) {
+    if (flags) {
+        c->active = 0;
+        return;
+    }
+    const double eps = 2.220446049250313e-16;
+    const double remaining = c->t_end - c->t;
+    double scale = fmax(fabs(c->t), fabs(c->t_end));
+    scale = scale < 1.0 ? 1.0 : scale;
+    if (!(remaining > 64.0 * eps * scale) || c->steps >= c->max_steps) {
+        c->active = 0;  // dt keeps the last step's size
+        return;
+    }
+    double limit = remaining;
+    if (c->write_interval > 0.0 && c->next_out - c->t < limit) limit = c->next_out - c->t;
+    if (c->limit < limit) limit = c->limit;
+    double dt = __longlong_as_double((long long)__ldcg(&c->dt_bits));
+    if (c->max_dt < dt) dt = c->max_dt;
+    if (limit < dt) dt = limit;
+    c->dt = dt;
+    c->active = 1;
+    c->dt_bits = 0x7FEFFFFFFFFFFFFFull;  // consumed: re-armed for the next minimum
+    c->dt_ready = 0;
+}
+
+// TimeCommit: t += dt, ++step, output-time bookkeeping.  `cfl_next`: the
+// step's last stage reduced the CFL minimum of the new state into dt_bits.
+__device__ __forceinline__ void clock_commit_step(Clock* c, double* dt_log, long long dt_cap, int cfl_next) {
+    if (c->active) {
+        if (dt_log && c->steps - c->log_base < dt_cap && c->steps >= c->log_base) dt_log[c->steps - c->log_base] = c->dt;
+        c->t += c->dt;
+        c->steps += 1;
+        double sc = fabs(c->t);
+        sc = sc < 1.0 ? 1.0 : sc;
+        if (c->write_interval > 0.0 && c->t >= c->next_out - 1.0e-11 * sc) c->next_out += c->write_interval;
+    }
+    c->dt_ready = c->active && cfl_next ? 1 : 0;
+    c->limit = __longlong_as_double(0x7FF0000000000000ll);
+}
+
+// The end of a step's last launch (MODE_STEP; every block of the launch calls
+// it, every thread of a block, after its status and CFL flushes): the block
+// that finishes last commits the step and opens the next.  No wait anywhere:
+// a block counts itself in and leaves.  This takes three one-thread launches
+// (dt, finalize, commit: 2-4 us each inside a graph) out of every step.
+__device__ __forceinline__ void step_tail(const StageView& sv) {
+    __syncthreads();  // the block's atomics are issued
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&sv.clock->blocks_done, 1u) == gridDim.x - 1) {
+            __threadfence();  // every block's flags and CFL minimum are visible
+            sv.clock->blocks_done = 0;
+            clock_commit_step(sv.clock, sv.dt_log, sv.dt_cap, 1);
+            clock_open_step(sv.clock, __ldcg(sv.flags));
+        }
+    }
+}
+
 }  // namespace sfg

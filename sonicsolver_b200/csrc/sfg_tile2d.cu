@@ -15,6 +15,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) tile2d_kernel(GridView g, Sta
     tile2d_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smem, flags, cut, cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 template <int SCHEME, int FLUX, int TX, int TY>
@@ -28,6 +29,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) tile2d_f32_kernel(GridView g,
     tile2d_f32_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smemf, flags, cut, cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 template <int SCHEME, int FLUX, typename T, int TX, int TY>
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(TILE_THREADS) tile1d_kernel(GridView g, StageV
                                  cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 template <int SCHEME, int FLUX, typename T>

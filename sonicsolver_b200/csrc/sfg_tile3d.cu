@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
     }
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
+    if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
 template <int SCHEME, int FLUX, typename T>

@@ -50,5 +50,5 @@ def test_residual_in_differences(recipe, kind, scale, oracle):
     for variant in (0, 1, 2):
         s = case.solver()
         s.variant = variant
-        got = s.residual().reshape(q.shape)
-        assert np.abs(got - want).max() <= bound, (variant, np.abs(got - want).max() / bound)
+        err = np.abs(s.residual().reshape(q.shape) - want)[:, 1:-1, 1:-1]  # the solved nodes
+        assert err.max() <= bound, (variant, err.max() / bound)

@@ -1,0 +1,65 @@
+"""A run's steps however they are launched: graphs, a graph of the rest, single
+launches, the step's end in its last kernel or in a launch of its own.
+
+sfg_advance(max_steps = k) for k around the graph length must give the bits,
+the time and the step count of k sfg_step calls at its step sizes (which commit
+every step with a launch of their own), and must do so again when the same run
+is repeated (the second one replays a captured rest)."""
+import numpy as np
+import pytest
+
+from sonicsolver_b200 import capi, cases
+
+
+def _grid(name):
+    if name == "tiles2d":
+        return cases.isentropic_vortex(48, recipe="teno5Rusanov"), {}
+    if name == "sweeps3d":
+        return cases.taylor_green(16), {"variant": 0}
+    if name == "tiles3d":
+        return cases.taylor_green(16), {"variant": 1}
+    if name == "curved":
+        return cases.wavy_vortex(32, recipe="weno5Rusanov"), {}
+    if name == "laws":
+        c = cases.sod_1d(60)
+        c.bc_lo, c.bc_hi = (capi.BC_LAW, 0, 0), (capi.BC_LAW, 0, 0)
+        return c, {"variant": 1}
+    return cases.sod_1d(90), {"variant": 1}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("time_recipe", ["SSPRK3", "forwardEuler", "classicalRK4"])
+@pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_FP32_FLUX])
+@pytest.mark.parametrize("name", ["tiles1d", "tiles2d", "sweeps3d", "tiles3d", "curved", "laws"])
+def test_advance_equals_single_steps(name, precision, time_recipe):
+    case, kw = _grid(name)
+    G = 4
+
+    def solver():
+        s = case.solver(precision=precision, time_recipe=time_recipe, cfl=0.2)
+        if "variant" in kw:
+            s.variant = kw["variant"]
+        return s
+
+    a, b = solver(), solver()
+    q0 = np.ascontiguousarray(case.q)
+    for k in (1, 3, 3, 3, G, G + 1, G + 1, 2 * G + 3):
+        a.upload(q0)
+        st, dts = a.advance(1e30, max_steps=k, graph_steps=G, dt_capacity=16)
+        assert st.steps == k and len(dts) == k and st.last_dt == dts[-1]
+        b.upload(q0)
+        for dt in dts:
+            b.step(float(dt))
+        assert a.time() == b.time()
+        np.testing.assert_array_equal(a.download(), b.download())
+    # a run that ends on time: the same end however the graph's rest is launched
+    t_end = 2.5 * dts[0] + dts[1]
+    ends = []
+    for g in (1, 3, 64):
+        a.upload(q0)
+        st, d = a.advance(t_end, graph_steps=g, dt_capacity=16)
+        assert abs(st.time - t_end) <= 1e-14 * max(1.0, t_end)
+        ends.append((st.steps, a.download()))
+    for n, q in ends[1:]:
+        assert n == ends[0][0]
+        np.testing.assert_array_equal(q, ends[0][1])
