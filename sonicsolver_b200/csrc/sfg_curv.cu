@@ -192,33 +192,14 @@ __device__ __forceinline__ void recon_field(const CharBasisT<T>& e, const T (&st
         ch[s] = acc;
     }
     T wl, wr;
-    if constexpr (std::is_same<T, float>::value && (SCHEME == WENO5 || SCHEME == TENO5)) {
-        // FP32 WENO5 / TENO5: the left- and right-biased stencils as the two
-        // lanes of one paired core (the Cartesian kernels' cores)
-        float2 v[5];
+    T sl[8], sr[8];
 #pragma unroll
-        for (int s = 0; s < 5; ++s) v[s] = make_float2(ch[s], ch[NST - 1 - s]);
-        float2 bad = f2(0.f), kept = f2(0.f);
-        float2 w;
-        if constexpr (SCHEME == TENO5) {
-            w = teno5_core2(v, bad, true, kept);
-            cut += 6u - unsigned(kept.x + kept.y);
-        } else {
-            w = weno5_core2(v, bad);
-        }
-        flag_bad(bad, flags);
-        wl = w.x;
-        wr = w.y;
-    } else {
-        T sl[8], sr[8];
-#pragma unroll
-        for (int s = 0; s < W; ++s) {
-            sl[s] = ch[s];
-            sr[s] = ch[NST - 1 - s];
-        }
-        wl = recon_core<SCHEME, T>(sl, flags, cut);
-        wr = recon_core<SCHEME, T>(sr, flags, cut);
+    for (int s = 0; s < W; ++s) {
+        sl[s] = ch[s];
+        sr[s] = ch[NST - 1 - s];
     }
+    wl = recon_core<SCHEME, T>(sl, flags, cut);
+    wr = recon_core<SCHEME, T>(sr, flags, cut);
     T col[5];
     right_col<K, T>(e, col);
 #pragma unroll
@@ -257,28 +238,26 @@ __device__ __forceinline__ void rusanov_n(const double (&qL)[5], const double (&
                                           double gamma, double (&F)[5], unsigned& flags) {
     const double iL = 1.0 / qL[0], iR = 1.0 / qR[0];
     const double uL[3] = {qL[1] * iL, qL[2] * iL, qL[3] * iL}, uR[3] = {qR[1] * iR, qR[2] * iR, qR[3] * iR};
-    const double eL = (qL[4] - 0.5 * qL[0] * (uL[0] * uL[0] + uL[1] * uL[1] + uL[2] * uL[2])) / qL[0];
-    const double eR = (qR[4] - 0.5 * qR[0] * (uR[0] * uR[0] + uR[1] * uR[1] + uR[2] * uR[2])) / qR[0];
-    const double pL = (gamma - 1.0) * qL[0] * eL, pR = (gamma - 1.0) * qR[0] * eR;
+    const double kL = fma(qL[1], uL[0], fma(qL[2], uL[1], mul_rn(qL[3], uL[2])));  // 2 x kinetic energy
+    const double kR = fma(qR[1], uR[0], fma(qR[2], uR[1], mul_rn(qR[3], uR[2])));
+    const double pL = (gamma - 1.0) * fma(-0.5, kL, qL[4]), pR = (gamma - 1.0) * fma(-0.5, kR, qR[4]);
     if (!(qL[0] > 0.0) || !(qR[0] > 0.0)) flags |= FLAG_DENSITY;
     if (!(pL > 0.0) || !(pR > 0.0)) flags |= FLAG_PRESSURE;
-    const double cL = sqrt(gamma * pL / qL[0]), cR = sqrt(gamma * pR / qR[0]);
-    const double unL = uL[0] * n[0] + uL[1] * n[1] + uL[2] * n[2];
-    const double unR = uR[0] * n[0] + uR[1] * n[1] + uR[2] * n[2];
-    double fL[5], fR[5];
-    fL[0] = qL[0] * unL;
-    fR[0] = qR[0] * unR;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        fL[1 + d] = qL[1 + d] * unL + pL * n[d];
-        fR[1 + d] = qR[1 + d] * unR + pR * n[d];
-    }
-    fL[4] = (qL[4] + pL) * unL;
-    fR[4] = (qR[4] + pR) * unR;
-    const double lam = fmax(fabs(unL) + cL, fabs(unR) + cR);
+    const double cL = sqrt(gamma * pL * iL), cR = sqrt(gamma * pR * iR);
+    const double unL = fma(uL[0], n[0], fma(uL[1], n[1], mul_rn(uL[2], n[2])));
+    const double unR = fma(uR[0], n[0], fma(uR[1], n[1], mul_rn(uR[2], n[2])));
+    const double lam = fmax(add_rn(fabs(unL), cL), add_rn(fabs(unR), cR));
     if (!isfinite(lam) || !(lam > 0.0)) flags |= FLAG_NONFINITE;
+    // F = (f_L + f_R) / 2 - lam / 2 (q_R - q_L), the halves on u_n, p and lam
+    const double hl = mul_rn(0.5, lam), hL = mul_rn(0.5, unL), hR = mul_rn(0.5, unR);
+    const double hp = mul_rn(0.5, add_rn(pL, pR));
 #pragma unroll
-    for (int k = 0; k < 5; ++k) F[k] = 0.5 * (fL[k] + fR[k]) - 0.5 * lam * (qR[k] - qL[k]);
+    for (int k = 0; k < 5; ++k) {
+        double f = fma(qL[k], hL, mul_rn(qR[k], hR));
+        if (k >= 1 && k <= 3) f = fma(hp, n[k >= 1 && k <= 3 ? k - 1 : 0], f);
+        if (k == 4) f = fma(pL, hL, fma(pR, hR, f));
+        F[k] = fma(-hl, add_rn(qR[k], -qL[k]), f);
+    }
 }
 
 // Roe with the entropy fix and the reference's eigenvalue / eigenvector
@@ -501,13 +480,249 @@ __device__ __forceinline__ void flux_dev_n(const Ref32& r, const float (&dL)[5],
     }
 }
 
+// ---- WENO5 / TENO5 faces in differences -----------------------------------
+// The five state differences of the stencil are projected (not the six
+// points), the cores are those of the Cartesian faces (indicators64 /
+// indicators2), and the face states are q-bar + R (deltas).  The projection
+// runs through A and B (as the compact Cartesian form) instead of five dense
+// rows: 20 operations a difference instead of 25 a point and the rows.
+template <typename T>
+struct CurvEig {
+    T u[3], n[3], l[3], m[3];
+    T un, ul, um, h, H, c, b1, b2, x1;
+};
+
+template <typename T>
+__device__ __forceinline__ T dot3(const T (&a)[3], const T (&b)[3]) {
+    return fma(a[0], b[0], fma(a[1], b[1], mul_rn(a[2], b[2])));
+}
+
+template <typename T>
+__device__ __forceinline__ void curv_eig(const T (&q)[5], T p, const T (&n)[3], T gamma, CurvEig<T>& e) {
+    const T inv = rcp<T>(q[0]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        e.u[k] = mul_rn(q[1 + k], inv);
+        e.n[k] = n[k];
+    }
+    // tangents as the reference builds them: l = (-n2, n1, 0) or (-n3, 0, n1), unit; m = n x l
+    const bool flat = fabs(n[2]) <= fabs(n[1]);
+    const T t = flat ? n[1] : n[2];
+    const T is = rsqrt_<T>(fma(n[0], n[0], mul_rn(t, t)));
+    const T a = mul_rn(-t, is), b = mul_rn(n[0], is);
+    e.l[0] = a;
+    e.l[1] = flat ? b : T(0);
+    e.l[2] = flat ? T(0) : b;
+    e.m[0] = fma(n[1], e.l[2], -mul_rn(n[2], e.l[1]));
+    e.m[1] = fma(n[2], e.l[0], -mul_rn(n[0], e.l[2]));
+    e.m[2] = fma(n[0], e.l[1], -mul_rn(n[1], e.l[0]));
+    e.un = dot3(e.u, e.n);
+    e.ul = dot3(e.u, e.l);
+    e.um = dot3(e.u, e.m);
+    e.h = mul_rn(T(0.5), dot3(e.u, e.u));
+    e.H = mul_rn(add_rn(q[4], p), inv);
+    const T c2 = mul_rn(mul_rn(gamma, p), inv);
+    const T ic = rsqrt_<T>(c2);
+    e.c = mul_rn(c2, ic);
+    e.b1 = mul_rn(add_rn(gamma, T(-1)), mul_rn(ic, ic));
+    e.b2 = mul_rn(T(0.5), e.b1);
+    e.x1 = mul_rn(T(0.5), ic);
+}
+
+// Overloads so that one text serves T = double (a point) and float2 (a pair
+// of points, basis values broadcast).
+__device__ __forceinline__ double bc(double x, double) { return x; }
+__device__ __forceinline__ float bc(float x, float) { return x; }
+__device__ __forceinline__ float2 bc(float x, float2) { return f2(x); }
+__device__ __forceinline__ double fmaT(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fmaT(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float2 fmaT(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ double mulT(double a, double b) { return mul_rn(a, b); }
+__device__ __forceinline__ float mulT(float a, float b) { return mul_rn(a, b); }
+__device__ __forceinline__ float2 mulT(float2 a, float2 b) { return mul2(a, b); }
+__device__ __forceinline__ double addT(double a, double b) { return add_rn(a, b); }
+__device__ __forceinline__ float2 addT(float2 a, float2 b) { return add2(a, b); }
+__device__ __forceinline__ double subT(double a, double b) { return add_rn(a, -b); }
+__device__ __forceinline__ float2 subT(float2 a, float2 b) { return sub2(a, b); }
+
+template <typename S, typename T>
+__device__ __forceinline__ void curv_project(const CurvEig<S>& e, const T (&q)[5], T (&w)[5]) {
+    const T o = q[0];
+    const T nA = fmaT(bc(-e.u[0], o), q[1], fmaT(bc(-e.u[1], o), q[2], fmaT(bc(-e.u[2], o), q[3],
+                      fmaT(bc(e.h, o), q[0], q[4]))));
+    auto along = [&](const S (&d)[3], S ud) {  // d . m - u_d rho
+        return fmaT(bc(d[0], o), q[1], fmaT(bc(d[1], o), q[2], fmaT(bc(d[2], o), q[3], mulT(bc(-ud, o), q[0]))));
+    };
+    const T nB = along(e.n, e.un);
+    const T y = mulT(bc(e.b2, o), nA);
+    w[0] = fmaT(bc(-e.b1, o), nA, q[0]);
+    w[1] = along(e.l, e.ul);
+    w[2] = along(e.m, e.um);
+    w[3] = fmaT(bc(-e.x1, o), nB, y);
+    w[4] = fmaT(bc(e.x1, o), nB, y);
+}
+
+// R w.
+template <typename S, typename T>
+__device__ __forceinline__ void curv_back(const CurvEig<S>& e, const T (&w)[5], T (&q)[5]) {
+    const T o = w[0];
+    const T P = addT(w[3], w[4]);
+    const T s = addT(w[0], P);
+    const T cD = mulT(bc(e.c, o), subT(w[4], w[3]));
+    q[0] = s;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        q[1 + k] = fmaT(bc(e.u[k], o), s, fmaT(bc(e.n[k], o), cD, fmaT(bc(e.l[k], o), w[1], mulT(bc(e.m[k], o), w[2]))));
+    q[4] = fmaT(bc(e.h, o), w[0], fmaT(bc(e.ul, o), w[1], fmaT(bc(e.um, o), w[2],
+           fmaT(bc(e.H, o), P, mulT(bc(e.un, o), cD)))));
+}
+
+// FP64 face: flux per unit area along n.
+template <int SCHEME, int FLUX>
+__device__ __forceinline__ void curv_face64(const double (&st)[SchemeInfo<SCHEME>::NST][5], const double (&n)[3],
+                                            double gamma, double (&F)[5], unsigned& flags, unsigned& cut) {
+    constexpr int NST = SchemeInfo<SCHEME>::NST, W = SchemeInfo<SCHEME>::W;
+    double qavg[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) qavg[v] = 0.5 * (st[NST / 2 - 1][v] + st[NST / 2][v]);
+    double qL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, qR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if constexpr (SCHEME == WENO5 || SCHEME == TENO5) {
+        CurvEig<double> e;
+        curv_eig<double>(qavg, pressure_n(qavg, gamma, flags), n, gamma, e);
+        double w[5][5];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            double d[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) d[v] = add_rn(st[s + 1][v], -st[s][v]);
+            curv_project(e, d, w[s]);
+        }
+        double wl[5], wr[5], dl[5], dr[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            const double x[5] = {w[0][v], w[1][v], w[2][v], w[3][v], w[4][v]};
+            if constexpr (SCHEME == WENO5) weno5_pair64(x, wl[v], wr[v], flags);
+            else teno5_pair64(x, wl[v], wr[v], flags, cut);
+        }
+        curv_back(e, wl, dl);
+        curv_back(e, wr, dr);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            qL[v] = add_rn(qavg[v], dl[v]);
+            qR[v] = add_rn(qavg[v], dr[v]);
+        }
+    } else {
+        CharBasis e;
+        char_basis_n(qavg, n, gamma, e, flags);
+        recon_field<0, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+        recon_field<1, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+        recon_field<2, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+        recon_field<3, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+        recon_field<4, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+    }
+    flux_n<FLUX>(qL, qR, n, gamma, F, flags);
+}
+
+// phys_flux_dev_n for the (left, right) pair and the Rusanov flux deviation.
+__device__ __forceinline__ void rusanov_dev_n2(const Ref32& r, const float2 (&d)[5], const float (&n)[3], float gamma,
+                                               float (&F)[5], unsigned& flags) {
+    const float2 rho = add2(f2(r.q[0]), d[0]);
+    const float2 irho = rcp2(rho);
+    float2 du[3], u[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        du[k] = mul2(fma2(f2(-r.u[k]), d[0], d[1 + k]), irho);
+        u[k] = add2(f2(r.u[k]), du[k]);
+    }
+    const float2 dmu = fma2(f2(r.q[1]), du[0], fma2(f2(r.q[2]), du[1], fma2(f2(r.q[3]), du[2],
+                       fma2(d[1], u[0], fma2(d[2], u[1], mul2(d[3], u[2]))))));
+    const float2 dp = mul2(f2(gamma - 1.f), fma2(f2(-0.5f), dmu, d[4]));
+    const float2 p = add2(f2(r.p), dp);
+    if (!(rho.x > 0.f) || !(rho.y > 0.f)) flags |= FLAG_DENSITY;
+    if (!(p.x > 0.f) || !(p.y > 0.f)) flags |= FLAG_PRESSURE;
+    const float2 dun = fma2(du[0], f2(n[0]), fma2(du[1], f2(n[1]), mul2(du[2], f2(n[2]))));
+    const float2 un = fma2(u[0], f2(n[0]), fma2(u[1], f2(n[1]), mul2(u[2], f2(n[2]))));
+    float2 f[5];
+    f[0] = fma2(d[1], f2(n[0]), fma2(d[2], f2(n[1]), mul2(d[3], f2(n[2]))));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) f[1 + k] = fma2(f2(r.q[1 + k]), dun, fma2(d[1 + k], un, mul2(dp, f2(n[k]))));
+    f[4] = fma2(f2(r.q[4] + r.p), dun, mul2(add2(d[4], dp), un));
+    const float2 x = mul2(mul2(f2(gamma), p), irho);
+    const float2 c = f2(x.x * rsqrtf(x.x), x.y * rsqrtf(x.y));
+    const float lam = fmaxf(fabsf(un.x) + c.x, fabsf(un.y) + c.y);
+    const float2 lr = f2(lam, -lam);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        const float2 y = fma2(lr, d[v], f[v]);
+        F[v] = (y.x + y.y) * 0.5f;
+    }
+}
+
+// WENO5 / TENO5 face in the FP32-flux form (face_flux_dev32x2 along n).
+template <int SCHEME, int FLUX>
+__device__ __forceinline__ void curv_face_dev32x2(const float (&d)[6][5], const Ref32& ref, const float (&n)[3],
+                                                  float gamma, float (&F)[5], unsigned& flags, unsigned& cut,
+                                                  bool count) {
+    float dbar[5], qa[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        dbar[v] = 0.5f * (d[2][v] + d[3][v]);
+        qa[v] = ref.q[v] + dbar[v];
+    }
+    const float pa = (gamma - 1.f) * (qa[4] - 0.5f * (qa[1] * qa[1] + qa[2] * qa[2] + qa[3] * qa[3]) * rcp_approx(qa[0]));
+    if (!(qa[0] > 0.f) || !(pa > 0.f)) flags |= FLAG_PRESSURE;
+    CurvEig<float> e;
+    curv_eig<float>(qa, pa, n, gamma, e);
+    float2 E[2][5];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        float2 x[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[4 - k][v]), f2(d[k][v], d[5 - k][v]));
+        curv_project(e, x, E[k]);
+    }
+    float mid[5], E2[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) mid[v] = d[3][v] - d[2][v];
+    curv_project(e, mid, E2);
+    float2 w[5], dq[5], kept = f2(0.f), bad = f2(0.f);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        const float2 e2 = f2(E2[v], -E2[v]);
+        if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], e2, bad, count, kept);
+        else w[v] = weno5_delta2(E[0][v], E[1][v], e2, bad);
+    }
+    flag_bad(bad, flags);
+    if constexpr (SCHEME == TENO5) {
+        if (count) cut += 30u - unsigned(kept.x + kept.y);
+    }
+    curv_back(e, w, dq);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) dq[v] = add2(f2(dbar[v]), dq[v]);
+    if constexpr (FLUX == RUSANOV) {
+        rusanov_dev_n2(ref, dq, n, gamma, F, flags);
+    } else {
+        float dL[5], dR[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            dL[v] = dq[v].x;
+            dR[v] = dq[v].y;
+        }
+        flux_dev_n<FLUX>(ref, dL, dR, n, gamma, F, flags);
+    }
+}
+
 // One face in the FP32-flux form: stencil deviations d from the reference
 // ref, eigen basis at the face average, characteristic reconstruction, flux
 // deviation along the unit normal n (per unit area).
 template <int SCHEME, int FLUX>
 __device__ __forceinline__ void curv_face_dev32(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
                                                 const float (&n)[3], float gamma, float (&F)[5], unsigned& flags,
-                                                unsigned& cut) {
+                                                unsigned& cut, bool count) {
+    if constexpr (SCHEME == WENO5 || SCHEME == TENO5) {
+        curv_face_dev32x2<SCHEME, FLUX>(d, ref, n, gamma, F, flags, cut, count);
+        return;
+    }
     constexpr int NST = SchemeInfo<SCHEME>::NST, W = SchemeInfo<SCHEME>::W, CL = NST / 2 - 1;
     float qa[5];
 #pragma unroll
@@ -527,6 +742,14 @@ __device__ __forceinline__ void curv_face_dev32(const float (&d)[SchemeInfo<SCHE
 
 }  // namespace
 
+// Unit normal (x, y, z) and area (w) of the face whose lower node is `face`:
+// one 32-byte record.
+__device__ __forceinline__ double4 face_geometry(const GridView& g, int axis, long long face) {
+    const double2* p = reinterpret_cast<const double2*>(g.geom[axis]) + 2 * face;
+    const double2 a = __ldg(p), b = __ldg(p + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+
 // ---------------------------------------------------------------------------
 // Face geometry from node metrics (SF_canonicalFace.h:56-118): stored for the
 // faces whose lower node is i; the upper node wraps on periodic axes and
@@ -534,7 +757,7 @@ __device__ __forceinline__ void curv_face_dev32(const float (&d)[SchemeInfo<SCHE
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) curv_geometry_kernel(GridView g, const double* __restrict__ nm,
                                                             double* geom0, double* geom1, double* geom2,
-                                                            unsigned* flags) {
+                                                            float4* geom32, unsigned* flags) {
     const long long nodes = (long long)g.n[0] * g.n[1] * g.n[2];
     const long long vs = g.vs;
     double* geom[3] = {geom0, geom1, geom2};
@@ -560,11 +783,33 @@ __global__ void __launch_bounds__(256) curv_geometry_kernel(GridView g, const do
                                                      __dmul_rn(cof[2], cof[2])));
             if (!isfinite(area) || !(area > 0.0)) fl |= FLAG_NONFINITE;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) geom[a][k * vs + t] = __ddiv_rn(cof[k], area);
-            geom[a][3 * vs + t] = area;
+            for (int k = 0; k < 3; ++k) geom[a][4 * t + k] = __ddiv_rn(cof[k], area);
+            geom[a][4 * t + 3] = area;
+            if (geom32)
+                geom32[a * vs + t] = make_float4(float(geom[a][4 * t]), float(geom[a][4 * t + 1]),
+                                                 float(geom[a][4 * t + 2]), float(area));
         }
     }
     if (fl) atomicOr(flags, fl);
+}
+
+// Net face cofactor of every solved node of a 2-D grid: sum over the axes of
+// (upper - lower face) normal x area, which multiplies F(q_ref) in the
+// FP32-flux tile (3 x vs).
+__global__ void __launch_bounds__(256) curv_net_kernel(GridView g, double* net) {
+    const long long cx = g.hi[0] - g.lo[0], total = cx * (g.hi[1] - g.lo[1]);
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int i = g.lo[0] + (int)(t % cx), j = g.lo[1] + (int)(t / cx);
+        const long long node = (long long)j * g.n[0] + i;
+        const long long xl = (long long)j * g.n[0] + (i > 0 ? i - 1 : g.n[0] - 1);
+        const long long yl = (long long)(j > 0 ? j - 1 : g.n[1] - 1) * g.n[0] + i;
+        const double4 xu = face_geometry(g, 0, node), xd = face_geometry(g, 0, xl);
+        const double4 yu = face_geometry(g, 1, node), yd = face_geometry(g, 1, yl);
+        net[node] = xu.x * xu.w - xd.x * xd.w + yu.x * yu.w - yd.x * yd.w;
+        net[g.vs + node] = xu.y * xu.w - xd.y * xd.w + yu.y * yu.w - yd.y * yd.w;
+        net[2 * g.vs + node] = xu.z * xu.w - xd.z * xd.w + yu.z * yu.w - yd.z * yd.w;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -575,7 +820,7 @@ __global__ void __launch_bounds__(256) curv_geometry_kernel(GridView g, const do
 template <int SCHEME, int FLUX>
 __global__ void __launch_bounds__(128, 4) curv_face_kernel(GridView g, StageView sv, int axis, double* fl) {
     if (sv.require_active && !sv.clock->active) return;
-    constexpr int NST = SchemeInfo<SCHEME>::NST, W = SchemeInfo<SCHEME>::W;
+    constexpr int NST = SchemeInfo<SCHEME>::NST;
     const int a = axis;
     int base[3], span[3];
 #pragma unroll
@@ -606,22 +851,11 @@ __global__ void __launch_bounds__(128, 4) curv_face_kernel(GridView g, StageView
             for (int v = 0; v < 5; ++v) st[s][v] = sv.qs[v * vs + node];
         }
         const long long face = ((long long)c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
-        const double* gm = g.geom[a];
-        const double n[3] = {gm[face], gm[vs + face], gm[2 * vs + face]};
-        const double area = gm[3 * vs + face];
-        double qavg[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) qavg[v] = 0.5 * (st[NST / 2 - 1][v] + st[NST / 2][v]);
-        CharBasis e;
-        char_basis_n(qavg, n, g.gamma, e, flags);
-        double qL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, qR[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, F[5];
-        recon_field<0, SCHEME, NST, W>(e, st, qL, qR, flags, cut);
-        recon_field<1, SCHEME, NST, W>(e, st, qL, qR, flags, cut);
-        recon_field<2, SCHEME, NST, W>(e, st, qL, qR, flags, cut);
-        recon_field<3, SCHEME, NST, W>(e, st, qL, qR, flags, cut);
-        recon_field<4, SCHEME, NST, W>(e, st, qL, qR, flags, cut);
+        const double4 gm = face_geometry(g, a, face);
+        const double n[3] = {gm.x, gm.y, gm.z}, area = gm.w;
+        double F[5];
+        curv_face64<SCHEME, FLUX>(st, n, g.gamma, F, flags, cut);
         if (SCHEME == TENO5) cores += 10;
-        flux_n<FLUX>(qL, qR, n, g.gamma, F, flags);
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
             const double x = F[v] * area;
@@ -674,12 +908,11 @@ __global__ void __launch_bounds__(128, 4) curv_face_f32_kernel(GridView g, Stage
             for (int v = 0; v < 5; ++v) d[s][v] = float(sv.qs[v * vs + node[s]] - qref[v]);
         const Ref32 ref = make_ref32(qref, g.gamma);
         const long long face = ((long long)c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
-        const double* gm = g.geom[a];
-        const double n64[3] = {gm[face], gm[vs + face], gm[2 * vs + face]};
-        const double area = gm[3 * vs + face];
+        const double4 gm = face_geometry(g, a, face);
+        const double n64[3] = {gm.x, gm.y, gm.z}, area = gm.w;
         const float n[3] = {float(n64[0]), float(n64[1]), float(n64[2])};
         float F[5];
-        curv_face_dev32<SCHEME, FLUX>(d, ref, n, float(g.gamma), F, flags, cut);
+        curv_face_dev32<SCHEME, FLUX>(d, ref, n, float(g.gamma), F, flags, cut, sv.counters != nullptr);
         if (SCHEME == TENO5) cores += 10;
         double fref[5];
         euler_flux_n(qref, n64, g.gamma, fref, flags);
@@ -721,15 +954,13 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) curv_tile2d_f32_kernel(GridVi
     double qref[5];
     load_ref(g, sv.qs, qref);
     const Ref32 ref = make_ref32(qref, g.gamma);
-    for (int t = threadIdx.x; t < SX * SY; t += blockDim.x) {
-        const int r = t / SX, c = t - r * SX;
-        if ((r < H || r >= TY + H) && (c < H || c >= TX + H)) continue;
-        const int gx = map_tile_index(x0 - H + c, g.n[0], g.bc_lo[0], g.bc_hi[0]);
-        const int gy = map_tile_index(y0 - H + r, g.n[1], g.bc_lo[1], g.bc_hi[1]);
-        const long long at = (long long)gy * nx + gx;
+    stage_rows<TX, TY, H>(g, x0, y0, [&](int t, long long at) {
+        double q[5];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) sq[v * SX * SY + t] = float(__ldg(sv.qs + v * vs + at) - qref[v]);
-    }
+        for (int v = 0; v < 5; ++v) q[v] = __ldg(sv.qs + v * vs + at);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) sq[v * SX * SY + t] = float(q[v] - qref[v]);
+    });
     __syncthreads();
     const float gamma = float(g.gamma);
     // face (i | i+1) geometry sits at its lower node; only the periodic wrap
@@ -753,9 +984,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) curv_tile2d_f32_kernel(GridVi
 #pragma unroll
                 for (int v = 0; v < 5; ++v) st[s][v] = base[v * SX * SY + s];
             const long long face = (long long)gy * nx + lower(gl, 0);
-            const float n[3] = {float(g.geom[0][face]), float(g.geom[0][vs + face]), float(g.geom[0][2 * vs + face])};
-            curv_face_dev32<SCHEME, FLUX>(st, ref, n, gamma, Ft, flags, cut);
-            const float area = float(g.geom[0][3 * vs + face]);
+            const float4 gm = __ldg(reinterpret_cast<const float4*>(g.geom32) + face);
+            const float n[3] = {gm.x, gm.y, gm.z};
+            curv_face_dev32<SCHEME, FLUX>(st, ref, n, gamma, Ft, flags, cut, sv.counters != nullptr);
+            const float area = gm.w;
 #pragma unroll
             for (int v = 0; v < 5; ++v) fx[v * NFX + f] = Ft[v] * area;
         } else {
@@ -774,9 +1006,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) curv_tile2d_f32_kernel(GridVi
 #pragma unroll
                 for (int v = 0; v < 5; ++v) st[s][v] = base[v * SX * SY + s * SX];
             const long long face = (long long)lower(gl, 1) * nx + gx;
-            const float n[3] = {float(g.geom[1][face]), float(g.geom[1][vs + face]), float(g.geom[1][2 * vs + face])};
-            curv_face_dev32<SCHEME, FLUX>(st, ref, n, gamma, Ft, flags, cut);
-            const float area = float(g.geom[1][3 * vs + face]);
+            const float4 gm = __ldg(reinterpret_cast<const float4*>(g.geom32) + vs + face);
+            const float n[3] = {gm.x, gm.y, gm.z};
+            curv_face_dev32<SCHEME, FLUX>(st, ref, n, gamma, Ft, flags, cut, sv.counters != nullptr);
+            const float area = gm.w;
 #pragma unroll
             for (int v = 0; v < 5; ++v) fy[v * NFY + k] = Ft[v] * area;
         }
@@ -804,13 +1037,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) curv_tile2d_f32_kernel(GridVi
         const int gx = x0 + c, gy = y0 + r;
         if (gx >= g.hi[0] || gy >= g.hi[1]) continue;
         const long long node = (long long)gy * nx + gx;
-        // the node's net face cofactor: upper minus lower face of each axis
-        const long long fxl = (long long)gy * nx + lower(gx - 1, 0), fyl = (long long)lower(gy - 1, 1) * nx + gx;
-        double gc[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            gc[k] = g.geom[0][k * vs + node] * g.geom[0][3 * vs + node] - g.geom[0][k * vs + fxl] * g.geom[0][3 * vs + fxl] +
-                    g.geom[1][k * vs + node] * g.geom[1][3 * vs + node] - g.geom[1][k * vs + fyl] * g.geom[1][3 * vs + fyl];
+        const double gc[3] = {__ldg(g.net + node), __ldg(g.net + vs + node), __ldg(g.net + 2 * vs + node)};
         double div[5], qn[5];
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
@@ -836,7 +1063,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
     if (sv.require_active && !sv.clock->active) return;
     extern __shared__ double smem_d[];
     using S = TileShape<SCHEME, TX, TY>;
-    constexpr int NST = S::NST, W = S::NST == 8 ? 7 : (S::NST == 4 ? 4 : 5), H = S::H, SX = S::SX, SY = S::SY;
+    constexpr int NST = S::NST, H = S::H, SX = S::SX, SY = S::SY;
     constexpr int NFX = S::NFX, NFY = S::NFY, NFXP = S::NFXP, NFYP = S::NFYP;
     const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
     const int x0 = g.lo[0] + (blockIdx.x % ntx) * TX, y0 = g.lo[1] + (blockIdx.x / ntx) * TY;
@@ -845,20 +1072,18 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
     double* fy = fx + 5 * NFX;      // [5][TY+1][TX]
     const long long nx = g.n[0], vs = g.vs;
     unsigned flags = 0, cut = 0, cores = 0;
-    for (int t = threadIdx.x; t < SX * SY; t += blockDim.x) {
-        const int r = t / SX, c = t - r * SX;
-        if ((r < H || r >= TY + H) && (c < H || c >= TX + H)) continue;
-        const int gx = map_tile_index(x0 - H + c, g.n[0], g.bc_lo[0], g.bc_hi[0]);
-        const int gy = map_tile_index(y0 - H + r, g.n[1], g.bc_lo[1], g.bc_hi[1]);
-        const long long at = (long long)gy * nx + gx;
+    stage_rows<TX, TY, H>(g, x0, y0, [&](int t, long long at) {
+        double q[5];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) sq[v * SX * SY + t] = __ldg(sv.qs + v * vs + at);
-    }
+        for (int v = 0; v < 5; ++v) q[v] = __ldg(sv.qs + v * vs + at);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) sq[v * SX * SY + t] = q[v];
+    });
     __syncthreads();
     auto lower = [&](int i, int a) { return i < 0 ? i + g.n[a] : i; };
     for (int f = threadIdx.x; f < NFXP + NFYP; f += blockDim.x) {
         double st[NST][5];
-        const double* gm;
+        int axis;
         double* out;
         long long face;
         int slot, stride;
@@ -874,7 +1099,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
             }
             base = sq + (r + H) * SX + c;
             stride = 1;
-            gm = g.geom[0];
+            axis = 0;
             face = (long long)gy * nx + lower(gl, 0);
             out = fx;
             slot = f;
@@ -890,7 +1115,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
             }
             base = sq + r * SX + (c + H);
             stride = SX;
-            gm = g.geom[1];
+            axis = 1;
             face = (long long)lower(gl, 1) * nx + gx;
             out = fy;
             slot = k;
@@ -899,20 +1124,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) curv_tile2d_kernel(GridView g
         for (int s2 = 0; s2 < NST; ++s2)
 #pragma unroll
             for (int v = 0; v < 5; ++v) st[s2][v] = base[v * SX * SY + s2 * stride];
-        const double n[3] = {gm[face], gm[vs + face], gm[2 * vs + face]};
-        const double area = gm[3 * vs + face];
-        double qavg[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) qavg[v] = 0.5 * (st[NST / 2 - 1][v] + st[NST / 2][v]);
-        CharBasis e;
-        char_basis_n(qavg, n, g.gamma, e, flags);
-        double qL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, qR[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, F[5];
-        recon_field<0, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<1, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<2, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<3, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<4, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        flux_n<FLUX>(qL, qR, n, g.gamma, F, flags);
+        const double4 gm = face_geometry(g, axis, face);
+        const double n[3] = {gm.x, gm.y, gm.z}, area = gm.w;
+        double F[5];
+        curv_face64<SCHEME, FLUX>(st, n, g.gamma, F, flags, cut);
         const int nf = out == fx ? NFX : NFY;
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
@@ -980,11 +1195,17 @@ __global__ void __launch_bounds__(256) curv_stage_kernel(GridView g, StageView s
 }
 
 // ---------------------------------------------------------------------------
-cudaError_t launch_curv_geometry(const GridView& g, const double* nm, double* const geom[3], unsigned* flags,
-                                 cudaStream_t st) {
+cudaError_t launch_curv_geometry(const GridView& g, const double* nm, double* const geom[3], float* geom32,
+                                 double* net, unsigned* flags, cudaStream_t st) {
     const long long nodes = (long long)g.n[0] * g.n[1] * g.n[2];
     const unsigned blocks = (unsigned)std::min<long long>((nodes + 255) / 256, 148LL * 16);
-    curv_geometry_kernel<<<blocks, 256, 0, st>>>(g, nm, geom[0], geom[1], geom[2], flags);
+    curv_geometry_kernel<<<blocks, 256, 0, st>>>(g, nm, geom[0], geom[1], geom[2], reinterpret_cast<float4*>(geom32),
+                                                 flags);
+    if (net) {
+        GridView gv = g;
+        for (int a = 0; a < 3; ++a) gv.geom[a] = geom[a];
+        curv_net_kernel<<<blocks, 256, 0, st>>>(gv, net);
+    }
     return cudaGetLastError();
 }
 

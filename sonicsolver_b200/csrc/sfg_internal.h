@@ -71,7 +71,9 @@ struct GridView {
     int curv;
     const double* node_jac;     // Jac = 1/J per node (vs doubles)
     const double* node_metric;  // xi_x, xi_y, xi_z, eta_x, ..., zeta_z per node (9 x vs)
-    const double* geom[3];      // per axis, face (i | i+1) at its lower node i: unit normal, area (4 x vs)
+    const double* geom[3];      // per axis, face (i | i+1) at its lower node i: unit normal, area (4 doubles a face)
+    const float* geom32;        // 2-D: the same in FP32, axis 0 then axis 1 (4 floats a face)
+    const double* net;          // 2-D: net face cofactor per node (3 x vs)
 };
 
 // Physical boundary laws of the law ends of one grid (SFG_BC_LAW; the

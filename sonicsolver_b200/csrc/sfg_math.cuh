@@ -959,6 +959,72 @@ __device__ __forceinline__ float2 teno5_core2(const float2* v, float2& bad, bool
     return teno5_weights2(k, q, v[2]);
 }
 
+// FP32 WENO5 / TENO5 on a face's six points in differences, the left and right
+// sides as the two lanes of a pair; the mathematics of indicators64.  With the
+// mirror-signed difference pairs E0 = (c1 - c0, c4 - c5), E1 = (c2 - c1,
+// c3 - c4), E2 = (c3 - c2, c2 - c3):
+//   T1 = E1 - E0 = (t1, t4),  T2 = E2 - E1 = (t2, t3),  T2' = its swap
+//   4 b_k = 13/3 t^2 + r^2:  (T1, T1 + 2 E1), (T2, E1 + E2), (T2', T2' - 2 E2)
+//   p_k - mid = T1/3 - T2/2, -T2/6, -T2'/6
+// and the face states are d-bar + R (deltas).  Kept with N2 = -T2.
+struct Diff2 {
+    float2 T1, N2, N2s;  // (t1, t4), -(t2, t3), -(t3, t2)
+    float2 e[3];         // eps + 4 b_k
+};
+
+__device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 E2, float eps) {
+    Diff2 d;
+    d.T1 = sub2(E1, E0);
+    d.N2 = sub2(E1, E2);
+    d.N2s = swap2(d.N2);
+    const float2 r0 = fma2(f2(2.f), E1, d.T1), r1 = add2(E1, E2), r2 = fma2(f2(2.f), E2, d.N2s);
+    const float2 c = f2(13.f / 3.f);
+    const float2 b0 = fma2(mul2(c, d.T1), d.T1, f2(eps)), b1 = fma2(mul2(c, d.N2), d.N2, f2(eps));
+    d.e[0] = fma2(r0, r0, b0);
+    d.e[1] = fma2(r1, r1, b1);
+    d.e[2] = fma2(r2, r2, swap2(b1));
+    return d;
+}
+
+// WENO5-JS deltas of both sides.
+__device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 E2, float2& bad) {
+    const Diff2 d = indicators2(E0, E1, E2, 4.f * 1e-6f);
+    const float2 s0 = mul2(d.e[0], d.e[0]), s1 = mul2(d.e[1], d.e[1]), s2 = mul2(d.e[2], d.e[2]);
+    const float2 wa = mul2(s1, s2), wb = mul2(s0, s2), wc = mul2(s0, s1);  // weights 1 : 6 : 3
+    const float2 den = fma2(f2(3.f), fma2(f2(2.f), wb, wc), wa);
+    const float2 h = mul2(f2(0.5f), d.N2);
+    const float2 num = fma2(wa, fma2(f2(1.f / 3.f), d.T1, h), fma2(wb, d.N2, mul2(wc, swap2(h))));
+    bad = watch2(bad, den);  // den >= 10 eps^4 > 0 unless an input was not finite
+    return mul2(num, rcp2(den));
+}
+
+// TENO5 deltas of both sides.  With `count` (a launch-uniform switch: the
+// cut-off accounting of sfg_set_counting), `kept` accumulates the kept
+// sub-stencils of each lane.  A lane that keeps all three sub-stencils takes
+// the linear weights' sum on the cut-off path too, so its bits do not depend
+// on the vote.
+__device__ __forceinline__ float2 teno5_delta2(float2 E0, float2 E1, float2 E2, float2& bad, bool count,
+                                               float2& kept) {
+    const Diff2 d = indicators2(E0, E1, E2, 0.f);
+    const float2 all = fma2(f2(1.f / 30.f), d.T1, fma2(f2(0.15f), d.N2, mul2(f2(0.05f), d.N2s)));
+    if (warp_all(teno_smooth2(d.e))) {
+        if (count) kept = add2(kept, f2(3.f));
+        return all;
+    }
+    float2 k[3];
+    teno_keep32x2(d.e[0], d.e[1], d.e[2], k, bad);
+    if (count) kept = add2(kept, add2(add2(k[0], k[1]), k[2]));
+    // the sub-stencil with x = 1 always passes (G ~ 1 > lim <= 3e-5, and a NaN
+    // lim fails every test), so act >= 0.1 for finite indicators
+    const float2 d0 = mul2(f2(0.1f), k[0]), d1 = mul2(f2(0.6f), k[1]), d2 = mul2(f2(0.3f), k[2]);
+    const float2 act = add2(add2(d0, d1), d2);
+    const float2 p0 = fma2(f2(1.f / 3.f), d.T1, mul2(f2(0.5f), d.N2));
+    const float2 num = fma2(d0, p0, mul2(f2(1.f / 6.f), fma2(d1, d.N2, mul2(d2, d.N2s))));
+    const float2 w = mul2(num, rcp2(act));
+    const float2 n3 = add2(add2(k[0], k[1]), k[2]);
+    return f2(n3.x == 3.f ? all.x : w.x, n3.y == 3.f ? all.y : w.y);
+}
+
 // The eigen-structure as lane pairs, signs folded in, built once per face.
 // The tangential characteristic variables are taken with the raw Cartesian
 // components, w_t = m_t - u_t rho: the reference's signed tangents (+-e_t)

@@ -41,8 +41,8 @@ cudaError_t launch_tile1d(int scheme, int flux, int prec64, const GridView& g, c
 cudaError_t launch_tile3d(int scheme, int flux, int prec64, const GridView& g, const StageView& sv, cudaStream_t st);
 cudaError_t launch_law_fill(const GridView& g, const LawView& lv, const double* old, double* q, const Clock* clock,
                             int require_active, unsigned* flags, cudaStream_t st);
-cudaError_t launch_curv_geometry(const GridView& g, const double* nm, double* const geom[3], unsigned* flags,
-                                 cudaStream_t st);
+cudaError_t launch_curv_geometry(const GridView& g, const double* nm, double* const geom[3], float* geom32,
+                                 double* net, unsigned* flags, cudaStream_t st);
 cudaError_t launch_curv_stage(int scheme, int flux, int prec64, int tiles, const GridView& g, const StageView& sv,
                               double* fl, cudaStream_t st);
 cudaError_t launch_teno_flips(const GridView& g, const double* q, unsigned long long* out, cudaStream_t st);
@@ -834,7 +834,11 @@ int sfg_set_metrics(sfg_solver s, const double* host, int layout) {
     GridView g = s->gv;
     double* geom[3] = {s->face_geom, s->face_geom + 4 * s->gv.vs, s->face_geom + 8 * s->gv.vs};
     CUDA_TRY(cudaMemsetAsync(s->flags, 0, 64, s->stream));
-    CUDA_TRY(launch_curv_geometry(g, s->node_metrics, geom, s->flags, s->stream));
+    // 2-D tiles: the FP32 face records and the net cofactors live in the parts
+    // of face_flux (5 x vs) and face_geom (4 x vs) that only a third axis uses
+    float* geom32 = g.dim == 2 ? reinterpret_cast<float*>(s->face_flux + 10 * s->gv.vs) : nullptr;
+    double* net = g.dim == 2 ? geom[2] : nullptr;
+    CUDA_TRY(launch_curv_geometry(g, s->node_metrics, geom, geom32, net, s->flags, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     unsigned bits = 0;
     CUDA_TRY(cudaMemcpy(&bits, s->flags, sizeof bits, cudaMemcpyDeviceToHost));
@@ -843,6 +847,8 @@ int sfg_set_metrics(sfg_solver s, const double* host, int layout) {
     s->gv.node_jac = s->node_metrics;
     s->gv.node_metric = s->node_metrics + s->gv.vs;
     for (int a = 0; a < 3; ++a) s->gv.geom[a] = geom[a];
+    s->gv.geom32 = geom32;
+    s->gv.net = net;
     drop_graphs(s);  // the captured launches hold the previous grid view
     return SFG_OK;
 }
