@@ -915,26 +915,6 @@ __device__ __forceinline__ void stencil5x2(const float2* v, float2 (&B)[3], floa
     q[2] = sub2(D2, r2);
 }
 
-// WENO5-JS on a (left, right) stencil pair; same folding as weno5_core.
-__device__ __forceinline__ float2 weno5_core2(const float2* v, float2& bad) {
-    float2 B[3], q[3];
-    stencil5x2(v, B, q);
-    const float2 eps = f2(4.f * 1e-6f);  // the reference's 1e-6 on B_k / 3 = 4 b_k
-    const float2 e0 = add2(eps, B[0]), e1 = add2(eps, B[1]), e2 = add2(eps, B[2]);
-    const float2 s0 = mul2(e0, e0), s1 = mul2(e1, e1), s2 = mul2(e2, e2);
-    const float2 w0 = mul2(f2(0.1f), mul2(s1, s2));
-    const float2 w1 = mul2(f2(0.6f), mul2(s0, s2));
-    const float2 w2 = mul2(f2(0.3f), mul2(s0, s1));
-    const float2 den = mul2(f2(6.f), add2(add2(w0, w1), w2));
-    const float2 num = fma2(w0, q[0], fma2(w1, q[1], mul2(w2, q[2])));
-    bad = watch2(bad, den);  // den >= 6 eps^4 > 0 unless an input was not finite
-    return fma2(num, rcp2(den), v[2]);
-}
-
-// TENO5 on a (left, right) stencil pair, all of it paired: polynomials,
-// smoothness indicators, the cut-off (teno_keep32x2) and the weights.  With
-// `count` (a launch-uniform switch: the cut-off accounting of
-// sfg_set_counting), `kept` accumulates the kept sub-stencils of each lane.
 // TENO5 weights from the keep flags k (1 or 0 per lane): the kept linear
 // weights, renormalised.  No all-cut check: the sub-stencil with x = 1
 // always passes (G ~ 1 > lim <= 3e-5, and a NaN lim fails every '<'), so
@@ -946,13 +926,23 @@ __device__ __forceinline__ float2 teno5_weights2(const float2 (&k)[3], const flo
     return fma2(num, rcp2(act), v2);
 }
 
-__device__ __forceinline__ float2 teno5_core2(const float2* v, float2& bad, bool count, float2& kept) {
+// 1 / act of teno5_weights2 when every sub-stencil is kept, the same bits: one
+// reciprocal a face instead of ten.
+__device__ __forceinline__ float teno5_all_kept() {
+    return rcp_approx(fmaf(6.f, 0.1f, fmaf(6.f, 0.6f, 6.f * 0.3f)));
+}
+
+// TENO5 on a (left, right) stencil pair of points: polynomials, smoothness
+// indicators, the cut-off (teno_keep32x2) and the weights.  With `count` (a
+// launch-uniform switch: the cut-off accounting of sfg_set_counting), `kept`
+// accumulates the kept sub-stencils of each lane; `all`: teno5_all_kept().
+__device__ __forceinline__ float2 teno5_core2(const float2* v, float2& bad, bool count, float2& kept, float all) {
     float2 B[3], q[3], k[3];
     stencil5x2(v, B, q);
     if (warp_all(teno_smooth2(B))) {
-        const float2 all[3] = {f2(1.f), f2(1.f), f2(1.f)};
         if (count) kept = add2(kept, f2(3.f));
-        return teno5_weights2(all, q, v[2]);
+        const float2 num = fma2(f2(0.1f), q[0], fma2(f2(0.6f), q[1], mul2(f2(0.3f), q[2])));
+        return fma2(num, f2(all), v[2]);
     }
     teno_keep32x2(B[0], B[1], B[2], k, bad);
     if (count) kept = add2(kept, add2(add2(k[0], k[1]), k[2]));
@@ -1059,6 +1049,21 @@ __device__ __forceinline__ void to_characteristic2(const Eig2& e, const float2 q
     w[2] = fma2(e.nu[B::M - 1], q[0], q[B::M]);
     w[3] = fma2(e.nx1, nB, b2nA);
     w[4] = fma2(e.x1, nB, b2nA);
+}
+
+// The same for one point (signs of the tangential variables as the pair's).
+template <int AX>
+__device__ __forceinline__ void project32(const Eigen<float>& e, const float (&q)[5], float (&w)[5]) {
+    using B = AxisBasis<AX>;
+    const float vel[3] = {e.u, e.v, e.w};
+    const float nA = fmaf(-e.u, q[1], fmaf(-e.v, q[2], fmaf(-e.w, q[3], fmaf(e.h, q[0], q[4]))));
+    const float nB = fmaf(-vel[B::N - 1], q[0], q[B::N]);
+    const float y = mul_rn(e.b2, nA);
+    w[0] = fmaf(-e.b1, nA, q[0]);
+    w[1] = fmaf(-vel[B::L - 1], q[0], q[B::L]);
+    w[2] = fmaf(-vel[B::M - 1], q[0], q[B::M]);
+    w[3] = fmaf(-e.x1, nB, y);
+    w[4] = fmaf(e.x1, nB, y);
 }
 
 template <int AX>
@@ -1253,23 +1258,44 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[6][5], const 
     Eigen<float> es;
     if (!eigen_at<AX, float>(qbar, gamma, es)) flags |= FLAG_PRESSURE;
     const Eig2 e = eig2(es);
-    // point pairs (k, 5-k): P[k][v] = (c_k, c_{5-k}) of component v
-    float2 P[3][5];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float2 x[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k][v], d[5 - k][v]), f2(dbar[v]));
-        to_characteristic2<AX>(e, x, P[k]);
-    }
     float2 w[5];
     float2 kept = f2(0.f), bad = f2(0.f);
+    if constexpr (SCHEME == TENO5) {
+        // point pairs (k, 5-k): P[k][v] = (c_k, c_{5-k}) of component v.  TENO5
+        // stays on points: in a coarse far field its FP32 cut-offs turn on the
+        // last bits, so another rounding of the indicators moves a run by what
+        // FP32 is off FP64 there (1e-4 on a 48^2 vortex).
+        float2 P[3][5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        // left stencil c0..c4 and right stencil c5..c1 as one paired stencil
-        const float2 st[5] = {P[0][v], P[1][v], P[2][v], swap2(P[2][v]), swap2(P[1][v])};
-        if constexpr (SCHEME == TENO5) w[v] = teno5_core2(st, bad, count, kept);
-        else w[v] = weno5_core2(st, bad);
+        for (int k = 0; k < 3; ++k) {
+            float2 x[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k][v], d[5 - k][v]), f2(dbar[v]));
+            to_characteristic2<AX>(e, x, P[k]);
+        }
+        const float all = teno5_all_kept();
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            // left stencil c0..c4 and right stencil c5..c1 as one paired stencil
+            const float2 st[5] = {P[0][v], P[1][v], P[2][v], swap2(P[2][v]), swap2(P[1][v])};
+            w[v] = teno5_core2(st, bad, count, kept, all);
+        }
+    } else {
+        // WENO5: mirror-signed difference pairs (d_{k+1} - d_k, d_{4-k} - d_{5-k}), projected
+        float2 E[2][5];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            float2 x[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[4 - k][v]), f2(d[k][v], d[5 - k][v]));
+            to_characteristic2<AX>(e, x, E[k]);
+        }
+        float m[5], E2[5];  // the middle difference, the same on both sides up to its sign
+#pragma unroll
+        for (int v = 0; v < 5; ++v) m[v] = d[3][v] - d[2][v];
+        project32<AX>(es, m, E2);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) w[v] = weno5_delta2(E[0][v], E[1][v], f2(E2[v], -E2[v]), bad);
     }
     flag_bad(bad, flags);
     if constexpr (SCHEME == TENO5) {
