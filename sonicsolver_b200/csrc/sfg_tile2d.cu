@@ -1,79 +1,11 @@
-// sfg_tile2d.cu -- single-grid fused stage kernels for 2-D grids: one launch
-// per stage, one block per tile (bodies in sfg_tile.cuh).
-#include "sfg_tile.cuh"
+// sfg_tile2d.cu -- the 2-D tile launcher with its full-size tiles (32 x 15,
+// 22 x 22), and the 1-D tiles.
+#include "sfg_tile2d.cuh"
 
 namespace sfg {
 
-template <int SCHEME, int FLUX, int TX, int TY>
-__global__ void __launch_bounds__(TILE_THREADS, 2) tile2d_kernel(GridView g, StageView sv) {
-    extern __shared__ __align__(16) double smem[];
-    if (sv.require_active && !sv.clock->active) return;
-    const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
-    const int x0 = g.lo[0] + (blockIdx.x % ntx) * TX, y0 = g.lo[1] + (blockIdx.x / ntx) * TY;
-    unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
-    tile2d_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smem, flags, cut, cores, sr);
-    flush_status(sv, flags, cores, cut);
-    if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
-    if (sv.mode & MODE_STEP) step_tail(sv);
-}
-
-template <int SCHEME, int FLUX, int TX, int TY>
-__global__ void __launch_bounds__(TILE_THREADS, 4) tile2d_f32_kernel(GridView g, StageView sv) {
-    extern __shared__ __align__(16) float smemf[];
-    if (sv.require_active && !sv.clock->active) return;
-    const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
-    const int x0 = g.lo[0] + (blockIdx.x % ntx) * TX, y0 = g.lo[1] + (blockIdx.x / ntx) * TY;
-    unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
-    tile2d_f32_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smemf, flags, cut, cores, sr);
-    flush_status(sv, flags, cores, cut);
-    if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
-    if (sv.mode & MODE_STEP) step_tail(sv);
-}
-
-template <int SCHEME, int FLUX, typename T, int TX, int TY>
-static cudaError_t launch_tile(const GridView& g, const StageView& sv, cudaStream_t st) {
-    using S = TileShape<SCHEME, TX, TY>;
-    constexpr size_t smem = sizeof(T) * S::ELEMS;
-    static std::atomic<unsigned long long> configured{0};
-    unsigned long long bit = 0;
-    const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
-    const int nty = (g.hi[1] - g.lo[1] + TY - 1) / TY;
-    auto kern = sizeof(T) == sizeof(float) ? tile2d_f32_kernel<SCHEME, FLUX, TX, TY> : tile2d_kernel<SCHEME, FLUX, TX, TY>;
-    if (attributes_pending(configured, bit)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        configured.fetch_or(bit, std::memory_order_release);
-    }
-    kern<<<ntx * nty, TILE_THREADS, smem, st>>>(g, sv);
-    return cudaGetLastError();
-}
-
-template <int FLUX, typename T, int TX, int TY>
-static cudaError_t launch_tile_s(int scheme, const GridView& g, const StageView& sv, cudaStream_t st) {
-    switch (scheme) {
-    case WENO5: return launch_tile<WENO5, FLUX, T, TX, TY>(g, sv, st);
-    case TENO5: return launch_tile<TENO5, FLUX, T, TX, TY>(g, sv, st);
-    case WENO3: return launch_tile<WENO3, FLUX, T, TX, TY>(g, sv, st);
-    case WENO7: return launch_tile<WENO7, FLUX, T, TX, TY>(g, sv, st);
-    }
-    return cudaErrorInvalidValue;
-}
-
-// Rusanov and Roe in both precisions; Steger-Warming, Lax-Friedrichs and
-// Lax-Wendroff faces in FP64 (the FP32 deviation form is Rusanov / Roe).
-template <typename T, int TX, int TY>
-static cudaError_t launch_tile_t(int scheme, int flux, const GridView& g, const StageView& sv, cudaStream_t st) {
-    if (flux == RUSANOV) return launch_tile_s<RUSANOV, T, TX, TY>(scheme, g, sv, st);
-    if (flux == ROE) return launch_tile_s<ROE, T, TX, TY>(scheme, g, sv, st);
-    if constexpr (sizeof(T) == sizeof(double)) {
-        if (flux == STEGER) return launch_tile_s<STEGER, T, TX, TY>(scheme, g, sv, st);
-        if (flux == LAXF) return launch_tile_s<LAXF, T, TX, TY>(scheme, g, sv, st);
-        if (flux == LAXW) return launch_tile_s<LAXW, T, TX, TY>(scheme, g, sv, st);
-    }
-    return cudaErrorInvalidValue;
-}
+cudaError_t launch_tile2d_small(int rounds, int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
+                                cudaStream_t st);
 
 // 1-D grids: one block per 511-node tile (the body the batched kernels use,
 // so a 1-D grid gives the same bits alone and in a batch).
@@ -132,16 +64,26 @@ cudaError_t launch_tile1d(int scheme, int flux, int prec64, const GridView& g, c
     return prec64 ? launch_tile1_t<double>(scheme, flux, g, sv, st) : launch_tile1_t<float>(scheme, flux, g, sv, st);
 }
 
-// variant 1: 32 x 15 tile, variant 2: 22 x 22 tile (256 threads each).
+// variant 1: 32 x 15 tile, variant 2: 22 x 22 tile (256 threads each, four
+// rounds of faces); every shape gives the same bits.  A grid too small to
+// fill the GPU with them takes 32 x 7 (two rounds) or 16 x 7 (one round):
+// the smallest whose blocks are all resident at once (2 per SM in FP64, 4 in
+// FP32), because then a stage lasts as long as one block, and a block as long
+// as its rounds.  Measured, us per SSPRK3 step of three launches, 32 x 15 /
+// 32 x 7 / 16 x 7: FP64 WENO5 64^2 43 / 31 / 26, 192 x 160 48 / 34 / 30,
+// 257 x 193 48 / 42 / 44, 320^2 62 / 64 / 72, 512^2 107 / 114 / 145; FP32
+// 64^2 36 / 28 / 24, 257 x 193 42 / 35 / 34, 320^2 48 / 44 / 44, 400^2 59 /
+// 56 / 59, 512^2 69 / 71 / 87 (more blocks repeat more halo and edge faces).
 cudaError_t launch_tile2d(int variant, int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
                           cudaStream_t st) {
-    if (variant == 1)
-        return prec64 ? launch_tile_t<double, 32, 15>(scheme, flux, g, sv, st)
-                      : launch_tile_t<float, 32, 15>(scheme, flux, g, sv, st);
-    if (variant == 2)
-        return prec64 ? launch_tile_t<double, 22, 22>(scheme, flux, g, sv, st)
-                      : launch_tile_t<float, 22, 22>(scheme, flux, g, sv, st);
-    return cudaErrorInvalidValue;
+    if (variant < 1 || variant > 2) return cudaErrorInvalidValue;
+    const int nx = g.hi[0] - g.lo[0], ny = g.hi[1] - g.lo[1];
+    const long long resident = 148LL * (prec64 ? 2 : 4);
+    auto blocks = [&](int tx, int ty) { return (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty); };
+    if (blocks(16, 7) <= resident) return launch_tile2d_small(1, scheme, flux, prec64, g, sv, st);
+    if (blocks(32, 7) <= resident) return launch_tile2d_small(2, scheme, flux, prec64, g, sv, st);
+    if (variant == 2) return launch_tile_p<22, 22>(prec64, scheme, flux, g, sv, st);
+    return launch_tile_p<32, 15>(prec64, scheme, flux, g, sv, st);
 }
 
 }  // namespace sfg
