@@ -29,8 +29,11 @@ namespace sfg {
 // ---------------------------------------------------------------------------
 // x sweep: blockDim = (32, ROWS); one warp per 31 nodes of one row.
 // ---------------------------------------------------------------------------
+// 5 blocks per SM (96 registers); WENO7 in FP64 4 (its seven projected
+// differences spill 0.8 KB a face at 96).
 template <int SCHEME, int FLUX, typename T>
-__global__ void __launch_bounds__(128, 5) sweep_x(GridView g, StageView sv) {
+__global__ void __launch_bounds__(128, SCHEME == WENO7 && sizeof(T) == sizeof(double) ? 4 : 5)
+    sweep_x(GridView g, StageView sv) {
     constexpr int NST = SchemeInfo<SCHEME>::NST;
     if (sv.require_active && !sv.clock->active) return;
     const int lane = threadIdx.x;
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(128, 5) sweep_x(GridView g, StageView sv) {
 }
 
 // ---------------------------------------------------------------------------
-// y / z sweep: blockDim = (32, SEGS); thread = (x node, segment of SEGLEN
+// y / z sweep: blockDim = (32, SEGS); thread = (x node, segment of seglen
 // nodes along AX); blockIdx.z = the remaining axis.
 // ---------------------------------------------------------------------------
 constexpr int SEGLEN = 16;
@@ -111,11 +114,11 @@ constexpr int SEGLEN = 16;
 // segments.  The FP64 node value for the stage update is re-read (L1 / L2).
 template <int AX, int SCHEME, int FLUX>
 __device__ __forceinline__ void sweep_yz_f32_segment(const GridView& g, const StageView& sv, int i, int o, int s0,
-                                                     unsigned& flags, unsigned& cut, unsigned& cores,
+                                                     int seglen, unsigned& flags, unsigned& cut, unsigned& cores,
                                                      double& sr_max) {
     constexpr int NST = SchemeInfo<SCHEME>::NST;
     constexpr int OTHER = AX == 1 ? 2 : 1;
-    const int s1 = min(s0 + SEGLEN, g.hi[AX]);
+    const int s1 = min(s0 + seglen, g.hi[AX]);
     const long long vs = g.vs;
     const long long sy = g.n[0], sz = (long long)g.n[0] * g.n[1];
     const long long sa = AX == 1 ? sy : sz;
@@ -176,36 +179,55 @@ __device__ __forceinline__ void sweep_yz_f32_segment(const GridView& g, const St
 }
 
 template <int AX, int SCHEME, int FLUX, typename T>
-__global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv) {
+__global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv, int seglen) {
     constexpr int NST = SchemeInfo<SCHEME>::NST;
     if (sv.require_active && !sv.clock->active) return;
     constexpr int OTHER = AX == 1 ? 2 : 1;
     const int i = g.lo[0] + blockIdx.x * 32 + threadIdx.x;
     const int o = g.lo[OTHER] + blockIdx.z;
-    const int s0 = g.lo[AX] + (blockIdx.y * blockDim.y + threadIdx.y) * SEGLEN;
+    const int s0 = g.lo[AX] + (blockIdx.y * blockDim.y + threadIdx.y) * seglen;
     const bool live = i < g.hi[0] && s0 < g.hi[AX];
     unsigned flags = 0, cut = 0, cores = 0;
     double sr = 0.0;
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (live) sweep_yz_f32_segment<AX, SCHEME, FLUX>(g, sv, i, o, s0, flags, cut, cores, sr);
+        if (live) sweep_yz_f32_segment<AX, SCHEME, FLUX>(g, sv, i, o, s0, seglen, flags, cut, cores, sr);
     } else if (live) {
-        const int s1 = min(s0 + SEGLEN, g.hi[AX]);
+        // FP64: a face's points are read again for every face (the five planes
+        // that the previous face read are in L1), because a register window of
+        // NST x 5 doubles beside the face's projected differences spills: 1 KB of
+        // local stores a face at 128 registers.  The new plane of the next face is
+        // loaded ahead, before this face's arithmetic.  One stage at 128^3, WENO5:
+        // y 149 -> 137 us, z 183 -> 156 us (FP64 pipe 51-56 %, then load latency).
+        const int s1 = min(s0 + seglen, g.hi[AX]);
         const long long vs = g.vs;
         const long long sx = 1, sy = g.n[0], sz = (long long)g.n[0] * g.n[1];
         const long long sa = AX == 1 ? sy : sz;
-        const long long base = i * sx + (long long)o * (OTHER == 1 ? sy : sz);
+        const double* qs = sv.qs + (i * sx + (long long)o * (OTHER == 1 ? sy : sz));
+        const long long base = qs - sv.qs;
         const int n = g.n[AX];
         const int bl = g.bc_lo[AX], bh = g.bc_hi[AX];
         const double dt = sv.clock->dt;
-        double st[NST][5];
+        double Fp[5], next[5];
+        {
+            const double* at = qs + map_index(s0 + NST / 2 - 1, n, bl, bh) * sa;
 #pragma unroll
-        for (int s = 0; s < NST; ++s) {
-            const int a = map_index(s0 - NST / 2 + s, n, bl, bh);
-#pragma unroll
-            for (int v = 0; v < 5; ++v) st[s][v] = sv.qs[v * vs + base + a * sa];
+            for (int v = 0; v < 5; ++v) next[v] = __ldg(at + v * vs);
         }
-        double Fp[5];
         for (int f = s0; f <= s1; ++f) {
+            double st[NST][5], qn[5];
+#pragma unroll
+            for (int s = 0; s < NST - 1; ++s) {
+                const double* at = qs + map_index(f - NST / 2 + s, n, bl, bh) * sa;
+#pragma unroll
+                for (int v = 0; v < 5; ++v) st[s][v] = __ldg(at + v * vs);
+            }
+#pragma unroll
+            for (int v = 0; v < 5; ++v) st[NST - 1][v] = next[v];
+            {
+                const double* at = qs + map_index(min(f + NST / 2, s1 + NST / 2 - 1), n, bl, bh) * sa;
+#pragma unroll
+                for (int v = 0; v < 5; ++v) next[v] = __ldg(at + v * vs);
+            }
             T Ft[5];
             face_flux<AX, SCHEME, FLUX, T>(st, T(g.gamma), Ft, flags, cut,
                                            T(FLUX == LAXW ? sv.clock->dt / g.h[AX] : 0.0));
@@ -223,9 +245,8 @@ __global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv) {
                     for (int v = 0; v < 5; ++v) div[v] = sv.r[v * vs + node] + div[v];
                 }
                 if (sv.mode & MODE_FINAL) {
-                    double qn[5];
 #pragma unroll
-                    for (int v = 0; v < 5; ++v) qn[v] = st[NST / 2 - 1][v];
+                    for (int v = 0; v < 5; ++v) qn[v] = __ldg(sv.qs + v * vs + node);
                     finish_node(g, sv, dt, node, qn, div, flags, sr);
                 } else {
 #pragma unroll
@@ -234,15 +255,6 @@ __global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv) {
             }
 #pragma unroll
             for (int v = 0; v < 5; ++v) Fp[v] = F[v];
-            if (f < s1) {
-#pragma unroll
-                for (int s = 0; s < NST - 1; ++s)
-#pragma unroll
-                    for (int v = 0; v < 5; ++v) st[s][v] = st[s + 1][v];
-                const int a = map_index(f + 1 - NST / 2 + NST - 1, n, bl, bh);
-#pragma unroll
-                for (int v = 0; v < 5; ++v) st[NST - 1][v] = sv.qs[v * vs + base + a * sa];
-            }
         }
     }
     flush_status(sv, flags, cores, cut);
@@ -404,6 +416,22 @@ __global__ void totals_kernel(GridView g, const double* __restrict__ q, double* 
 // Launchers
 // ---------------------------------------------------------------------------
 
+// y / z sweep blocks for segments of `seglen` nodes, and the faces one of them
+// computes in turn times the rounds of resident blocks (4 per SM): a sweep
+// lasts about that long.  Large grids keep SEGLEN (one face in 17 is computed
+// twice); a grid of few segments takes shorter ones: 97 x 83 x 61 has 354 (y)
+// and 243 (z) blocks of 16-node segments for 592 resident ones, and WENO7
+// stages of 229 and 214 us; with 8 nodes 531 and 486 blocks, 78 and 79 us
+// (together with the WENO7 core).
+static dim3 sweep_grid(const GridView& g, int axis, int other, int seglen) {
+    const int segs = (g.hi[axis] - g.lo[axis] + seglen - 1) / seglen;
+    return dim3((g.hi[0] - g.lo[0] + 31) / 32, (segs + 3) / 4, g.hi[other] - g.lo[other]);
+}
+static long long sweep_faces(const dim3& grid, int seglen) {
+    const long long blocks = (long long)grid.x * grid.y * grid.z, resident = 148 * 4;
+    return (blocks + resident - 1) / resident * (seglen + 1);
+}
+
 template <int SCHEME, int FLUX, typename T>
 static cudaError_t launch_axis(int axis, const GridView& g, const StageView& sv, cudaStream_t st) {
     if (axis == 0) {
@@ -413,11 +441,18 @@ static cudaError_t launch_axis(int axis, const GridView& g, const StageView& sv,
         sweep_x<SCHEME, FLUX, T><<<grid, block, 0, st>>>(g, sv);
     } else {
         const int other = axis == 1 ? 2 : 1;
-        const int segs = (g.hi[axis] - g.lo[axis] + SEGLEN - 1) / SEGLEN;
         dim3 block(32, 4);
-        dim3 grid((g.hi[0] - g.lo[0] + 31) / 32, (segs + 3) / 4, g.hi[other] - g.lo[other]);
-        if (axis == 1) sweep_yz<1, SCHEME, FLUX, T><<<grid, block, 0, st>>>(g, sv);
-        else sweep_yz<2, SCHEME, FLUX, T><<<grid, block, 0, st>>>(g, sv);
+        int seglen = SEGLEN;
+        dim3 grid = sweep_grid(g, axis, other, seglen);
+        for (int s = SEGLEN / 2; s >= 2; s /= 2) {
+            const dim3 shorter = sweep_grid(g, axis, other, s);
+            if (sweep_faces(shorter, s) < sweep_faces(grid, seglen)) {
+                seglen = s;
+                grid = shorter;
+            }
+        }
+        if (axis == 1) sweep_yz<1, SCHEME, FLUX, T><<<grid, block, 0, st>>>(g, sv, seglen);
+        else sweep_yz<2, SCHEME, FLUX, T><<<grid, block, 0, st>>>(g, sv, seglen);
     }
     return cudaGetLastError();
 }
