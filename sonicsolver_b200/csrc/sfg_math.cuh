@@ -425,7 +425,7 @@ template <> struct Teno<float> {
 };
 
 // ---------------------------------------------------------------------------
-// FP64 WENO5 / TENO5 on a face's six points in differences.  With the
+// FP64 WENO5 / TENO5 on a face's six points (WENO7: eight) in differences.  With the
 // characteristic first differences W_i = c_{i+1} - c_i (i = 0..4) and second
 // differences t_i = W_{i+1} - W_i (centred on the points 1..4), and the
 // reconstructions taken relative to the midpoint (c_2 + c_3) / 2:
@@ -490,6 +490,71 @@ __device__ __forceinline__ void weno5_pair64(const double (&W)[5], double& dl, d
     const double r = mul_rn(inv, 1.0 / 6.0);
     dl = mul_rn(mul_rn(num[0], den[1]), r);
     dr = mul_rn(mul_rn(num[1], den[0]), r);
+}
+
+// WENO7-JS (SF_WENO7.cpp:41-98) in the same form, from the seven projected
+// differences W_i of eight points, t_i = W_i - W_{i-1}, G_i = t_{i+1} - t_i.
+// The indicator of a sub-stencil is the integral over the cell of its cubic's
+// squared derivatives; with the cubic written about the cell's centre it is a
+// sum of squares,
+//   b_k = (a + G/24)^2 + 13/12 b^2 + 781/720 G^2,
+// a, b the first and second derivative at the point nearest the face and G the
+// third difference, so the G^2 and t^2 terms are shared by the two sides:
+//   left  a + G/24: W2 + t2/2 + 3/8 G1, (W2 + W3)/2 - G2/8, (W2 + W3)/2 - G3/8, W3 - t4/2 + 3/8 G4
+//   right (signs dropped): W4 - t5/2 + 3/8 G5, (W3 + W4)/2 - G4/8, (W3 + W4)/2 - G3/8, W3 + t3/2 + 3/8 G2
+//   12 (p_k - mid) left: -3 t1 + 7 t2 - 6 t3, t2 - 3 t3, -(t3 + t4), t5 - 3 t4 (right mirrored)
+// One division a side, the weights folded as products of the other three
+// s_j = (eps + b_j)^2 (the point form takes five: about 135 FP64 operations a
+// field against 350; an x sweep of 97 x 83 x 61 nodes 131 -> 54 us).  When that product leaves FP64 range (differences above
+// 1e25) the side falls back to the point form.
+static __device__ __noinline__ double weno7_far(const double* W, int right, unsigned* flags) {
+    double c[8], v[7];
+    c[0] = 0.0;
+    for (int i = 0; i < 7; ++i) c[i + 1] = c[i] + W[i];
+    for (int i = 0; i < 7; ++i) v[i] = right ? c[7 - i] : c[i];
+    return weno7_core<double>(v, *flags) - 0.5 * (c[3] + c[4]);
+}
+
+__device__ __forceinline__ void weno7_pair64(const double (&W)[7], double& dl, double& dr, unsigned& flags) {
+    double t[7], G[6], q[6];  // t[1..6], G[1..5], q = 781/720 G^2 + eps
+#pragma unroll
+    for (int i = 1; i < 7; ++i) t[i] = add_rn(W[i], -W[i - 1]);
+#pragma unroll
+    for (int i = 1; i < 6; ++i) {
+        G[i] = add_rn(t[i + 1], -t[i]);
+        q[i] = fma(mul_rn(781.0 / 720.0, G[i]), G[i], 1e-6);
+    }
+    const double c13 = 13.0 / 12.0;
+    const double u3 = mul_rn(mul_rn(c13, t[3]), t[3]), u4 = mul_rn(mul_rn(c13, t[4]), t[4]);
+    const double m23 = mul_rn(0.5, add_rn(W[2], W[3])), m34 = mul_rn(0.5, add_rn(W[3], W[4]));
+    const double x0 = add_rn(t[2], G[1]), x3 = add_rn(t[4], -G[4]);  // second derivatives of the outer left cubics
+    const double y0 = add_rn(t[5], -G[5]), y3 = add_rn(t[3], G[2]);  // and of the right ones
+    auto sq = [](double a, double b) { return fma(a, a, b); };
+    const double el[4] = {sq(fma(0.375, G[1], fma(0.5, t[2], W[2])), fma(mul_rn(c13, x0), x0, q[1])),
+                          sq(fma(-0.125, G[2], m23), add_rn(u3, q[2])), sq(fma(-0.125, G[3], m23), add_rn(u3, q[3])),
+                          sq(fma(0.375, G[4], fma(-0.5, t[4], W[3])), fma(mul_rn(c13, x3), x3, q[4]))};
+    const double er[4] = {sq(fma(0.375, G[5], fma(-0.5, t[5], W[4])), fma(mul_rn(c13, y0), y0, q[5])),
+                          sq(fma(-0.125, G[4], m34), add_rn(u4, q[4])), sq(fma(-0.125, G[3], m34), add_rn(u4, q[3])),
+                          sq(fma(0.375, G[2], fma(0.5, t[3], W[3])), fma(mul_rn(c13, y3), y3, q[2]))};
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const double* e = side ? er : el;
+        const double s0 = mul_rn(e[0], e[0]), s1 = mul_rn(e[1], e[1]), s2 = mul_rn(e[2], e[2]), s3 = mul_rn(e[3], e[3]);
+        const double s01 = mul_rn(s0, s1), s23 = mul_rn(s2, s3);
+        const double w0 = mul_rn(s1, s23), w1 = mul_rn(s0, s23), w2 = mul_rn(s3, s01), w3 = mul_rn(s2, s01);
+        const double den = fma(4.0, w3, fma(18.0, w2, fma(12.0, w1, w0)));  // weights 1 : 12 : 18 : 4
+        const double ta = side ? t[6] : t[1], tb = side ? t[5] : t[2], tc = side ? t[4] : t[3], td = side ? t[3] : t[4],
+                     te = side ? t[2] : t[5];
+        const double p0 = fma(-6.0, tc, fma(7.0, tb, mul_rn(-3.0, ta)));
+        const double p1 = fma(-3.0, tc, tb), p2 = add_rn(tc, td), p3 = fma(-3.0, td, te);
+        const double num = fma(w0, p0, fma(mul_rn(12.0, w1), p1, fma(mul_rn(-18.0, w2), p2, mul_rn(mul_rn(4.0, w3), p3))));
+        const double inv = 1.0 / den;
+        double x = mul_rn(mul_rn(num, 1.0 / 12.0), inv);
+        // 1 / den positive and normal, the quotient finite: else out of range (or not finite)
+        if ((unsigned)(__double2hiint(inv) - 0x00100000) >= 0x7fe00000u || hi_abs(x) >= 0x7ff00000)
+            x = weno7_far(W, side, &flags);
+        (side ? dr : dl) = x;
+    }
 }
 
 // The smooth-stencil test on the indicators e_k = 4 b_k + eps of one side:
@@ -797,19 +862,20 @@ __device__ __forceinline__ void flux_of(const T (&ql)[5], const T (&qr)[5], T ga
     else laxw<AX, T>(ql, qr, gamma, lam, F, flags);
 }
 
-// FP64 WENO5 / TENO5 face: the five state differences are projected, not the
-// six points, and the face states are q-bar + R (deltas).
+// FP64 face of WENO5 / TENO5 / WENO7: the state differences are projected, not
+// the points, and the face states are q-bar + R (deltas).
 template <int AX, int SCHEME, int FLUX>
-__device__ __forceinline__ void face_flux64(const double (&st)[6][5], double gamma, double F[5], unsigned& flags,
-                                            unsigned& cut, double lam) {
+__device__ __forceinline__ void face_flux64(const double (&st)[SchemeInfo<SCHEME>::NST][5], double gamma, double F[5],
+                                            unsigned& flags, unsigned& cut, double lam) {
+    constexpr int ND = SchemeInfo<SCHEME>::NST - 1, CL = ND / 2;
     double qbar[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) qbar[v] = 0.5 * (st[2][v] + st[3][v]);
+    for (int v = 0; v < 5; ++v) qbar[v] = 0.5 * (st[CL][v] + st[CL + 1][v]);
     Eigen<double> e;
     if (!eigen_at<AX, double>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
-    double W[5][5];
+    double W[ND][5];
 #pragma unroll
-    for (int s = 0; s < 5; ++s) {
+    for (int s = 0; s < ND; ++s) {
         double d[5];
 #pragma unroll
         for (int v = 0; v < 5; ++v) d[v] = add_rn(st[s + 1][v], -st[s][v]);
@@ -818,9 +884,12 @@ __device__ __forceinline__ void face_flux64(const double (&st)[6][5], double gam
     double wl[5], wr[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        const double w[5] = {W[0][v], W[1][v], W[2][v], W[3][v], W[4][v]};
+        double w[ND];
+#pragma unroll
+        for (int s = 0; s < ND; ++s) w[s] = W[s][v];
         if constexpr (SCHEME == WENO5) weno5_pair64(w, wl[v], wr[v], flags);
-        else teno5_pair64(w, wl[v], wr[v], flags, cut);
+        else if constexpr (SCHEME == TENO5) teno5_pair64(w, wl[v], wr[v], flags, cut);
+        else weno7_pair64(w, wl[v], wr[v], flags);
     }
     double ql[5], qr[5];
     back_project64<AX>(e, qbar, wl, ql);
@@ -836,7 +905,7 @@ __device__ __forceinline__ void face_flux64(const double (&st)[6][5], double gam
 template <int AX, int SCHEME, int FLUX, typename T>
 __device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>::NST][5], T gamma, T F[5],
                                           unsigned& flags, unsigned& cut, T lam = T(0)) {
-    if constexpr (sizeof(T) == sizeof(double) && (SCHEME == WENO5 || SCHEME == TENO5)) {
+    if constexpr (sizeof(T) == sizeof(double) && SCHEME != WENO3) {
         face_flux64<AX, SCHEME, FLUX>(st, gamma, F, flags, cut, lam);
         return;
     }

@@ -7,7 +7,7 @@ from sonicsolver_b200 import capi, cases
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_FP32_FLUX])
-@pytest.mark.parametrize("recipe", ["weno3Rusanov", "weno5Roe", "teno5Rusanov"])
+@pytest.mark.parametrize("recipe", ["weno3Rusanov", "weno5Roe", "teno5Rusanov", "weno7Rusanov"])
 @pytest.mark.parametrize("n", [(9, 9), (16, 7), (17, 8), (33, 15), (34, 16), (255, 120), (320, 200), (640, 300)])
 def test_small_tiles_give_the_bits_of_the_large(n, recipe, precision):
     """Grids on both sides of the tile-shape rule's lines, and of one tile's
