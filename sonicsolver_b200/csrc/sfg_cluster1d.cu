@@ -1,5 +1,5 @@
 // sfg_cluster1d.cu -- whole runs of small 1-D grids in one launch: a single
-// thread-block cluster of CL_CTAS CTAs steps the grid from sfg_advance's
+// thread-block cluster of 16 (or 8) CTAs steps the grid from sfg_advance's
 // start to its end time (or step limit) without returning to the host, with
 // the state held in the cluster's distributed shared memory.
 //
@@ -13,8 +13,8 @@
 //   * a face stencil reads its nodes from the owning CTA's shared memory
 //     (its own, or a neighbour's through distributed shared memory);
 //   * one lane computes one face; the upper face of a node comes from the
-//     next lane by a warp shuffle, so a warp of 32 faces finishes 31 nodes
-//     (the face at a warp boundary is computed by both warps);
+//     next lane by a warp shuffle, so a warp of 32 faces finishes up to 31
+//     nodes (the face at a warp boundary is computed by both warps);
 //   * one hardware cluster barrier (barrier.cluster: release / acquire at
 //     cluster scope) closes each stage; the last stage of a step also
 //     publishes each CTA's CFL maximum and status bits into CTA 0's shared
@@ -38,11 +38,13 @@ namespace cg = cooperative_groups;
 
 namespace sfg {
 
-constexpr int CL_CTAS = 8;
-constexpr int CL_THREADS = 256;
-constexpr int CL_WARPS = CL_THREADS / 32;
-constexpr int CL_MAX_NODES = 8192;  // per CTA 1024 nodes: 4 buffers x 5 x 1024 doubles = 160 KB
-constexpr int CL_NODES_PER_PASS = CL_WARPS * 31;
+constexpr int CL_CTAS_MAX = 16;     // a cluster of 16 (opt-in size), or of 8 where 16 cannot be placed
+constexpr int CL_WARPS_MAX = 8;
+// One pass of eight warps (248 nodes) in each of 16 CTAs.  Beyond it a stage
+// takes two passes and the graph path is faster (us a step, cluster / graph:
+// WENO5 3000 nodes 12.2 / 19.8, 4000 19.9 / 20.1, 6000 20.9 / 20.3; WENO7 3000
+// 17.0 / 24.5, 4000 29.3 / 24.7; TENO5 3000 16.7 / 23.4, 4000 24.8 / 23.4).
+constexpr int CL_MAX_NODES = CL_CTAS_MAX * 31 * CL_WARPS_MAX;
 
 namespace {
 
@@ -68,15 +70,23 @@ __host__ __device__ __forceinline__ int buffer_count(int time_id) {
 
 }  // namespace
 
-template <int SCHEME, int FLUX>
-__global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS)
+// A stage lasts as long as the FP64 chain of one warp of faces (about 1400
+// instructions), and two warps on one SM sub-partition take turns on its FP64
+// pipe.  So the cluster is as wide as it gets, and a CTA's nodes are dealt
+// evenly to four warps, one a sub-partition, when they fit (124 nodes), else to
+// eight.  WENO5, us a step, 8 CTAs with full warps of 31 nodes -> 16 CTAs: 1001
+// nodes 11.8 -> 10.8, 3000 23.8 -> 12.2.
+template <int CTAS, int SCHEME, int FLUX>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(CL_WARPS_MAX * 32)
     cluster1d_kernel(GridView g, ClusterRun run) {
     constexpr int NST = SchemeInfo<SCHEME>::NST;
+    constexpr int CL_CTAS = CTAS;
+    const int CL_THREADS = blockDim.x, CL_WARPS = blockDim.x >> 5;
     extern __shared__ double cl_smem[];                 // [buffer][5][per]
     __shared__ double slots[2][CL_CTAS];                // CFL maxima (in CTA 0), by step parity
     __shared__ unsigned fslots[2][CL_CTAS];             // status bits (in CTA 0)
-    __shared__ double warp_max[CL_WARPS];
-    __shared__ unsigned warp_flags[CL_WARPS];
+    __shared__ double warp_max[CL_WARPS_MAX];
+    __shared__ unsigned warp_flags[CL_WARPS_MAX];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -166,7 +176,10 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS)
     bool more = false;  // stopped by the per-launch step bound, not by the run's end
     int parity = 0;     // Euler: buffer holding the current state
     unsigned cores = 0, cut = 0;
-    const int passes = s1 > s0 ? (s1 - s0 + CL_NODES_PER_PASS - 1) / CL_NODES_PER_PASS : 0;
+    // nodes of a warp per pass: the CTA's dealt evenly, at most 31 (its faces are one more)
+    const int share = min(31, max(1, (s1 - s0 + CL_WARPS - 1) / CL_WARPS));
+    const int per_pass = share * CL_WARPS;
+    const int passes = s1 > s0 ? (s1 - s0 + per_pass - 1) / per_pass : 0;
     for (int it = 0;; ++it) {
         // finalize_dt_kernel
         const double remaining = c.t_end - c.t;
@@ -196,29 +209,33 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS)
             sv.mode = MODE_FINAL | (s == run.stages - 1 ? MODE_CFL : 0);
             const double* in_local = cl_smem + bin * bstride;
             for (int p = 0; p < passes; ++p) {
-                const int f = s0 + p * CL_NODES_PER_PASS + warp * 31 + lane;  // face f: lower face of node f
+                const int f0 = s0 + p * per_pass + warp * share;
+                const int f = f0 + lane;  // face f: lower face of node f
+                const int fend = min(s1, f0 + share);
                 double Fa[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-                if (f <= s1) {
+                if (f <= fend && f0 < s1) {
                     double st[NST][5];
 #pragma unroll
                     for (int k = 0; k < NST; ++k) {
                         const int j = map_index(f - NST / 2 + k, n, g.bc_lo[0], g.bc_hi[0]);
-                        const int owner = j / per;
-                        const double* src =
-                            owner == rank ? in_local : cluster.map_shared_rank(in_local, owner);
+                        const double* src = in_local + (j - c0);
+                        if ((unsigned)(j - c0) >= (unsigned)(c1 - c0)) {  // a neighbour's node
+                            const int owner = j / per;
+                            src = cluster.map_shared_rank(in_local, owner) + (j - owner * per);
+                        }
 #pragma unroll
-                        for (int v = 0; v < 5; ++v) st[k][v] = src[v * per + (j - owner * per)];
+                        for (int v = 0; v < 5; ++v) st[k][v] = src[v * per];
                     }
                     double F[5];
                     face_flux<0, SCHEME, FLUX, double>(st, g.gamma, F, flags, cut, 0.0);
 #pragma unroll
                     for (int v = 0; v < 5; ++v) Fa[v] = F[v] * g.area[0];
-                    if (SCHEME == TENO5 && (lane < 31 || f == s1)) cores += 10;
+                    if (SCHEME == TENO5 && (lane < share || f == s1)) cores += 10;
                 }
                 double div[5];
 #pragma unroll
                 for (int v = 0; v < 5; ++v) div[v] = __shfl_down_sync(0xffffffffu, Fa[v], 1) - Fa[v];
-                if (lane < 31 && f < s1) {
+                if (lane < share && f < fend) {
                     const int li = f - c0;
                     double qn[5];
 #pragma unroll
@@ -264,41 +281,55 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS)
     cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-template <int SCHEME, int FLUX>
-static cudaError_t launch_cluster(const GridView& g, const ClusterRun& run, size_t smem, cudaStream_t st) {
-    auto kern = cluster1d_kernel<SCHEME, FLUX>;
+template <int CTAS, int SCHEME, int FLUX>
+static cudaError_t launch_cluster_n(const GridView& g, const ClusterRun& run, cudaStream_t st) {
+    const int per = (g.n[0] + CTAS - 1) / CTAS;
+    const size_t smem = sizeof(double) * 5 * (size_t)per * buffer_count(run.sv[0].time_id);
+    auto kern = cluster1d_kernel<CTAS, SCHEME, FLUX>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<CL_CTAS, CL_THREADS, smem, st>>>(g, run);
+    if (CTAS > 8) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<CTAS, per <= 124 ? 128 : 256, smem, st>>>(g, run);
     return cudaGetLastError();
 }
 
+template <int SCHEME, int FLUX>
+static cudaError_t launch_cluster(const GridView& g, const ClusterRun& run, cudaStream_t st) {
+    // 16 CTAs from 8 nodes each on: below that there is nothing to spread
+    if (g.hi[0] - g.lo[0] >= CL_CTAS_MAX * 8) {
+        const cudaError_t e = launch_cluster_n<CL_CTAS_MAX, SCHEME, FLUX>(g, run, st);
+        if (e == cudaSuccess) return e;
+        (void)cudaGetLastError();  // not placed: nothing ran
+    }
+    return launch_cluster_n<8, SCHEME, FLUX>(g, run, st);
+}
+
 template <int SCHEME>
-static cudaError_t launch_cluster_f(int flux, const GridView& g, const ClusterRun& run, size_t smem,
-                                    cudaStream_t st) {
+static cudaError_t launch_cluster_f(int flux, const GridView& g, const ClusterRun& run, cudaStream_t st) {
     switch (flux) {
-    case RUSANOV: return launch_cluster<SCHEME, RUSANOV>(g, run, smem, st);
-    case ROE: return launch_cluster<SCHEME, ROE>(g, run, smem, st);
-    case STEGER: return launch_cluster<SCHEME, STEGER>(g, run, smem, st);
-    case LAXF: return launch_cluster<SCHEME, LAXF>(g, run, smem, st);
+    case RUSANOV: return launch_cluster<SCHEME, RUSANOV>(g, run, st);
+    case ROE: return launch_cluster<SCHEME, ROE>(g, run, st);
+    case STEGER: return launch_cluster<SCHEME, STEGER>(g, run, st);
+    case LAXF: return launch_cluster<SCHEME, LAXF>(g, run, st);
     }
     return cudaErrorInvalidValue;
 }
 
 // Whether a 1-D grid can run in the cluster kernel.
 bool cluster1d_eligible(const GridView& g, int flux, int prec64) {
-    return g.dim == 1 && prec64 && flux != LAXW && !g.curv && g.hi[0] - g.lo[0] >= CL_CTAS &&
+    return g.dim == 1 && prec64 && flux != LAXW && !g.curv && g.hi[0] - g.lo[0] >= 8 &&
            g.n[0] <= CL_MAX_NODES;
 }
 
 cudaError_t launch_cluster1d(int scheme, int flux, const GridView& g, const ClusterRun& run, cudaStream_t st) {
-    const int per = (g.n[0] + CL_CTAS - 1) / CL_CTAS;
-    const size_t smem = sizeof(double) * 5 * (size_t)per * buffer_count(run.sv[0].time_id);
     switch (scheme) {
-    case WENO5: return launch_cluster_f<WENO5>(flux, g, run, smem, st);
-    case TENO5: return launch_cluster_f<TENO5>(flux, g, run, smem, st);
-    case WENO3: return launch_cluster_f<WENO3>(flux, g, run, smem, st);
-    case WENO7: return launch_cluster_f<WENO7>(flux, g, run, smem, st);
+    case WENO5: return launch_cluster_f<WENO5>(flux, g, run, st);
+    case TENO5: return launch_cluster_f<TENO5>(flux, g, run, st);
+    case WENO3: return launch_cluster_f<WENO3>(flux, g, run, st);
+    case WENO7: return launch_cluster_f<WENO7>(flux, g, run, st);
     }
     return cudaErrorInvalidValue;
 }

@@ -7,34 +7,43 @@ namespace sfg {
 cudaError_t launch_tile2d_small(int rounds, int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
                                 cudaStream_t st);
 
-// 1-D grids: one block per 511-node tile (the body the batched kernels use,
-// so a 1-D grid gives the same bits alone and in a batch).
-template <int SCHEME, int FLUX, typename T>
+// 1-D grids: one block per T1-node tile (the body the batched kernels use, so a
+// 1-D grid gives the same bits alone and in a batch): 511 nodes, two rounds of
+// faces, or 255 and one round while the blocks then still fit the GPU at once
+// (a stage then lasts as long as one block's rounds).
+template <int SCHEME, int FLUX, typename T, int T1>
 __global__ void __launch_bounds__(TILE_THREADS) tile1d_kernel(GridView g, StageView sv) {
     extern __shared__ __align__(16) unsigned char smem1[];
     if (sv.require_active && !sv.clock->active) return;
     unsigned flags = 0, cut = 0, cores = 0;
     double sr = 0.0;
-    tile1d_body<SCHEME, FLUX, T>(g, sv, g.lo[0] + blockIdx.x * TILE1D, reinterpret_cast<T*>(smem1), flags, cut,
-                                 cores, sr);
+    tile1d_body<SCHEME, FLUX, T, T1>(g, sv, g.lo[0] + blockIdx.x * T1, reinterpret_cast<T*>(smem1), flags, cut,
+                                     cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
     if (sv.mode & MODE_STEP) step_tail(sv);
 }
 
-template <int SCHEME, int FLUX, typename T>
-static cudaError_t launch_tile1(const GridView& g, const StageView& sv, cudaStream_t st) {
-    constexpr size_t smem = sizeof(T) * Tile1Shape<SCHEME>::ELEMS;
+template <int SCHEME, int FLUX, typename T, int T1>
+static cudaError_t launch_tile1_n(const GridView& g, const StageView& sv, cudaStream_t st) {
+    constexpr size_t smem = sizeof(T) * Tile1Shape<SCHEME, T1>::ELEMS;
     static std::atomic<unsigned long long> configured{0};
     unsigned long long bit = 0;
-    auto kern = tile1d_kernel<SCHEME, FLUX, T>;
+    auto kern = tile1d_kernel<SCHEME, FLUX, T, T1>;
     if (attributes_pending(configured, bit)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    kern<<<(g.hi[0] - g.lo[0] + TILE1D - 1) / TILE1D, TILE_THREADS, smem, st>>>(g, sv);
+    kern<<<(g.hi[0] - g.lo[0] + T1 - 1) / T1, TILE_THREADS, smem, st>>>(g, sv);
     return cudaGetLastError();
+}
+
+template <int SCHEME, int FLUX, typename T>
+static cudaError_t launch_tile1(const GridView& g, const StageView& sv, cudaStream_t st) {
+    if ((g.hi[0] - g.lo[0] + TILE1D_SHORT - 1) / TILE1D_SHORT <= 2 * 148)
+        return launch_tile1_n<SCHEME, FLUX, T, TILE1D_SHORT>(g, sv, st);
+    return launch_tile1_n<SCHEME, FLUX, T, TILE1D>(g, sv, st);
 }
 
 template <int FLUX, typename T>
