@@ -1,6 +1,6 @@
 // sfg_tile3d.cu -- fused stage kernel for 3-D grids: one launch per stage.
 //
-// A block owns a column of nodes TX x TY (x, y) by up to KZ planes (z) and
+// A block owns a column of nodes TX x TY (x, y) by up to kz planes (z) and
 // marches up the planes.  Per plane k it
 //   1. stages plane k+H of its TX x TY interior into a ring of 2H planes
 //      (the z stencils of the block's columns), and plane k with its x-y halo
@@ -25,7 +25,7 @@
 
 namespace sfg {
 
-constexpr int T3X = 16, T3Y = 15, T3Z = 32;
+constexpr int T3X = 16, T3Y = 15;
 // resident CTAs per SM of the FP32 kernel: 64 registers a thread and 48 KB
 // of shared memory each (with the full shared-memory carveout)
 constexpr int T3_F32_CTAS = 4;
@@ -43,7 +43,7 @@ struct Tile3Shape {
 
 template <int SCHEME, int FLUX, typename T>
 __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_F32_CTAS : 2)
-    tile3d_kernel(GridView g, StageView sv) {
+    tile3d_kernel(GridView g, StageView sv, int kz) {
     using S = Tile3Shape<SCHEME, T>;
     constexpr int NST = S::NST, H = S::H, R = S::R, COL = S::COL, SX = S::SX, SY = S::SY;
     constexpr int NFX = S::NFX, NFY = S::NFY;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
     const int nty = (g.hi[1] - g.lo[1] + T3Y - 1) / T3Y;
     const int bxy = blockIdx.x % (ntx * nty), bz = blockIdx.x / (ntx * nty);
     const int x0 = g.lo[0] + (bxy % ntx) * T3X, y0 = g.lo[1] + (bxy / ntx) * T3Y;
-    const int z0 = g.lo[2] + bz * T3Z, z1 = min(z0 + T3Z, g.hi[2]);
+    const int z0 = g.lo[2] + bz * kz, z1 = min(z0 + kz, g.hi[2]);
     const long long nx = g.n[0], nxy = (long long)g.n[0] * g.n[1], vs = g.vs;
     const int t = threadIdx.x;
     const int ci = t % T3X, cj = t / T3X;  // this thread's column (t < COL)
@@ -242,8 +242,20 @@ static cudaError_t launch_tile3(const GridView& g, const StageView& sv, cudaStre
     }
     const int ntx = (g.hi[0] - g.lo[0] + T3X - 1) / T3X;
     const int nty = (g.hi[1] - g.lo[1] + T3Y - 1) / T3Y;
-    const int ntz = (g.hi[2] - g.lo[2] + T3Z - 1) / T3Z;
-    kern<<<ntx * nty * ntz, TILE_THREADS, smem, st>>>(g, sv);
+    // Planes per block: a launch lasts about (rounds of resident blocks) x
+    // (planes + 2, the 2 for the block's first ring and face).  Large grids
+    // keep 32; a grid whose 32-plane blocks leave SMs without takes shorter ones
+    // (128^3 FP32: 288 blocks for 592 slots; 16 planes make it 576).
+    const int nz = g.hi[2] - g.lo[2], resident = 148 * (sizeof(T) == sizeof(float) ? T3_F32_CTAS : 2);
+    auto cost = [&](int k) {
+        const long long blocks = (long long)ntx * nty * ((nz + k - 1) / k);
+        return (blocks + resident - 1) / resident * (k + 2);
+    };
+    int kz = 32;
+    for (int k = 16; k >= 2; k /= 2)
+        if (cost(k) < cost(kz)) kz = k;
+    const int ntz = (nz + kz - 1) / kz;
+    kern<<<ntx * nty * ntz, TILE_THREADS, smem, st>>>(g, sv, kz);
     return cudaGetLastError();
 }
 
