@@ -403,6 +403,7 @@ struct sfg_batch_s {
     size_t law_items_cap = 0;
     std::vector<LawItem> h_law_items;
     int law_grid = 0;
+    bool items_stale = false;  // grids came or went since publish_items
     BatchCtl* d_ctl = nullptr;
     BatchCtl* h_ctl = nullptr;  // pinned
     double* staging = nullptr;
@@ -529,8 +530,10 @@ void slab_free(sfg_batch_s* b, size_t off, size_t bytes) {
 }
 
 // Rebuilds the tile list of all live instances and publishes it (and the
-// instance count) to device memory.
+// instance count) to device memory.  Grids that join or leave mark it stale
+// (items_stale) and the next step rebuilds it once for all of them.
 int publish_items(sfg_batch_s* b) {
+    b->items_stale = false;
     b->h_items.clear();
     // 1-D tiles of one face round once the live tiles no longer fill the
     // SMs: a drained batch's last grids then take half the time per stage
@@ -1005,8 +1008,8 @@ int sfg_batch_add_laws(sfg_batch b, const sfg_grid_desc* grid, const sfg_numeric
     b->inst_pub[idx] = *grid;
     b->inst_off[idx] = {off[0], off[1], off[2]};
     b->inst_law[idx] = lv;
-    rc = publish_items(b);  // synchronises the stream
-    if (rc) return rc;
+    b->items_stale = true;
+    BCUDA(cudaStreamSynchronize(b->stream));  // the caller's arrays are read
     *slot = idx;
     return SFG_OK;
 }
@@ -1031,19 +1034,21 @@ int sfg_batch_set_write_interval(sfg_batch b, int slot, double write_interval) {
 int sfg_batch_remove(sfg_batch b, int slot) {
     if (!b || slot < 0 || slot >= (int)b->h_inst.size() || !b->h_inst[slot].live)
         return bfail(SFG_ERR_NOT_FOUND, "no live instance in slot %d", slot);
-    BCUDA(cudaStreamSynchronize(b->stream));
     b->h_inst[slot].live = 0;
     const int zero = 0;
     BCUDA(cudaMemcpyAsync(&b->d_inst[slot].live, &zero, sizeof zero, cudaMemcpyHostToDevice, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));  // ordered on the batch's (non-blocking) stream
     slab_free(b, b->inst_offset[slot], b->inst_bytes[slot]);
-    return publish_items(b);
+    b->items_stale = true;
+    return SFG_OK;
 }
 
 int sfg_batch_step(sfg_batch b, int steps, int graph_steps, int* active) {
     sfg::NvtxRange nvtx_("sfg_batch_step");
     if (!b) return bfail(SFG_ERR_ARG, "null batch");
     if (graph_steps <= 0) graph_steps = 16;
+    if (b->items_stale)
+        if (int rc = publish_items(b)) return rc;
     if (!b->graph || b->graph_steps != graph_steps) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -1178,7 +1183,11 @@ int sfg_batch_info(sfg_batch b, size_t* used_bytes, size_t* budget_bytes, int* l
         for (const auto& r : b->h_inst) n += r.live;
         *live = n;
     }
-    if (items) *items = (int)b->h_items.size();
+    if (items) {
+        if (b->items_stale)
+            if (int rc = publish_items(b)) return rc;
+        *items = (int)b->h_items.size();
+    }
     return SFG_OK;
 }
 
