@@ -83,10 +83,8 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(CL_WARPS_MAX * 32
     constexpr int CL_CTAS = CTAS;
     const int CL_THREADS = blockDim.x, CL_WARPS = blockDim.x >> 5;
     extern __shared__ double cl_smem[];                 // [buffer][5][per]
-    __shared__ double slots[2][CL_CTAS];                // CFL maxima (in CTA 0), by step parity
-    __shared__ unsigned fslots[2][CL_CTAS];             // status bits (in CTA 0)
-    __shared__ double warp_max[CL_WARPS_MAX];
-    __shared__ unsigned warp_flags[CL_WARPS_MAX];
+    __shared__ double slots[2][CL_CTAS * CL_WARPS_MAX];     // CFL maxima of every warp of the cluster, by step parity
+    __shared__ unsigned fslots[2][CL_CTAS * CL_WARPS_MAX];  // and their status bits
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -111,40 +109,36 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(CL_WARPS_MAX * 32
         }
     }
 
-    // the CTA's CFL maximum and status bits -> slot `par` of CTA 0 (every
-    // thread calls; visible to the cluster after the next cluster barrier)
+    // largest of the warp's non-negative doubles: high words, then the low words
+    // of those that share the largest
+    auto warp_largest = [](double x) {
+        const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+        const unsigned h = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
+        return __hiloint2double((int)h, (int)l);
+    };
+    // Every warp writes its CFL maximum and status bits into its slot of every
+    // CTA (remote stores, one lane a CTA: nothing waits for them but the next
+    // cluster barrier, and the reads after it are local).
     auto publish = [&](double sr, unsigned fl, int par) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sr = fmax(sr, __shfl_xor_sync(0xffffffffu, sr, o));
+        sr = warp_largest(sr);
         fl = __reduce_or_sync(0xffffffffu, fl);
-        if (lane == 0) {
-            warp_max[warp] = sr;
-            warp_flags[warp] = fl;
+        const int slot = rank * CL_WARPS + warp;
+        if (lane < CL_CTAS) {
+            cluster.map_shared_rank(&slots[par][0], lane)[slot] = sr;
+            cluster.map_shared_rank(&fslots[par][0], lane)[slot] = fl;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double m = warp_max[0];
-            unsigned f = warp_flags[0];
-            for (int w = 1; w < CL_WARPS; ++w) {
-                m = fmax(m, warp_max[w]);
-                f |= warp_flags[w];
-            }
-            cluster.map_shared_rank(&slots[par][0], 0)[rank] = m;
-            cluster.map_shared_rank(&fslots[par][0], 0)[rank] = f;
-            if (f) atomicOr(run.flags, f);
-        }
+        if (lane == 0 && fl) atomicOr(run.flags, fl);
     };
     // after the barrier: the cluster's maximum and status bits (every thread)
     auto gather = [&](int par, double& m, unsigned& f) {
         double x = 0.0;
         unsigned b = 0;
-        if (lane < CL_CTAS) {
-            x = cluster.map_shared_rank(&slots[par][0], 0)[lane];
-            b = cluster.map_shared_rank(&fslots[par][0], 0)[lane];
+        for (int k = lane; k < CL_CTAS * CL_WARPS; k += 32) {
+            x = fmax(x, slots[par][k]);
+            b |= fslots[par][k];
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-        m = x;
+        m = warp_largest(x);
         f = __reduce_or_sync(0xffffffffu, b);
     };
 
@@ -162,6 +156,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(CL_WARPS_MAX * 32
             if (!(r > 0.0) || !isfinite(r)) fl |= FLAG_NONFINITE;  // as dt_kernel
             sr = fmax(sr, r);
         }
+        cluster.sync();  // every CTA of the cluster runs before its shared memory is written
         publish(sr, fl, 1);
     }
     cluster.sync();  // the loaded chunks and the first slots are visible cluster-wide
