@@ -49,9 +49,9 @@ __device__ __forceinline__ void teno_flips_face(const GridView& g, const double*
     for (int v = 0; v < 5; ++v) {
         // FP32: the (left, right) stencil pair through the paired indicators
         // and cut-off of the FP32-flux kernels
-        float2 b2[5], B[3], q[3], keep[3];
-        for (int s = 0; s < 5; ++s) b2[s] = make_float2(c32[s][v], c32[NST - 1 - s][v]);
-        stencil5x2(b2, B, q);
+        float2 b2[3], B[3], q[3], keep[3];
+        for (int s = 0; s < 3; ++s) b2[s] = make_float2(c32[s][v], c32[NST - 1 - s][v]);
+        stencil5m2(b2[0], b2[1], b2[2], B, q);
         float2 bad = make_float2(0.f, 0.f);
         teno_keep32x2(B[0], B[1], B[2], keep, bad);
         flag_bad(bad, fl);

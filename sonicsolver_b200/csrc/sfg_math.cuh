@@ -387,17 +387,19 @@ __device__ __forceinline__ void teno_keep32x2(float2 b0, float2 b1, float2 b2, f
 
 // A smooth stencil pair keeps every sub-stencil, which the cut-off would
 // find only after its reciprocals: with tau = |B0 - B2| <= 4 e_min (e_min =
-// min B + eps <= 1e30) in both lanes, t = e_min / (e_min + tau) >= 0.2 up to
+// min B + eps) in both lanes, t = e_min / (e_min + tau) >= 0.2 up to
 // a few ulps, every x_k >= t, so G_k >= 6.39e-5 > 2 lim (lim = 1e-5 sum G <=
-// 3.0001e-5): teno_keep32x2 would return k = 1 for all three.  The test
-// fails for NaN or infinite indicators (they take the cut-off path and its
-// non-finite watch), and a pair that passes has finite differences, so the
-// weights computed with k = 1 are the cut-off path's to the bit.
+// 3.0001e-5): teno_keep32x2 would return k = 1 for all three.  (Where e_min +
+// tau is beyond 8.5e37 its reciprocal is 0 and so are t, every x_k and lim: k
+// = 1 for all three too.)  The test fails for NaN or infinite indicators (they
+// take the cut-off path and its non-finite watch), and a pair that passes has
+// finite differences, so the weights computed with k = 1 are the cut-off
+// path's to the bit.
 __device__ __forceinline__ bool teno_smooth2(const float2 (&B)[3]) {
     const float2 em = add2(f2(fminf(B[0].x, fminf(B[1].x, B[2].x)), fminf(B[0].y, fminf(B[1].y, B[2].y))),
                            f2(TENO32_EPS));
     const float2 d02 = sub2(B[0], B[2]);
-    return fabsf(d02.x) <= 4.f * em.x && fabsf(d02.y) <= 4.f * em.y && em.x <= 1e30f && em.y <= 1e30f;
+    return fabsf(d02.x) <= 4.f * em.x && fabsf(d02.y) <= 4.f * em.y;
 }
 
 template <> struct Teno<float> {
@@ -971,9 +973,16 @@ __device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>:
 // The indicators are returned as B_k / 3 = 4 b_k = 13/3 t_k^2 + r_k^2 (one
 // multiply fewer than 12 b_k) and the epsilons are scaled with them, which
 // leaves every weight unchanged; only differences of the stencil are rounded.
-__device__ __forceinline__ void stencil5x2(const float2* v, float2 (&B)[3], float2 (&q)[3]) {
-    const float2 D0 = sub2(v[1], v[0]), D1 = sub2(v[2], v[1]), D2 = sub2(v[3], v[2]), D3 = sub2(v[4], v[3]);
-    const float2 t0 = sub2(D1, D0), t1 = sub2(D2, D1), t2 = sub2(D3, D2);
+//
+// Left c0..c4 and right c5..c1 come as the point pairs v0 = (c0, c5), v1 = (c1,
+// c4), v2 = (c2, c3): D2 = (d, -d) with d = c3 - c2 and D3 = -swap(D1), so
+// t2 = swap(t1), exactly (three operations and two moves a field fewer than
+// forming them).
+__device__ __forceinline__ void stencil5m2(float2 v0, float2 v1, float2 v2, float2 (&B)[3], float2 (&q)[3]) {
+    const float2 D0 = sub2(v1, v0), D1 = sub2(v2, v1);
+    const float d = v2.y - v2.x;
+    const float2 D2 = f2(d, -d);
+    const float2 t0 = sub2(D1, D0), t1 = sub2(D2, D1), t2 = swap2(t1);
     const float2 r0 = fma2(f2(2.f), D1, t0), r1 = add2(D1, D2), r2 = fma2(f2(-2.f), D2, t2);
     const float2 c = f2(13.f / 3.f);
     B[0] = fma2(mul2(c, t0), t0, mul2(r0, r0));
@@ -1005,17 +1014,18 @@ __device__ __forceinline__ float teno5_all_kept() {
 // indicators, the cut-off (teno_keep32x2) and the weights.  With `count` (a
 // launch-uniform switch: the cut-off accounting of sfg_set_counting), `kept`
 // accumulates the kept sub-stencils of each lane; `all`: teno5_all_kept().
-__device__ __forceinline__ float2 teno5_core2(const float2* v, float2& bad, bool count, float2& kept, float all) {
+__device__ __forceinline__ float2 teno5_core2(float2 v0, float2 v1, float2 v2, float2& bad, bool count,
+                                              float2& kept, float all) {
     float2 B[3], q[3], k[3];
-    stencil5x2(v, B, q);
+    stencil5m2(v0, v1, v2, B, q);
     if (warp_all(teno_smooth2(B))) {
         if (count) kept = add2(kept, f2(3.f));
         const float2 num = fma2(f2(0.1f), q[0], fma2(f2(0.6f), q[1], mul2(f2(0.3f), q[2])));
-        return fma2(num, f2(all), v[2]);
+        return fma2(num, f2(all), v2);
     }
     teno_keep32x2(B[0], B[1], B[2], k, bad);
     if (count) kept = add2(kept, add2(add2(k[0], k[1]), k[2]));
-    return teno5_weights2(k, q, v[2]);
+    return teno5_weights2(k, q, v2);
 }
 
 // FP32 WENO5 / TENO5 on a face's six points in differences, the left and right
@@ -1346,8 +1356,7 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[6][5], const 
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
             // left stencil c0..c4 and right stencil c5..c1 as one paired stencil
-            const float2 st[5] = {P[0][v], P[1][v], P[2][v], swap2(P[2][v]), swap2(P[1][v])};
-            w[v] = teno5_core2(st, bad, count, kept, all);
+            w[v] = teno5_core2(P[0][v], P[1][v], P[2][v], bad, count, kept, all);
         }
     } else {
         // WENO5: mirror-signed difference pairs (d_{k+1} - d_k, d_{4-k} - d_{5-k}), projected
