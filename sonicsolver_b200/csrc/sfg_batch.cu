@@ -148,9 +148,12 @@ __global__ void __launch_bounds__(TILE_THREADS, F32 ? 4 : 2)
         if (!b.live || !b.clock.active) continue;  // uniform across the block
         StageView sv = batch_stage_view(b, stage, time_id);
         const bool last = stage == (time_id == T_EULER ? 0 : (time_id == T_SSPRK3 ? 2 : 3));
-        if (last) sv.mode |= MODE_CFL;  // the step's result: reduce its CFL minimum here
+        if (last) {  // the step's result: reduce its CFL minimum here
+            sv.mode |= MODE_CFL;
+            if ((long long)(b.g.hi[0] - b.g.lo[0]) * (b.g.hi[1] - b.g.lo[1]) >= SCREEN_NODES) sv.mode |= MODE_SCREEN;
+        }
         unsigned flags = 0, cut = 0, cores = 0;
-        double sr = 0.0;
+        double sr = cfl_seen(b.g, sv);
         if (w.dim == 2) {
             if constexpr (F32) tile2d_f32_body<SCHEME, FLUX, TX, TY>(b.g, sv, w.x0, w.y0, smem, flags, cut, cores, sr);
             else tile2d_body<SCHEME, FLUX, TX, TY>(b.g, sv, w.x0, w.y0, smem, flags, cut, cores, sr);

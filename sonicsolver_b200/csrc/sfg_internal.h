@@ -121,6 +121,11 @@ constexpr int MODE_RESIDUAL = 4;   // final output is R = Jac * div (no stage up
 constexpr int MODE_CFL = 8;        // last stage of a step: also reduce the CFL minimum of
                                    // the new state into clock->dt_bits (the next step's dt)
 
+constexpr int MODE_SCREEN = 32;    // with MODE_CFL: bound a node's rate before evaluating it (cfl_may_exceed)
+// Solved nodes from which a launch screens: about one and a half rounds of
+// resident 2-D blocks.  Below, every block starts with nothing reduced yet and
+// the bound costs more than it saves (257 x 193: 1.5 % of a step).
+constexpr long long SCREEN_NODES = 400000;
 constexpr int MODE_STEP = 16;      // last stage of a step: the launch's last block commits the step
                                    // and opens the next one (step_tail)
 

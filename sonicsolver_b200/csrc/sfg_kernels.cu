@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128, SCHEME == WENO7 && sizeof(T) == sizeof(do
     const long long rowbase = ((long long)k * g.n[1] + j) * g.n[0];
     const long long vs = g.vs;
     unsigned flags = 0, cut = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     double st[NST][5];
     double F[5] = {0, 0, 0, 0, 0};
     if (lane <= nodes) {
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv, int
     const int s0 = g.lo[AX] + (blockIdx.y * blockDim.y + threadIdx.y) * seglen;
     const bool live = i < g.hi[0] && s0 < g.hi[AX];
     unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     if constexpr (sizeof(T) == sizeof(float)) {
         if (live) sweep_yz_f32_segment<AX, SCHEME, FLUX>(g, sv, i, o, s0, seglen, flags, cut, cores, sr);
     } else if (live) {
@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(256) dt_kernel(GridView g, const double* __res
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     double best = 0.0;  // largest spectral-radius sum; dt = CFL / best
     unsigned fl = 0;
+    const bool screen = !g.curv && (long long)cx * cy * cz >= SCREEN_NODES;
     for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < items; w += nwarps) {
         const long long row = w / chunks;
         const int i0 = g.lo[0] + (int)(w - row * chunks) * 64;
@@ -291,6 +292,8 @@ __global__ void __launch_bounds__(256) dt_kernel(GridView g, const double* __res
                 const long long node = base + i;
                 const double qq[5] = {q[node], q[g.vs + node], q[2 * g.vs + node], q[3 * g.vs + node],
                                       q[4 * g.vs + node]};
+                // a node whose bound stays below `best` is finite and not a vacuum
+                if (screen && best > 0.0 && !cfl_may_exceed(g, qq, best)) continue;
                 const double sr = cfl_rate_node(g, qq, node);
                 if (!(sr > 0.0) || !isfinite(sr)) fl |= FLAG_NONFINITE;
                 best = fmax(best, sr);

@@ -447,7 +447,10 @@ int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_a
     sv.dt_log = s->dt_log;
     sv.dt_cap = s->dt_log_cap;
     const int dim = s->grid.dim;
-    const int cfl_bit_all = (cfl && !residual_only ? MODE_CFL : 0) | (tail ? MODE_STEP : 0);
+    const GridView& gv = s->gv;
+    const bool large = (long long)(gv.hi[0] - gv.lo[0]) * (gv.hi[1] - gv.lo[1]) * (gv.hi[2] - gv.lo[2]) >= SCREEN_NODES;
+    const int cfl_bit_all = (cfl && !residual_only ? MODE_CFL | (large && !gv.curv ? MODE_SCREEN : 0) : 0) |
+                            (tail ? MODE_STEP : 0);
     if (s->has_laws) {
         // prepareBoundaryState before the RHS: the laws on the stage's input;
         // the previous application's values sit in the previous stage's input

@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(TILE_THREADS) tile1d_kernel(GridView g, StageV
     extern __shared__ __align__(16) unsigned char smem1[];
     if (sv.require_active && !sv.clock->active) return;
     unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     tile1d_body<SCHEME, FLUX, T, T1>(g, sv, g.lo[0] + blockIdx.x * T1, reinterpret_cast<T*>(smem1), flags, cut,
                                      cores, sr);
     flush_status(sv, flags, cores, cut);

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) tile2d_kernel(GridView g, Sta
     const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
     const int x0 = g.lo[0] + (blockIdx.x % ntx) * TX, y0 = g.lo[1] + (blockIdx.x / ntx) * TY;
     unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     tile2d_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smem, flags, cut, cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) tile2d_f32_kernel(GridView g,
     const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX;
     const int x0 = g.lo[0] + (blockIdx.x % ntx) * TX, y0 = g.lo[1] + (blockIdx.x / ntx) * TY;
     unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     tile2d_f32_body<SCHEME, FLUX, TX, TY>(g, sv, x0, y0, smemf, flags, cut, cores, sr);
     flush_status(sv, flags, cores, cut);
     if (sv.mode & MODE_CFL) flush_cfl_block(g, sv.clock, sr);

@@ -70,16 +70,18 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
     const Ref32 ref = F32 ? make_ref32(qref, g.gamma) : Ref32{};
     auto load = [&](long long at, int v) -> T { return T(__ldg(sv.qs + v * vs + at) - qref[v]); };
 
+    // this thread's column (COL < the block's threads): node offset in a plane
+    const int col_at = t < COL ? map_tile_index(y0 + cj, g.n[1], g.bc_lo[1], g.bc_hi[1]) * g.n[0] +
+                                     map_tile_index(x0 + ci, g.n[0], g.bc_lo[0], g.bc_hi[0])
+                               : 0;
     // stage plane p of the block's interior into its ring slot
     auto stage_ring = [&](int p) {
         const int zk = map_tile_index(p, g.n[2], g.bc_lo[2], g.bc_hi[2]);
         const int slot = ((p % R) + R) % R;
-        for (int c = t; c < COL; c += blockDim.x) {
-            const int gx = map_tile_index(x0 + c % T3X, g.n[0], g.bc_lo[0], g.bc_hi[0]);
-            const int gy = map_tile_index(y0 + c / T3X, g.n[1], g.bc_lo[1], g.bc_hi[1]);
-            const long long at = (long long)zk * nxy + (long long)gy * nx + gx;
+        if (t < COL) {
+            const long long at = (long long)zk * nxy + col_at;
 #pragma unroll
-            for (int v = 0; v < 5; ++v) ring[(v * R + slot) * COL + c] = load(at, v);
+            for (int v = 0; v < 5; ++v) ring[(v * R + slot) * COL + t] = load(at, v);
         }
     };
     // z face p + 1/2 of this thread's column from ring planes p+1-H .. p+H
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
     };
 
     unsigned flags = 0, cut = 0, cores = 0;
-    double sr = 0.0;
+    double sr = cfl_seen(g, sv);
     // prologue: ring planes z0-H .. z0+H-1, then the face z0 - 1/2
     for (int p = z0 - H; p < z0 + H; ++p) stage_ring(p);
     __syncthreads();
