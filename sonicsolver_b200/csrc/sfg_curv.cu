@@ -480,7 +480,7 @@ __device__ __forceinline__ void flux_dev_n(const Ref32& r, const float (&dL)[5],
     }
 }
 
-// ---- WENO5 / TENO5 faces in differences -----------------------------------
+// ---- WENO5 / TENO5 / WENO7 faces in differences ---------------------------
 // The five state differences of the stencil are projected (not the six
 // points), the cores are those of the Cartesian faces (indicators64 /
 // indicators2), and the face states are q-bar + R (deltas).  The projection
@@ -586,12 +586,13 @@ __device__ __forceinline__ void curv_face64(const double (&st)[SchemeInfo<SCHEME
 #pragma unroll
     for (int v = 0; v < 5; ++v) qavg[v] = 0.5 * (st[NST / 2 - 1][v] + st[NST / 2][v]);
     double qL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, qR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if constexpr (SCHEME == WENO5 || SCHEME == TENO5) {
+    if constexpr (SCHEME != WENO3) {
+        constexpr int ND = NST - 1;
         CurvEig<double> e;
         curv_eig<double>(qavg, pressure_n(qavg, gamma, flags), n, gamma, e);
-        double w[5][5];
+        double w[ND][5];
 #pragma unroll
-        for (int s = 0; s < 5; ++s) {
+        for (int s = 0; s < ND; ++s) {
             double d[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) d[v] = add_rn(st[s + 1][v], -st[s][v]);
@@ -600,9 +601,12 @@ __device__ __forceinline__ void curv_face64(const double (&st)[SchemeInfo<SCHEME
         double wl[5], wr[5], dl[5], dr[5];
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-            const double x[5] = {w[0][v], w[1][v], w[2][v], w[3][v], w[4][v]};
+            double x[ND];
+#pragma unroll
+            for (int s = 0; s < ND; ++s) x[s] = w[s][v];
             if constexpr (SCHEME == WENO5) weno5_pair64(x, wl[v], wr[v], flags);
-            else teno5_pair64(x, wl[v], wr[v], flags, cut);
+            else if constexpr (SCHEME == TENO5) teno5_pair64(x, wl[v], wr[v], flags, cut);
+            else weno7_pair64(x, wl[v], wr[v], flags);
         }
         curv_back(e, wl, dl);
         curv_back(e, wr, dr);
@@ -658,39 +662,41 @@ __device__ __forceinline__ void rusanov_dev_n2(const Ref32& r, const float2 (&d)
     }
 }
 
-// WENO5 / TENO5 face in the FP32-flux form (face_flux_dev32x2 along n).
+// WENO5 / TENO5 / WENO7 face in the FP32-flux form (face_flux_dev32x2 along n).
 template <int SCHEME, int FLUX>
-__device__ __forceinline__ void curv_face_dev32x2(const float (&d)[6][5], const Ref32& ref, const float (&n)[3],
-                                                  float gamma, float (&F)[5], unsigned& flags, unsigned& cut,
-                                                  bool count) {
+__device__ __forceinline__ void curv_face_dev32x2(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
+                                                  const float (&n)[3], float gamma, float (&F)[5], unsigned& flags,
+                                                  unsigned& cut, bool count) {
+    constexpr int CL = SchemeInfo<SCHEME>::NST / 2 - 1;
     float dbar[5], qa[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        dbar[v] = 0.5f * (d[2][v] + d[3][v]);
+        dbar[v] = 0.5f * (d[CL][v] + d[CL + 1][v]);
         qa[v] = ref.q[v] + dbar[v];
     }
     const float pa = (gamma - 1.f) * (qa[4] - 0.5f * (qa[1] * qa[1] + qa[2] * qa[2] + qa[3] * qa[3]) * rcp_approx(qa[0]));
     if (!(qa[0] > 0.f) || !(pa > 0.f)) flags |= FLAG_PRESSURE;
     CurvEig<float> e;
     curv_eig<float>(qa, pa, n, gamma, e);
-    float2 E[2][5];
+    float2 E[CL][5];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < CL; ++k) {
         float2 x[5];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[4 - k][v]), f2(d[k][v], d[5 - k][v]));
+        for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[2 * CL - k][v]), f2(d[k][v], d[2 * CL + 1 - k][v]));
         curv_project(e, x, E[k]);
     }
-    float mid[5], E2[5];
+    float mid[5], M[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) mid[v] = d[3][v] - d[2][v];
-    curv_project(e, mid, E2);
+    for (int v = 0; v < 5; ++v) mid[v] = d[CL + 1][v] - d[CL][v];
+    curv_project(e, mid, M);
     float2 w[5], dq[5], kept = f2(0.f), bad = f2(0.f);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        const float2 e2 = f2(E2[v], -E2[v]);
-        if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], e2, bad, count, kept);
-        else w[v] = weno5_delta2(E[0][v], E[1][v], e2, bad);
+        const float2 em = f2(M[v], -M[v]);
+        if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], em, bad, count, kept);
+        else if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], em, bad);
+        else w[v] = weno5_delta2(E[0][v], E[1][v], em, bad);
     }
     flag_bad(bad, flags);
     if constexpr (SCHEME == TENO5) {
@@ -719,7 +725,7 @@ template <int SCHEME, int FLUX>
 __device__ __forceinline__ void curv_face_dev32(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
                                                 const float (&n)[3], float gamma, float (&F)[5], unsigned& flags,
                                                 unsigned& cut, bool count) {
-    if constexpr (SCHEME == WENO5 || SCHEME == TENO5) {
+    if constexpr (SCHEME != WENO3) {
         curv_face_dev32x2<SCHEME, FLUX>(d, ref, n, gamma, F, flags, cut, count);
         return;
     }

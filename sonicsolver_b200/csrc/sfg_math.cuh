@@ -1028,7 +1028,7 @@ __device__ __forceinline__ float2 teno5_core2(float2 v0, float2 v1, float2 v2, f
     return teno5_weights2(k, q, v2);
 }
 
-// FP32 WENO5 / TENO5 on a face's six points in differences, the left and right
+// FP32 WENO5 / TENO5 (WENO7 below) on a face's points in differences, the left and right
 // sides as the two lanes of a pair; the mathematics of indicators64.  With the
 // mirror-signed difference pairs E0 = (c1 - c0, c4 - c5), E1 = (c2 - c1,
 // c3 - c4), E2 = (c3 - c2, c2 - c3):
@@ -1065,6 +1065,37 @@ __device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 E2, 
     const float2 num = fma2(wa, fma2(f2(1.f / 3.f), d.T1, h), fma2(wb, d.N2, mul2(wc, swap2(h))));
     bad = watch2(bad, den);  // den >= 10 eps^4 > 0 unless an input was not finite
     return mul2(num, rcp2(den));
+}
+
+// WENO7-JS deltas of both sides: weno7_pair64's form with E_k = (W_k, -W_{6-k}),
+// so the right side's t and G are the swapped left ones.  Its weights stay
+// quotients (four reciprocals a side): the folded products of three (eps + b)^2
+// leave FP32 range.  Against the scalar form, us a step: 700 x 520 267 -> 123,
+// 128 x 100 x 90 3314 -> 862 (with the 3-D tile's chunks), curved 500 x 400
+// 248 -> 88 (with the curved faces' other changes).
+__device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, float2 E3, float2& bad) {
+    const float2 T1 = sub2(E1, E0), T2 = sub2(E2, E1), T3 = sub2(E3, E2), T4 = swap2(T3), T5 = swap2(T2);
+    const float2 G[4] = {sub2(T2, T1), sub2(T3, T2), sub2(T4, T3), sub2(T5, T4)};
+    const float2 mid = mul2(f2(0.5f), add2(E2, E3));
+    const float2 a[4] = {fma2(f2(0.375f), G[0], fma2(f2(0.5f), T2, E2)), fma2(f2(-0.125f), G[1], mid),
+                         fma2(f2(-0.125f), G[2], mid), fma2(f2(0.375f), G[3], fma2(f2(-0.5f), T4, E3))};
+    const float2 b0 = add2(T2, G[0]), b3 = sub2(T4, G[3]);
+    const float2 c13 = f2(13.f / 12.f);
+    const float2 u = mul2(mul2(c13, T3), T3);
+    const float2 b[4] = {mul2(mul2(c13, b0), b0), u, u, mul2(mul2(c13, b3), b3)};
+    const float2 P[4] = {fma2(f2(-6.f), T3, fma2(f2(7.f), T2, mul2(f2(-3.f), T1))), fma2(f2(-3.f), T3, T2),
+                         mul2(f2(-1.f), add2(T3, T4)), fma2(f2(-3.f), T4, T5)};
+    const float d[4] = {1.f, 12.f, 18.f, 4.f};
+    float2 den = f2(0.f), num = f2(0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 e = fma2(a[k], a[k], fma2(mul2(f2(781.f / 720.f), G[k]), G[k], add2(b[k], f2(1e-6f))));
+        const float2 w = mul2(f2(d[k]), rcp2(mul2(e, e)));
+        den = add2(den, w);
+        num = fma2(w, P[k], num);
+    }
+    bad = watch2(bad, den);
+    return mul2(num, rcp2(mul2(f2(12.f), den)));
 }
 
 // TENO5 deltas of both sides.  With `count` (a launch-uniform switch: the
@@ -1324,14 +1355,16 @@ __device__ __forceinline__ void rusanov_dev2(const Ref32& r, const float2 d[5], 
     }
 }
 
-// face_flux_dev32 with the left / right work paired in float2 (WENO5, TENO5).
+// face_flux_dev32 with the left / right work paired in float2 (WENO5, TENO5, WENO7).
 template <int AX, int SCHEME, int FLUX>
-__device__ __forceinline__ void face_flux_dev32x2(const float (&d)[6][5], const Ref32& ref, float gamma, float F[5],
-                                                  unsigned& flags, unsigned& cut, bool count, float scale) {
+__device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
+                                                  float gamma, float F[5], unsigned& flags, unsigned& cut, bool count,
+                                                  float scale) {
+    constexpr int CL = SchemeInfo<SCHEME>::NST / 2 - 1;  // the face lies between points CL and CL + 1
     float dbar[5], qbar[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        dbar[v] = 0.5f * (d[2][v] + d[3][v]);
+        dbar[v] = 0.5f * (d[CL][v] + d[CL + 1][v]);
         qbar[v] = ref.q[v] + dbar[v];
     }
     Eigen<float> es;
@@ -1359,21 +1392,25 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[6][5], const 
             w[v] = teno5_core2(P[0][v], P[1][v], P[2][v], bad, count, kept, all);
         }
     } else {
-        // WENO5: mirror-signed difference pairs (d_{k+1} - d_k, d_{4-k} - d_{5-k}), projected
-        float2 E[2][5];
+        // WENO5, WENO7: mirror-signed difference pairs (d_{k+1} - d_k, d_{2CL-k} - d_{2CL+1-k}), projected
+        float2 E[CL][5];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < CL; ++k) {
             float2 x[5];
 #pragma unroll
-            for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[4 - k][v]), f2(d[k][v], d[5 - k][v]));
+            for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[2 * CL - k][v]), f2(d[k][v], d[2 * CL + 1 - k][v]));
             to_characteristic2<AX>(e, x, E[k]);
         }
-        float m[5], E2[5];  // the middle difference, the same on both sides up to its sign
+        float m[5], M[5];  // the middle difference, the same on both sides up to its sign
 #pragma unroll
-        for (int v = 0; v < 5; ++v) m[v] = d[3][v] - d[2][v];
-        project32<AX>(es, m, E2);
+        for (int v = 0; v < 5; ++v) m[v] = d[CL + 1][v] - d[CL][v];
+        project32<AX>(es, m, M);
 #pragma unroll
-        for (int v = 0; v < 5; ++v) w[v] = weno5_delta2(E[0][v], E[1][v], f2(E2[v], -E2[v]), bad);
+        for (int v = 0; v < 5; ++v) {
+            const float2 em = f2(M[v], -M[v]);
+            if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], em, bad);
+            else w[v] = weno5_delta2(E[0][v], E[1][v], em, bad);
+        }
     }
     flag_bad(bad, flags);
     if constexpr (SCHEME == TENO5) {
@@ -1412,7 +1449,7 @@ template <int AX, int SCHEME, int FLUX>
 __device__ __forceinline__ void face_flux_dev32(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
                                                 float gamma, float F[5], unsigned& flags, unsigned& cut,
                                                 bool count = true, float scale = 1.f) {
-    if constexpr (SCHEME == WENO5 || SCHEME == TENO5) {
+    if constexpr (SCHEME != WENO3) {
         face_flux_dev32x2<AX, SCHEME, FLUX>(d, ref, gamma, F, flags, cut, count, scale);
         return;
     }
