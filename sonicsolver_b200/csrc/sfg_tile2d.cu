@@ -1,10 +1,12 @@
-// sfg_tile2d.cu -- the 2-D tile launcher with its full-size tiles (32 x 15,
+// sfg_tile2d.cu -- the 2-D tile launcher with its middle tiles (32 x 15,
 // 22 x 22), and the 1-D tiles.
 #include "sfg_tile2d.cuh"
 
 namespace sfg {
 
 cudaError_t launch_tile2d_small(int rounds, int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
+                                cudaStream_t st);
+cudaError_t launch_tile2d_large(int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
                                 cudaStream_t st);
 
 // 1-D grids: one block per T1-node tile (the body the batched kernels use, so a
@@ -83,6 +85,11 @@ cudaError_t launch_tile1d(int scheme, int flux, int prec64, const GridView& g, c
 // 257 x 193 48 / 42 / 44, 320^2 62 / 64 / 72, 512^2 107 / 114 / 145; FP32
 // 64^2 36 / 28 / 24, 257 x 193 42 / 35 / 34, 320^2 48 / 44 / 44, 400^2 59 /
 // 56 / 59, 512^2 69 / 71 / 87 (more blocks repeat more halo and edge faces).
+// A grid of many rounds of blocks takes 32 x 23 (six rounds of faces): less halo
+// and fewer edge faces, once its coarser last round of blocks no longer counts.
+// 32 x 15 / 32 x 23: FP64 TENO5 700^2 182 / 184, 768^2 215 / 213, 1024^2 371 /
+// 358, 2048^2 1357 / 1287; FP32 WENO5 1024^2 202 / 201, 1600^2 454 / 443, 2048^2
+// 721 / 696; FP32 TENO5 1024^2 228 / 234, 2048^2 818 / 813.
 cudaError_t launch_tile2d(int variant, int scheme, int flux, int prec64, const GridView& g, const StageView& sv,
                           cudaStream_t st) {
     if (variant < 1 || variant > 2) return cudaErrorInvalidValue;
@@ -92,6 +99,7 @@ cudaError_t launch_tile2d(int variant, int scheme, int flux, int prec64, const G
     if (blocks(16, 7) <= resident) return launch_tile2d_small(1, scheme, flux, prec64, g, sv, st);
     if (blocks(32, 7) <= resident) return launch_tile2d_small(2, scheme, flux, prec64, g, sv, st);
     if (variant == 2) return launch_tile_p<22, 22>(prec64, scheme, flux, g, sv, st);
+    if (blocks(32, 15) >= (prec64 ? 4 : 8) * resident) return launch_tile2d_large(scheme, flux, prec64, g, sv, st);
     return launch_tile_p<32, 15>(prec64, scheme, flux, g, sv, st);
 }
 

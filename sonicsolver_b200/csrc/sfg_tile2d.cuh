@@ -1,6 +1,7 @@
 // sfg_tile2d.cuh -- single-grid fused stage kernels for 2-D grids: one launch
 // per stage, one block per tile (bodies in sfg_tile.cuh).  The tile shapes are
-// instantiated in two translation units (sfg_tile2d.cu, sfg_tile2d_small.cu).
+// instantiated in three translation units (sfg_tile2d.cu, sfg_tile2d_small.cu,
+// sfg_tile2d_large.cu).
 #pragma once
 
 #include "sfg_tile.cuh"

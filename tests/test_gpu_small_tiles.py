@@ -1,4 +1,5 @@
-"""2-D grids too small for the full-size tiles run one- and two-round tiles."""
+"""2-D grids too small for the full-size tiles run one- and two-round tiles, large
+ones 32 x 23 tiles."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,7 @@ from sonicsolver_b200 import capi, cases
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_FP32_FLUX])
 @pytest.mark.parametrize("recipe", ["weno3Rusanov", "weno5Roe", "teno5Rusanov", "weno7Rusanov"])
-@pytest.mark.parametrize("n", [(9, 9), (16, 7), (17, 8), (33, 15), (34, 16), (255, 120), (320, 200), (640, 300)])
+@pytest.mark.parametrize("n", [(9, 9), (16, 7), (17, 8), (33, 15), (34, 16), (255, 120), (320, 200), (640, 300), (863, 845), (1535, 1541)])
 def test_small_tiles_give_the_bits_of_the_large(n, recipe, precision):
     """Grids on both sides of the tile-shape rule's lines, and of one tile's
     edge: one step of the solver (the shape the rule picks) against the batch,
@@ -24,7 +25,7 @@ def test_small_tiles_give_the_bits_of_the_large(n, recipe, precision):
                       "SSPRK3")
     s = case.solver(precision=precision)
     s.advance(1e30, max_steps=2)
-    b = capi.Batch(64 << 20, 1, recipe=recipe, precision=precision, cfl=0.4)
+    b = capi.Batch((64 << 20) + 130 * nx * ny, 1, recipe=recipe, precision=precision, cfl=0.4)
     slot = b.add(case, t_end=1e30, max_steps=2)
     b.step(3)
     np.testing.assert_array_equal(s.download().reshape(q.shape), b.download(slot))
