@@ -1254,9 +1254,8 @@ static cudaError_t launch_curv_faces_f(int flux, int prec64, const GridView& g, 
     return cudaErrorInvalidValue;
 }
 
-template <int SCHEME, int FLUX>
+template <int SCHEME, int FLUX, int TX, int TY>
 static cudaError_t launch_curv_tile2d(const GridView& g, const StageView& sv, cudaStream_t st) {
-    constexpr int TX = 22, TY = 22;
     using S = TileShape<SCHEME, TX, TY>;
     const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX, nty = (g.hi[1] - g.lo[1] + TY - 1) / TY;
     const size_t smem = sizeof(float) * S::ELEMS;
@@ -1269,9 +1268,8 @@ static cudaError_t launch_curv_tile2d(const GridView& g, const StageView& sv, cu
     return cudaGetLastError();
 }
 
-template <int SCHEME, int FLUX>
+template <int SCHEME, int FLUX, int TX, int TY>
 static cudaError_t launch_curv_tile2d64(const GridView& g, const StageView& sv, cudaStream_t st) {
-    constexpr int TX = 22, TY = 22;
     using S = TileShape<SCHEME, TX, TY>;
     const int ntx = (g.hi[0] - g.lo[0] + TX - 1) / TX, nty = (g.hi[1] - g.lo[1] + TY - 1) / TY;
     const size_t smem = sizeof(double) * S::ELEMS;
@@ -1284,21 +1282,33 @@ static cudaError_t launch_curv_tile2d64(const GridView& g, const StageView& sv, 
     return cudaGetLastError();
 }
 
-template <int SCHEME>
+template <int SCHEME, int TX, int TY>
 static cudaError_t launch_curv_tile2d_f(int flux, int prec64, const GridView& g, const StageView& sv,
                                         cudaStream_t st) {
     if (prec64) {
         switch (flux) {
-        case RUSANOV: return launch_curv_tile2d64<SCHEME, RUSANOV>(g, sv, st);
-        case ROE: return launch_curv_tile2d64<SCHEME, ROE>(g, sv, st);
-        case STEGER: return launch_curv_tile2d64<SCHEME, STEGER>(g, sv, st);
-        case LAXF: return launch_curv_tile2d64<SCHEME, LAXF>(g, sv, st);
+        case RUSANOV: return launch_curv_tile2d64<SCHEME, RUSANOV, TX, TY>(g, sv, st);
+        case ROE: return launch_curv_tile2d64<SCHEME, ROE, TX, TY>(g, sv, st);
+        case STEGER: return launch_curv_tile2d64<SCHEME, STEGER, TX, TY>(g, sv, st);
+        case LAXF: return launch_curv_tile2d64<SCHEME, LAXF, TX, TY>(g, sv, st);
         }
         return cudaErrorInvalidValue;
     }
-    if (flux == RUSANOV) return launch_curv_tile2d<SCHEME, RUSANOV>(g, sv, st);
-    if (flux == ROE) return launch_curv_tile2d<SCHEME, ROE>(g, sv, st);
+    if (flux == RUSANOV) return launch_curv_tile2d<SCHEME, RUSANOV, TX, TY>(g, sv, st);
+    if (flux == ROE) return launch_curv_tile2d<SCHEME, ROE, TX, TY>(g, sv, st);
     return cudaErrorInvalidValue;
+}
+
+// 22 x 22 tiles (four rounds of faces), or 16 x 7 (one round) where those blocks
+// are all resident at once (2 per SM in FP64, 3 in FP32), as on uniform grids.
+// us a step, WENO5, before / after: FP64 100 x 80 49 / 23, 160^2 28 (22 x 22: 50 at
+// 256^2, where the rule keeps it); FP32 100 x 80 22, 200 x 150 25, 256^2 39 (22 x 22).
+template <int SCHEME>
+static cudaError_t launch_curv_tile2d_s(int flux, int prec64, const GridView& g, const StageView& sv,
+                                        cudaStream_t st) {
+    const long long small = (long long)((g.hi[0] - g.lo[0] + 15) / 16) * ((g.hi[1] - g.lo[1] + 6) / 7);
+    if (small <= 148 * (prec64 ? 2 : 3)) return launch_curv_tile2d_f<SCHEME, 16, 7>(flux, prec64, g, sv, st);
+    return launch_curv_tile2d_f<SCHEME, 22, 22>(flux, prec64, g, sv, st);
 }
 
 // One stage on a curvilinear grid: the face fluxes of every active axis, then
@@ -1308,10 +1318,10 @@ cudaError_t launch_curv_stage(int scheme, int flux, int prec64, int tiles, const
                               double* fl, cudaStream_t st) {
     if (g.dim == 2 && tiles) {
         switch (scheme) {
-        case WENO5: return launch_curv_tile2d_f<WENO5>(flux, prec64, g, sv, st);
-        case TENO5: return launch_curv_tile2d_f<TENO5>(flux, prec64, g, sv, st);
-        case WENO3: return launch_curv_tile2d_f<WENO3>(flux, prec64, g, sv, st);
-        case WENO7: return launch_curv_tile2d_f<WENO7>(flux, prec64, g, sv, st);
+        case WENO5: return launch_curv_tile2d_s<WENO5>(flux, prec64, g, sv, st);
+        case TENO5: return launch_curv_tile2d_s<TENO5>(flux, prec64, g, sv, st);
+        case WENO3: return launch_curv_tile2d_s<WENO3>(flux, prec64, g, sv, st);
+        case WENO7: return launch_curv_tile2d_s<WENO7>(flux, prec64, g, sv, st);
         default: return cudaErrorInvalidValue;
         }
     }
