@@ -1098,28 +1098,26 @@ static int capture_steps(sfg_solver_s* s, int n, cudaGraphExec_t* out) {
     return SFG_OK;
 }
 
-// Enqueues `n` steps as a graph kept in (*graph, *steps), captured when the
-// slot holds another count.
-static int launch_steps_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* steps) {
-    if (!*graph || *steps != n) {
-        if (*graph) cudaGraphExecDestroy(*graph);
-        *graph = nullptr;
-        if (int rc = capture_steps(s, n, graph)) return rc;
-        *steps = n;
-    }
-    CUDA_TRY(cudaGraphLaunch(*graph, s->stream));
-    return SFG_OK;
+// Captures `n` steps into (*graph, *steps) unless the slot holds them.
+static int keep_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* steps) {
+    if (*graph && *steps == n) return SFG_OK;
+    if (*graph) cudaGraphExecDestroy(*graph);
+    *graph = nullptr;
+    *steps = n;
+    return capture_steps(s, n, graph);
 }
 
 // sfg_advance outside the cluster kernel: graphs of `graph_steps` CFL steps,
 // relaunched until the clock stops.  Fewer steps than a graph holds (max_steps,
 // or what t_end leaves at the last dt) are launched one by one, or by a graph
 // of their own once a run has left the same number before (5-7 us a step less
-// on small grids; capturing at once would cost a single run more than it
-// gains): a graph's steps past the end return at once but still cost their
-// launches, 3.9 ms of the 14 ms a three-step run of 256^3 sweeps took.
+// on small grids): a graph's steps past the end return at once but still cost
+// their launches, 12 of the 42 ms a three-step run of 256^3 sweeps took.
+// Steps whose graph is not there yet are launched one by one too, and the graph
+// is captured behind them, while they run: at the first call of a caller that
+// names its graph length (`asked`), else when a run has that many steps to go.
 // `ms`: device time of the launches.
-static int advance_graph(sfg_solver_s* s, int graph_steps, float* ms) {
+static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms) {
     Clock* hc = s->host_clock;
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
@@ -1131,19 +1129,26 @@ static int advance_graph(sfg_solver_s* s, int graph_steps, float* ms) {
         // to spare for a shrinking dt
         double left = double(hc->max_steps - hc->steps);
         if (!first && hc->dt > 0.0) left = std::min(left, std::ceil((hc->t_end - hc->t) / hc->dt) + 2.0);
-        if (left >= graph_steps) {
-            rc = launch_steps_graph(s, graph_steps, &s->graph, &s->graph_steps);
+        const bool full = left >= graph_steps;
+        const int n = full ? graph_steps : std::max(1, int(left));
+        cudaGraphExec_t ready = full ? (s->graph_steps == n ? s->graph : nullptr)
+                                     : (s->rest_steps == n ? s->rest_graph : nullptr);
+        if (ready) {
+            if (cudaGraphLaunch(ready, s->stream) != cudaSuccess)
+                rc = fail(SFG_ERR_CUDA, "graph launch: %s", cudaGetErrorString(cudaGetLastError()));
         } else {
-            const int n = std::max(1, int(left));
-            if (s->rest_steps == n) {
-                rc = launch_steps_graph(s, n, &s->rest_graph, &s->rest_steps);
-            } else {
-                if (s->rest_graph) cudaGraphExecDestroy(s->rest_graph);
-                s->rest_graph = nullptr;
-                s->rest_steps = n;
-                for (int i = 0; i < n && !rc; ++i) rc = enqueue_cfl_step(s, true, true);
+            for (int i = 0; i < n && !rc; ++i) rc = enqueue_cfl_step(s, true, true);
+            if (!rc && !full) {
+                if (s->rest_steps == n) {
+                    rc = keep_graph(s, n, &s->rest_graph, &s->rest_steps);
+                } else {
+                    if (s->rest_graph) cudaGraphExecDestroy(s->rest_graph);
+                    s->rest_graph = nullptr;
+                    s->rest_steps = n;
+                }
             }
         }
+        if (!rc && (asked || full)) rc = keep_graph(s, graph_steps, &s->graph, &s->graph_steps);
         unsigned bits = 0;
         if (!rc && (cudaMemcpyAsync(hc, s->clock, sizeof(Clock), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
                     cudaStreamSynchronize(s->stream) != cudaSuccess ||
@@ -1211,7 +1216,8 @@ int sfg_advance(sfg_solver s, double t_end, int64_t max_steps, double write_inte
     if (!s) return fail(SFG_ERR_ARG, "null solver");
     if (s->next_stage != 0) return fail(SFG_ERR_ARG, "a step is in progress");
     if (!(t_end == t_end)) return fail(SFG_ERR_ARG, "t_end is NaN");
-    if (graph_steps <= 0) graph_steps = 32;
+    const bool asked = graph_steps > 0;
+    if (!asked) graph_steps = 32;
     int rc = pull_clock(s);
     if (rc) return rc;
     Clock* hc = s->host_clock;
@@ -1245,7 +1251,7 @@ int sfg_advance(sfg_solver s, double t_end, int64_t max_steps, double write_inte
         if (rc) return rc;
     }
     if (!ran) {
-        rc = advance_graph(s, graph_steps, &ms);
+        rc = advance_graph(s, graph_steps, asked, &ms);
         if (rc) return rc;
     }
     const long long done = hc->steps - steps0;
