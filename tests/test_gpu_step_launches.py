@@ -24,6 +24,8 @@ def _grid(name):
         c = cases.sod_1d(60)
         c.bc_lo, c.bc_hi = (capi.BC_LAW, 0, 0), (capi.BC_LAW, 0, 0)
         return c, {"variant": 1}
+    if name == "cluster1d":
+        return cases.sod_1d(90), {}
     return cases.sod_1d(90), {"variant": 1}
 
 
@@ -63,3 +65,23 @@ def test_advance_equals_single_steps(name, precision, time_recipe):
     for n, q in ends[1:]:
         assert n == ends[0][0]
         np.testing.assert_array_equal(q, ends[0][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("time_recipe", ["SSPRK3", "forwardEuler", "classicalRK4"])
+@pytest.mark.parametrize("name", ["tiles1d", "cluster1d", "tiles2d", "sweeps3d", "tiles3d", "curved", "laws"])
+def test_advance_without_a_step_keeps_the_state(name, time_recipe):
+    """A run that takes no step (its end time is reached) leaves a state handed
+    over after an earlier run as it is, to the bit."""
+    case, kw = _grid(name)
+    s = case.solver(time_recipe=time_recipe, cfl=0.2)
+    if "variant" in kw:
+        s.variant = kw["variant"]
+    s.advance(1e30, max_steps=3, graph_steps=2)
+    q = np.ascontiguousarray(case.q * 1.25)
+    for t_end, g in ((3.0, 2), (2.0, 1)):
+        s.upload(q, 3.0)
+        before = s.download()
+        st, _ = s.advance(t_end, graph_steps=g)
+        assert st.steps == 0 and s.time() == (3.0, 0)
+        np.testing.assert_array_equal(s.download(), before)
