@@ -1067,12 +1067,12 @@ int sfg_step(sfg_solver s, double dt, double limit) {
         }
         return SFG_OK;
     }
-    // CFL step on device; one-shot limit through the clock
-    s->host_clock->t_end = kInf;
-    s->host_clock->max_steps = std::numeric_limits<long long>::max();
+    // CFL step on device; one-shot limit through the clock.  The step has no end
+    // time: the largest finite one, because the stop test (remaining > 64 eps
+    // scale) compares inf with inf for an infinite one and opens nothing.
     int rc = pull_clock(s);
     if (rc) return rc;
-    s->host_clock->t_end = kInf;
+    s->host_clock->t_end = std::numeric_limits<double>::max();
     s->host_clock->max_steps = std::numeric_limits<long long>::max();
     s->host_clock->limit = limit > 0.0 ? limit : kInf;
     s->host_clock->dt_bits = 0x7FEFFFFFFFFFFFFFull;
@@ -1083,7 +1083,7 @@ int sfg_step(sfg_solver s, double dt, double limit) {
     if (rc) return rc;
     rc = enqueue_open_run(s);
     if (rc) return rc;
-    rc = enqueue_cfl_step(s, false, false);
+    rc = enqueue_cfl_step(s, true, false);  // an invalid state opens no step
     if (rc) return rc;
     return sync_and_check(s);
 }

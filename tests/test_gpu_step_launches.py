@@ -85,3 +85,33 @@ def test_advance_without_a_step_keeps_the_state(name, time_recipe):
         st, _ = s.advance(t_end, graph_steps=g)
         assert st.steps == 0 and s.time() == (3.0, 0)
         np.testing.assert_array_equal(s.download(), before)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("time_recipe", ["SSPRK3", "forwardEuler", "classicalRK4"])
+@pytest.mark.parametrize("name", ["tiles1d", "tiles2d", "sweeps3d", "tiles3d", "curved", "laws"])
+def test_cfl_step_is_one_step_of_a_run(name, time_recipe):
+    """sfg_step without a dt: the CFL step from the state handed over, at the
+    run's dt, with its bits; a limit clips it; an invalid state is refused and
+    stays as it is."""
+    case, kw = _grid(name)
+    a, b = (case.solver(time_recipe=time_recipe, cfl=0.2) for _ in range(2))
+    for s in (a, b):
+        if "variant" in kw:
+            s.variant = kw["variant"]
+    _, dts = a.advance(1e30, max_steps=3, dt_capacity=3)
+    for k in range(3):
+        b.step()
+        assert b.time() == (float(sum(dts[:k + 1])), k + 1)
+    np.testing.assert_array_equal(a.download(), b.download())
+    t, n = b.time()
+    b.step(limit=0.25 * float(dts[2]))
+    assert b.time() == (t + 0.25 * float(dts[2]), n + 1)
+    bad = np.ascontiguousarray(case.q).copy()
+    bad[0, -5 if case.dim > 1 else 0, 20 % case.n[0], 4] = np.nan
+    b.upload(bad)
+    before = b.download()
+    with pytest.raises(capi.SolverError) as e:
+        b.step()
+    assert e.value.code == capi.ERR_STATE and b.time() == (0.0, 0)
+    np.testing.assert_array_equal(b.download(), before)
