@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(TILE_THREADS, F32 ? 4 : 2)
         const bool last = stage == (time_id == T_EULER ? 0 : (time_id == T_SSPRK3 ? 2 : 3));
         if (last) {  // the step's result: reduce its CFL minimum here
             sv.mode |= MODE_CFL;
-            if ((long long)(b.g.hi[0] - b.g.lo[0]) * (b.g.hi[1] - b.g.lo[1]) >= SCREEN_NODES) sv.mode |= MODE_SCREEN;
+            if (cfl_screens(b.g)) sv.mode |= MODE_SCREEN;
         }
         unsigned flags = 0, cut = 0, cores = 0;
         double sr = cfl_seen(b.g, sv);

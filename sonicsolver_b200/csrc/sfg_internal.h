@@ -121,13 +121,21 @@ constexpr int MODE_RESIDUAL = 4;   // final output is R = Jac * div (no stage up
 constexpr int MODE_CFL = 8;        // last stage of a step: also reduce the CFL minimum of
                                    // the new state into clock->dt_bits (the next step's dt)
 
+constexpr int MODE_STEP = 16;      // last stage of a step: the launch's last block commits the step
+                                   // and opens the next one (step_tail)
 constexpr int MODE_SCREEN = 32;    // with MODE_CFL: bound a node's rate before evaluating it (cfl_may_exceed)
 // Solved nodes from which a launch screens: about one and a half rounds of
 // resident 2-D blocks.  Below, every block starts with nothing reduced yet and
 // the bound costs more than it saves (257 x 193: 1.5 % of a step).
 constexpr long long SCREEN_NODES = 400000;
-constexpr int MODE_STEP = 16;      // last stage of a step: the launch's last block commits the step
-                                   // and opens the next one (step_tail)
+// Whether a grid's launches bound a node's rate before evaluating it: from
+// SCREEN_NODES solved nodes on, uniform metrics that FP32 holds with room.
+__host__ __device__ inline bool cfl_screens(const GridView& g) {
+    if (g.curv || (long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]) < SCREEN_NODES) return false;
+    for (int a = 0; a < g.dim; ++a)
+        if (!(g.metric[a] > 1e-15 && g.metric[a] < 1e15)) return false;
+    return true;
+}
 
 // One launch of the 1-D whole-run cluster kernel (sfg_cluster1d.cu): the
 // stage views of a step, the clock it advances and where it logs.

@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) dt_kernel(GridView g, const double* __res
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     double best = 0.0;  // largest spectral-radius sum; dt = CFL / best
     unsigned fl = 0;
-    const bool screen = !g.curv && (long long)cx * cy * cz >= SCREEN_NODES;
+    const bool screen = cfl_screens(g);
     for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < items; w += nwarps) {
         const long long row = w / chunks;
         const int i0 = g.lo[0] + (int)(w - row * chunks) * 64;

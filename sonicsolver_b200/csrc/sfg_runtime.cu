@@ -448,10 +448,7 @@ int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_a
     sv.dt_log = s->dt_log;
     sv.dt_cap = s->dt_log_cap;
     const int dim = s->grid.dim;
-    const GridView& gv = s->gv;
-    const bool large = (long long)(gv.hi[0] - gv.lo[0]) * (gv.hi[1] - gv.lo[1]) * (gv.hi[2] - gv.lo[2]) >= SCREEN_NODES;
-    const int cfl_bit_all = (cfl && !residual_only ? MODE_CFL | (large && !gv.curv ? MODE_SCREEN : 0) : 0) |
-                            (tail ? MODE_STEP : 0);
+    const int cfl_bit = (cfl && !residual_only ? MODE_CFL | (cfl_screens(s->gv) ? MODE_SCREEN : 0) : 0) | (tail ? MODE_STEP : 0);
     if (s->has_laws) {
         // prepareBoundaryState before the RHS: the laws on the stage's input;
         // the previous application's values sit in the previous stage's input
@@ -460,13 +457,12 @@ int enqueue_stage(sfg_solver_s* s, int stage, bool residual_only, bool require_a
                                  s->flags, s->stream));
     }
     if (s->gv.curv) {  // per-face geometry: face-flux launches per axis, then the stage
-        sv.mode = MODE_FINAL | (residual_only ? MODE_RESIDUAL : 0) | cfl_bit_all;
+        sv.mode = MODE_FINAL | (residual_only ? MODE_RESIDUAL : 0) | cfl_bit;
         // 2-D: the fused tile unless variant 0 (face launches) is selected
         CUDA_TRY(launch_curv_stage(s->recipe->scheme, s->recipe->flux, s->num.precision == SFG_PREC_FP64,
                                    s->variant > 0, s->gv, sv, s->face_flux, s->stream));
         return SFG_OK;
     }
-    const int cfl_bit = cfl_bit_all;
     if (dim == 2 && s->variant > 0) {
         sv.mode = MODE_FINAL | (residual_only ? MODE_RESIDUAL : 0) | cfl_bit;
         CUDA_TRY(launch_tile2d(s->variant, s->recipe->scheme, s->recipe->flux, s->num.precision == SFG_PREC_FP64,

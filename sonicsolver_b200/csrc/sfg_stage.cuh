@@ -104,8 +104,12 @@ __device__ __forceinline__ double cfl_rate_node(const GridView& g, const double 
 // step with the other changes to that face; Taylor-Green 256^3 FP32 4 %.
 // The bound: every FP32 operation and the approximate reciprocal are within
 // 1.2e-7 relative, so the kinetic energy is within 5e-7 (covered by 1e-6 E in the
-// pressure, as it is at most E) and the rate within 1e-5.  Values outside FP32
-// range give inf or NaN, which do not skip.
+// pressure, as it is at most E) and the rate within 1e-5.  That needs values
+// FP32 holds as normal numbers, which the skip asks for: 1 / rho above 0 (an
+// infinite rho, or one whose reciprocal flushes, gives 0), E and c away from
+// the subnormals (the metrics are: cfl_screens), no near-vacuum.  NaN or
+// infinite intermediates fail one of the tests.  So a node that is skipped is
+// finite and has a positive rate.
 __device__ __forceinline__ bool cfl_may_exceed(const GridView& g, const double (&q)[5], double seen) {
     const float inv = rcp_approx(float(q[0]));
     const float u = float(q[1]) * inv, v = float(q[2]) * inv, w = float(q[3]) * inv;
@@ -116,7 +120,9 @@ __device__ __forceinline__ bool cfl_may_exceed(const GridView& g, const double (
     float sr = (fabsf(u) + c) * float(g.metric[0]);
     if (g.dim > 1) sr += (fabsf(v) + c) * float(g.metric[1]);
     if (g.dim > 2) sr += (fabsf(w) + c) * float(g.metric[2]);
-    return !(1.00001f * sr < float(seen) * 0.999999f) || !(E - ke > 1e-6f * E);  // near-vacuum: exact
+    const bool skip = inv > 0.f && E > 1e-10f && c > 1e-15f && E - ke > 1e-6f * E &&
+                      1.00001f * sr < float(seen) * 0.999999f;
+    return !skip;
 }
 
 // Start value of a thread's largest rate: 0, or in a MODE_SCREEN launch minus the
