@@ -391,15 +391,17 @@ __device__ __forceinline__ void teno_keep32x2(float2 b0, float2 b1, float2 b2, f
 // a few ulps, every x_k >= t, so G_k >= 6.39e-5 > 2 lim (lim = 1e-5 sum G <=
 // 3.0001e-5): teno_keep32x2 would return k = 1 for all three.  (Where e_min +
 // tau is beyond 8.5e37 its reciprocal is 0 and so are t, every x_k and lim: k
-// = 1 for all three too.)  The test fails for NaN or infinite indicators (they
-// take the cut-off path and its non-finite watch), and a pair that passes has
-// finite differences, so the weights computed with k = 1 are the cut-off
-// path's to the bit.
+// = 1 for all three too.)  The test is made on tau / 4, which cannot overflow,
+// so an infinite B0 or B2 fails it, as NaN does (they take the cut-off path and
+// its non-finite watch).  A B1 that alone has overflowed passes; the cut-off
+// path keeps all three for it as well (1 / e1 = 0, x1 = t) and its watch sees
+// nothing; and B1 is never the only NaN, made as it is from the differences of
+// B0 and B2.  So the weights computed with k = 1 are the cut-off path's to the bit.
 __device__ __forceinline__ bool teno_smooth2(const float2 (&B)[3]) {
     const float2 em = add2(f2(fminf(B[0].x, fminf(B[1].x, B[2].x)), fminf(B[0].y, fminf(B[1].y, B[2].y))),
                            f2(TENO32_EPS));
     const float2 d02 = sub2(B[0], B[2]);
-    return fabsf(d02.x) <= 4.f * em.x && fabsf(d02.y) <= 4.f * em.y;
+    return fabsf(0.25f * d02.x) <= em.x && fabsf(0.25f * d02.y) <= em.y;
 }
 
 template <> struct Teno<float> {
@@ -562,10 +564,12 @@ __device__ __forceinline__ void weno7_pair64(const double (&W)[7], double& dl, d
 // The smooth-stencil test on the indicators e_k = 4 b_k + eps of one side:
 // tau <= 4 e_min and e_max < 1e30, taken on the high words (order and factor
 // 4 of positive doubles to 2^-20), which keeps it off the FP64 pipe.  The
-// proof at teno_smooth64 leaves far more room than 2^-20.
+// proof at teno_smooth64 leaves far more room than 2^-20.  Unsigned: a NaN of
+// either sign is above 1e30.
 __device__ __forceinline__ bool teno_smooth_hi(const double (&e)[3], double tau) {
-    const int h0 = __double2hiint(e[0]), h1 = __double2hiint(e[1]), h2 = __double2hiint(e[2]);
-    return hi_abs(tau) <= min(h0, min(h1, h2)) + 0x00200000 && max(h0, max(h1, h2)) < 0x46293E59;
+    const unsigned h0 = (unsigned)__double2hiint(e[0]), h1 = (unsigned)__double2hiint(e[1]),
+                   h2 = (unsigned)__double2hiint(e[2]);
+    return (unsigned)hi_abs(tau) <= min(h0, min(h1, h2)) + 0x00200000u && max(h0, max(h1, h2)) < 0x46293E59u;
 }
 
 __device__ __forceinline__ void teno5_pair64(const double (&W)[5], double& dl, double& dr, unsigned& flags,
