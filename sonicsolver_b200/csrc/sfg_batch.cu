@@ -406,7 +406,11 @@ struct sfg_batch_s {
     size_t law_items_cap = 0;
     std::vector<LawItem> h_law_items;
     int law_grid = 0;
-    bool items_stale = false;  // grids came or went since publish_items
+    bool items_stale = false;  // grids came or went since the list last reached the device
+    // per slot: the most tiles and law runs its grid can have in the lists, and
+    // their sums over the live slots
+    std::vector<size_t> inst_tiles, inst_law_runs;
+    size_t tiles = 0, law_runs = 0;
     BatchCtl* d_ctl = nullptr;
     BatchCtl* h_ctl = nullptr;  // pinned
     double* staging = nullptr;
@@ -532,11 +536,47 @@ void slab_free(sfg_batch_s* b, size_t off, size_t bytes) {
     }
 }
 
+// The most tiles a grid can have in the list (1-D: short tiles).
+size_t tile_count(const sfg_batch_s* b, const GridView& g) {
+    const size_t sx = g.hi[0] - g.lo[0], sy = g.hi[1] - g.lo[1];
+    return g.dim == 1 ? (sx + TILE1D_SHORT - 1) / TILE1D_SHORT
+                      : ((sx + b->tx - 1) / b->tx) * ((sy + b->ty - 1) / b->ty);
+}
+
+// Room for `want` entries in a device list.  A list that cannot grow stays as
+// it is; one that grew holds nothing yet (items_stale) and no graph knows it.
+template <typename Item>
+int grow_list(sfg_batch_s* b, Item** list, size_t* cap, size_t want, size_t least) {
+    if (want <= *cap) return SFG_OK;
+    const size_t grown = std::max(want * 2, least);
+    Item* p = nullptr;
+    if (cudaMalloc((void**)&p, grown * sizeof(Item)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return bfail(SFG_ERR_NOMEM, "device allocation of a work list of %zu entries failed", grown);
+    }
+    b->items_stale = true;
+    if (b->graph) {  // it holds the old list's address
+        cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    if (*list) cudaFree(*list);
+    *list = p;
+    *cap = grown;
+    return SFG_OK;
+}
+
+int grow_lists(sfg_batch_s* b, size_t tiles, size_t law_runs) {
+    int rc = grow_list(b, &b->d_items, &b->items_cap, tiles, 1024);
+    return rc ? rc : grow_list(b, &b->d_law_items, &b->law_items_cap, law_runs, 256);
+}
+
 // Rebuilds the tile list of all live instances and publishes it (and the
 // instance count) to device memory.  Grids that join or leave mark it stale
-// (items_stale) and the next step rebuilds it once for all of them.
+// (items_stale) and the next step rebuilds it once for all of them; it stays
+// stale until all of it has reached the device.  sfg_batch_add has made room.
 int publish_items(sfg_batch_s* b) {
-    b->items_stale = false;
+    b->items_stale = true;
+    if (int rc = grow_lists(b, b->tiles, b->law_runs)) return rc;
     b->h_items.clear();
     // 1-D tiles of one face round once the live tiles no longer fill the
     // SMs: a drained batch's last grids then take half the time per stage
@@ -566,17 +606,6 @@ int publish_items(sfg_batch_s* b) {
         b->h_ctl->group_range[2 * grp] = first;
         b->h_ctl->group_range[2 * grp + 1] = (int)b->h_items.size() - first;
     }
-    if (b->h_items.size() > b->items_cap) {
-        size_t cap = std::max<size_t>(b->h_items.size() * 2, 1024);
-        if (b->d_items) cudaFree(b->d_items);
-        b->d_items = nullptr;
-        BCUDA(cudaMalloc((void**)&b->d_items, cap * sizeof(WorkItem)));
-        b->items_cap = cap;
-        if (b->graph) {  // the graph holds the old list address
-            cudaGraphExecDestroy(b->graph);
-            b->graph = nullptr;
-        }
-    }
     if (!b->h_items.empty())
         BCUDA(cudaMemcpyAsync(b->d_items, b->h_items.data(), b->h_items.size() * sizeof(WorkItem),
                               cudaMemcpyHostToDevice, b->stream));
@@ -588,17 +617,6 @@ int publish_items(sfg_batch_s* b) {
         const LawView& lv = b->inst_law[i];
         const int pts = (int)lv.start[lv.count];
         for (int f = 0; f < pts; f += LAW_CHUNK) b->h_law_items.push_back({i, f, std::min(LAW_CHUNK, pts - f), 0});
-    }
-    if (b->h_law_items.size() > b->law_items_cap) {
-        size_t cap = std::max<size_t>(b->h_law_items.size() * 2, 256);
-        if (b->d_law_items) cudaFree(b->d_law_items);
-        b->d_law_items = nullptr;
-        BCUDA(cudaMalloc((void**)&b->d_law_items, cap * sizeof(LawItem)));
-        b->law_items_cap = cap;
-        if (b->graph) {  // the graph holds the old list address
-            cudaGraphExecDestroy(b->graph);
-            b->graph = nullptr;
-        }
     }
     if (!b->h_law_items.empty())
         BCUDA(cudaMemcpyAsync(b->d_law_items, b->h_law_items.data(), b->h_law_items.size() * sizeof(LawItem),
@@ -612,6 +630,7 @@ int publish_items(sfg_batch_s* b) {
     BCUDA(cudaMemcpyAsync(b->d_ctl->group_range, b->h_ctl->group_range, sizeof b->h_ctl->group_range,
                           cudaMemcpyHostToDevice, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));
+    b->items_stale = false;
     return SFG_OK;
 }
 
@@ -932,7 +951,12 @@ int sfg_batch_add_laws(sfg_batch b, const sfg_grid_desc* grid, const sfg_numeric
         b->inst_pub.push_back(sfg_grid_desc{});
         b->inst_off.push_back({0, 0, 0});
         b->inst_law.push_back(LawView{});
+        b->inst_tiles.push_back(0);
+        b->inst_law_runs.push_back(0);
     }
+    const size_t tiles = tile_count(b, g), law_runs = (size_t)((pts + LAW_CHUNK - 1) / LAW_CHUNK);
+    rc = grow_lists(b, b->tiles + tiles, b->law_runs + law_runs);
+    if (rc) return rc;
     const size_t per = align256(sizeof(double) * 5 * (size_t)g.vs);
     const int bufs = b->num.time_recipe == T_RK4 ? 4 : 3;
     const size_t slab_bytes = instance_slab_bytes(b, *grid, g);
@@ -945,6 +969,7 @@ int sfg_batch_add_laws(sfg_batch b, const sfg_grid_desc* grid, const sfg_numeric
         b->staging = nullptr;
         b->staging_cap = 0;
         if (cudaMalloc((void**)&b->staging, aos_bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
             slab_free(b, soff, slab_bytes);
             return bfail(SFG_ERR_NOMEM, "staging allocation failed");
         }
@@ -1011,6 +1036,10 @@ int sfg_batch_add_laws(sfg_batch b, const sfg_grid_desc* grid, const sfg_numeric
     b->inst_pub[idx] = *grid;
     b->inst_off[idx] = {off[0], off[1], off[2]};
     b->inst_law[idx] = lv;
+    b->inst_tiles[idx] = tiles;
+    b->inst_law_runs[idx] = law_runs;
+    b->tiles += tiles;
+    b->law_runs += law_runs;
     b->items_stale = true;
     BCUDA(cudaStreamSynchronize(b->stream));  // the caller's arrays are read
     *slot = idx;
@@ -1042,6 +1071,8 @@ int sfg_batch_remove(sfg_batch b, int slot) {
     BCUDA(cudaMemcpyAsync(&b->d_inst[slot].live, &zero, sizeof zero, cudaMemcpyHostToDevice, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));  // ordered on the batch's (non-blocking) stream
     slab_free(b, b->inst_offset[slot], b->inst_bytes[slot]);
+    b->tiles -= b->inst_tiles[slot];
+    b->law_runs -= b->inst_law_runs[slot];
     b->items_stale = true;
     return SFG_OK;
 }
@@ -1153,6 +1184,9 @@ int sfg_batch_set_variant(sfg_batch b, int variant) {
     b->variant = variant;
     int rc = bind_kernels(b);
     if (rc) return rc;
+    b->tiles = 0;  // of the new tile shape
+    for (size_t i = 0; i < b->h_inst.size(); ++i)
+        if (b->h_inst[i].live) b->tiles += b->inst_tiles[i] = tile_count(b, b->h_inst[i].g);
     return publish_items(b);
 }
 
