@@ -410,7 +410,8 @@ int sfg_get_kernel_variant(sfg_solver s, int* variant);
  * runs the axis-sweep form, which scales each face flux by its area in FP64
  * where sfg_residual's tiles do it in FP32, so the two agree to FP32
  * round-off only.  It allocates nothing: the residual is formed in dev_r, and
- * its working memory (all of it used when dev_r overlaps dev_q) is one fixed array in
+ * its working memory (all of it used when dev_r overlaps dev_q or is not memory
+ * of the current device) is one fixed array in
  * the library's device image, of 32 + 5 * SFG_NOALLOC_MAX_NODES doubles
  * (~10 MiB), which every GPU that loads the library holds until the process
  * exits.

@@ -3,7 +3,7 @@
 //
 // The residual is formed in the caller's array.  The working memory (the step
 // clock the kernels read, the status word, and the residual of a call whose
-// two arrays overlap) lives in one file-scope __device__ array.  In host code `g_noalloc_scratch` only names a host-side
+// two arrays overlap or whose result is not on this device) lives in one file-scope __device__ array.  In host code `g_noalloc_scratch` only names a host-side
 // shadow of that array, never device memory: a kernel given it would fault or
 // silently use the wrong memory.  The device address is looked up once per
 // device with cudaGetSymbolAddress and that pointer is what the kernels get.
@@ -64,6 +64,25 @@ int scratch_address(double** out, bool** dirty) {
     *out = g_device_address[dev];
     *dirty = &g_header_dirty[dev];
     return SFG_OK;
+}
+
+// Whether kernels on the current device can write `bytes` at p themselves: this
+// device's memory (or managed memory) at both ends, on an 8-byte boundary.  Any
+// other destination (another device, host memory, an odd address) gets a copy,
+// which knows how or says why not.
+bool writable_here(const double* p, size_t bytes) {
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(double)) return false;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (const char* at : {reinterpret_cast<const char*>(p), reinterpret_cast<const char*>(p) + bytes - 1}) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, at) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeManaged && (a.type != cudaMemoryTypeDevice || a.device != dev)) return false;
+    }
+    return true;
 }
 
 struct RecipeParts {
@@ -149,11 +168,12 @@ extern "C" int sfg_residual_noalloc(const sfg_grid_desc* grid, const sfg_numeric
     Clock* clock = reinterpret_cast<Clock*>(base);
     unsigned* flags = reinterpret_cast<unsigned*>(base + 16);
     const size_t rbytes = sizeof(double) * 5 * (size_t)nodes;
-    // The residual goes straight to the caller's array; only when that overlaps
-    // the state does it take the fixed array and a copy.
+    // The residual goes straight to the caller's array; when that overlaps the
+    // state, or kernels here cannot write it, it takes the fixed array and a copy.
     const uintptr_t q0 = reinterpret_cast<uintptr_t>(dev_q), r0 = reinterpret_cast<uintptr_t>(dev_r);
     const bool overlap = q0 < r0 + rbytes && r0 < q0 + rbytes;
-    double* r = overlap ? base + kHeaderDoubles : dev_r;
+    const bool direct = !overlap && writable_here(dev_r, rbytes);
+    double* r = direct ? dev_r : base + kHeaderDoubles;
 
     cudaError_t e = cudaSuccess;
     if (*dirty) e = cudaMemsetAsync(base, 0, kHeaderDoubles * sizeof(double), st);
@@ -187,7 +207,7 @@ extern "C" int sfg_residual_noalloc(const sfg_grid_desc* grid, const sfg_numeric
         e = launch_sweep(rp->scheme, rp->flux, prec64, axis, g, sv, st);
         if (e != cudaSuccess) return noalloc_fail(SFG_ERR_CUDA, cudaGetErrorString(e));
     }
-    if (overlap) e = cudaMemcpyAsync(dev_r, r, rbytes, cudaMemcpyDeviceToDevice, st);
+    if (!direct) e = cudaMemcpyAsync(dev_r, r, rbytes, cudaMemcpyDeviceToDevice, st);
     unsigned host_flags = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&host_flags, flags, sizeof host_flags, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

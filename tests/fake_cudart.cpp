@@ -17,11 +17,13 @@
 namespace {
 
 std::map<const char*, size_t> g_live;           // allocations by address
+std::map<const char*, int> g_device;            // allocations of another device
 std::map<const void*, std::string> g_names;     // host stub -> device name
 struct Fail {
     int skip, times;
 };
 std::map<std::string, Fail> g_fail;             // call -> calls to let pass, then to fail
+const double* g_residual = nullptr;             // StageView::r of the last tile or sweep
 int g_violations = 0, g_capturing = 0, g_tiles = 0;
 std::string g_violation;
 cudaError_t g_last = cudaSuccess;
@@ -80,6 +82,13 @@ void check(const Launch& l) {
 #define API extern "C" __attribute__((visibility("default")))
 
 API void fake_fail(const char* call, int skip, int times) { g_fail[call] = {skip, times}; }
+API void* fake_alloc(size_t bytes, int device) {
+    void* p = nullptr;
+    cudaMalloc(&p, bytes);
+    if (device) g_device[(char*)p] = device;
+    return p;
+}
+API const void* fake_residual() { return g_residual; }
 API int fake_violations() { return g_violations; }
 API const char* fake_violation() { return g_violation.c_str(); }
 API int fake_tiles() { return g_tiles; }  // of the last batch stage launched
@@ -114,6 +123,8 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
 cudaError_t cudaLaunchKernel(const void* func, dim3, dim3, void** args, size_t, cudaStream_t) {
     if (cudaError_t e = failing("cudaLaunchKernel")) return e;
     Launch l{g_names[func], {}};
+    for (const char* k : {"tile1d_kernel", "tile2d_kernel", "sweep_x", "sweep_yz"})
+        if (l.name.find(k) != std::string::npos) g_residual = ((const sfg::StageView*)args[1])->r;
     for (const char* k : {"batch_stage_kernel", "batch_copy_kernel", "batch_law_kernel"})
         if (l.name.find(k) != std::string::npos)
             for (int i = 0; i < 3; ++i) l.p.push_back(*(const char**)args[i]);
@@ -143,9 +154,10 @@ cudaError_t cudaFreeHost(void* p) {
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind kind) {
     if (cudaError_t e = failing("cudaMemcpy")) return e;
-    if ((kind == cudaMemcpyHostToDevice || kind == cudaMemcpyDeviceToDevice) && !live(d, n)) violation("copy to memory that is not allocated");
-    else if ((kind == cudaMemcpyDeviceToHost || kind == cudaMemcpyDeviceToDevice) && !live(s, n)) violation("copy from memory that is not allocated");
-    else memmove(d, s, n);
+    if (((kind == cudaMemcpyHostToDevice || kind == cudaMemcpyDeviceToDevice) && !live(d, n)) ||
+        ((kind == cudaMemcpyDeviceToHost || kind == cudaMemcpyDeviceToDevice) && !live(s, n)))
+        return g_last = cudaErrorInvalidValue;
+    memmove(d, s, n);
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t) {
@@ -160,6 +172,16 @@ cudaError_t cudaGetSymbolAddress(void** p, const void*) {
     static void* image = nullptr;
     if (!image) cudaMalloc(&image, 16 << 20), memset(image, 0, 16 << 20);
     *p = image;
+    return cudaSuccess;
+}
+
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+    *a = {};
+    a->type = live(p, 1) ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
+    if (live(p, 1)) {
+        auto it = g_device.find((--g_live.upper_bound((const char*)p))->first);
+        a->device = it == g_device.end() ? 0 : it->second;
+    }
     return cudaSuccess;
 }
 

@@ -33,6 +33,8 @@ def fake(fake_lib, monkeypatch):
     monkeypatch.setattr(capi, "_lib", None)
     lib = capi.lib()
     lib.fake_violation.restype = ctypes.c_char_p
+    lib.fake_alloc.restype = lib.fake_residual.restype = ctypes.c_void_p
+    lib.fake_alloc.argtypes = [ctypes.c_size_t, ctypes.c_int]
     lib.fake_reset()
     yield lib
     assert lib.fake_violations() == 0, lib.fake_violation().decode()
@@ -94,3 +96,31 @@ def test_batch_list_that_cannot_be_published(fake):
             b.step(3, graph_steps=2)
     b.step(3, graph_steps=2)
     assert fake.fake_tiles() == tiles[1]
+
+
+@pytest.mark.parametrize("dim,precision", [(1, capi.PREC_FP64), (2, capi.PREC_FP64), (2, capi.PREC_FP32_FLUX),
+                                           (3, capi.PREC_FP64)])
+def test_noalloc_residual_goes_only_where_kernels_can_write(fake, dim, precision):
+    """The kernels get the caller's result array when it is this device's memory
+    on an 8-byte boundary, all of it; any other gets a copy, which refuses what
+    is not there."""
+    n = (20, 20 if dim > 1 else 1, 20 if dim > 2 else 1)
+    nodes = n[0] * n[1] * n[2]
+    bc = tuple(1 if d < dim else 0 for d in range(3))
+
+    def call(q, r):
+        capi.residual_noalloc(dim, n, (0.1, 0.1, 0.1), bc, bc, q, r, recipe="weno5Rusanov", precision=precision)
+        return fake.fake_residual()
+
+    q = fake.fake_alloc(40 * nodes, 0)
+    r, wide = fake.fake_alloc(40 * nodes, 0), fake.fake_alloc(40 * nodes + 8, 0)
+    assert call(q, r) == r and call(q, wide + 8) == wide + 8
+    for other in (fake.fake_alloc(40 * nodes, 1), wide + 4, q):
+        assert call(q, other) not in (other, r, q)
+        assert not any(ctypes.string_at(other, 40 * nodes))  # the fixed array's zeros, copied
+    host = np.ones(5 * nodes)
+    for missing in (fake.fake_alloc(40 * nodes - 8, 0), host.ctypes.data):
+        with pytest.raises(capi.SolverError) as e:
+            call(q, missing)
+        assert e.value.code == capi.ERR_CUDA and fake.fake_residual() != missing
+    assert host.all()

@@ -93,6 +93,41 @@ def test_noalloc_fp32_flux_within_fp32_tolerance(dim, n, h, bc, recipe):
     assert rel_linf(got, _oracle_residual(dim, n, h, bc, q, recipe)).max() <= TOL_F32, recipe
 
 
+@pytest.mark.parametrize("dim,n,bc,precision", [
+    (1, (700, 1, 1), capi.BC_PERIODIC, capi.PREC_FP64), (2, (61, 47, 1), capi.BC_TRANSMISSIVE, capi.PREC_FP64),
+    (2, (61, 47, 1), capi.BC_PERIODIC, capi.PREC_FP32_FLUX), (3, (20, 18, 16), capi.BC_TRANSMISSIVE, capi.PREC_FP64)])
+def test_noalloc_of_overlapping_arrays(dim, n, bc, precision):
+    """dev_r on top of dev_q, and a node's width into it: the residual of the
+    state as it was, by way of the fixed array."""
+    import torch
+    h = (0.02, 0.025, 0.03)
+    q = smooth_state(dim, n, seed=4)
+    want = _noalloc_residual(dim, n, h, bc, q, "weno5Rusanov", precision)
+    count = q.size
+    for shift in (0, 1, 3 * n[0]):
+        buf = torch.full((count + shift,), float("nan"), device="cuda", dtype=torch.float64)
+        buf[:count] = _device_soa(q).reshape(-1)
+        at = buf.data_ptr()
+        capi.residual_noalloc(dim, n, h, (bc,) * 3, (bc,) * 3, at, at + 8 * shift, recipe="weno5Rusanov",
+                              precision=precision)
+        got = buf[shift:].cpu().numpy().reshape(5, -1).T
+        np.testing.assert_array_equal(got, want)
+
+
+def test_noalloc_after_a_call_that_left_a_status():
+    """An invalid state is refused and leaves nothing behind for the next call."""
+    n, h = (61, 47, 1), (0.02, 0.025, 1.0)
+    q = smooth_state(2, n, seed=4)
+    want = _noalloc_residual(2, n, h, capi.BC_PERIODIC, q, "teno5Rusanov")
+    bad = q.copy()
+    bad[0, 20, 30, 4] = -1.0
+    for _ in range(2):
+        with pytest.raises(capi.SolverError) as e:
+            _noalloc_residual(2, n, h, capi.BC_PERIODIC, bad, "teno5Rusanov")
+        assert e.value.code == capi.ERR_STATE
+        np.testing.assert_array_equal(_noalloc_residual(2, n, h, capi.BC_PERIODIC, q, "teno5Rusanov"), want)
+
+
 def test_noalloc_rejects_grids_beyond_the_fixed_array():
     import torch
     n = (600, 600, 1)  # 360000 nodes > SFG_NOALLOC_MAX_NODES
