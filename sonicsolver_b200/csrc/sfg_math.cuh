@@ -470,9 +470,10 @@ __device__ __forceinline__ void indicators64(const double (&W)[5], double eps, d
 }
 
 // WENO5-JS: the folding of weno5_core on both sides, one division for the
-// two: with x/a and y/b needed, r = 1/(a b) gives x b r and y a r.  The
-// denominators lie in [1e-19, ~1e37] for any state the reference accepts, so
-// a b stays inside FP64 range.
+// two: with x/a and y/b needed, r = 1/(a b) gives x (b r) and y (a r): in that
+// order only a b has to stay in range (x b is larger by a difference), which it
+// does for differences up to 1e19; the denominators are at least 2.6e-21
+// (10 (4e-6)^4).
 __device__ __forceinline__ void weno5_pair64(const double (&W)[5], double& dl, double& dr, unsigned& flags) {
     double t[4], el[3], er[3];
     indicators64(W, 4e-6, t, el, er);
@@ -489,11 +490,11 @@ __device__ __forceinline__ void weno5_pair64(const double (&W)[5], double& dl, d
         num[side] = side ? fma(a, m0, fma(-b, v2, mul_rn(-c, u1))) : fma(a, m0, fma(-b, v1, mul_rn(-c, u2)));
     }
     const double inv = 1.0 / mul_rn(den[0], den[1]);
-    // positive and finite: 0 < high word < 0x7ff00000
-    if ((unsigned)(__double2hiint(inv) - 1) >= 0x7fefffffu) flags |= FLAG_NONFINITE;
+    // positive, normal and finite: 0x00100000 <= high word < 0x7ff00000
+    if ((unsigned)(__double2hiint(inv) - 0x00100000) >= 0x7fe00000u) flags |= FLAG_NONFINITE;
     const double r = mul_rn(inv, 1.0 / 6.0);
-    dl = mul_rn(mul_rn(num[0], den[1]), r);
-    dr = mul_rn(mul_rn(num[1], den[0]), r);
+    dl = mul_rn(num[0], mul_rn(den[1], r));
+    dr = mul_rn(num[1], mul_rn(den[0], r));
 }
 
 // WENO7-JS (SF_WENO7.cpp:41-98) in the same form, from the seven projected
@@ -581,14 +582,18 @@ __device__ __forceinline__ void teno5_pair64(const double (&W)[5], double& dl, d
     dl = fma(1.0 / 30.0, t[0], fma(-0.15, t[1], mul_rn(-0.05, t[2])));
     dr = fma(1.0 / 30.0, t[3], fma(-0.15, t[2], mul_rn(-0.05, t[1])));
     if (warp_all(teno_smooth_hi(e[0], tau[0]) && teno_smooth_hi(e[1], tau[1]))) return;
-    // tau / (e0 e1 e2) of both sides from one reciprocal; the products are >= 6e-119
+    // tau / (e0 e1 e2) of both sides from one reciprocal; the products are >=
+    // 6e-119.  The left one is taken with its tau at 2^-12 of its size, which
+    // leaves the pair the range it has with indicators b_k instead of 4 b_k
+    // (differences up to 4e25).
     double prod[2];
 #pragma unroll
     for (int side = 0; side < 2; ++side) prod[side] = mul_rn(e[side][0], mul_rn(e[side][1], e[side][2]));
+    prod[0] = mul_rn(0x1p-12, prod[0]);
     const double inv = 1.0 / mul_rn(prod[0], prod[1]);
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-        const double ti = mul_rn(mul_rn(tau[side], prod[1 - side]), inv);
+        const double ti = mul_rn(mul_rn(side ? tau[1] : mul_rn(0x1p-12, tau[0]), prod[1 - side]), inv);
         const double g0 = fma(ti, mul_rn(e[side][1], e[side][2]), 1.0);
         const double g1 = fma(ti, mul_rn(e[side][0], e[side][2]), 1.0);
         const double g2 = fma(ti, mul_rn(e[side][0], e[side][1]), 1.0);

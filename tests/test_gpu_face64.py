@@ -76,6 +76,35 @@ def test_weno7_beyond_the_folded_weights(scale, oracle):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("recipe,scale", [("weno5Rusanov", s) for s in (1e18, 4e18, 1e19)] +
+                                         [("teno5Rusanov", s) for s in (1e24, 1e25, 1e26)])
+def test_pair_denominators_keep_their_range(recipe, scale, oracle):
+    """Differences up to where the product of the two sides' denominators leaves
+    FP64 range (the scale is 3 to 4 times the differences); TENO5 on a field
+    rough everywhere (beside a uniform part its sixth powers leave the range
+    first, in the reference too)."""
+    nx = 41
+    q = _state("jump", nx, scale)
+    if recipe.startswith("teno5"):
+        rng = np.random.default_rng(3)
+        q = cases.conserved(scale * (1 + 0.3 * rng.random(nx)), 0.1 * rng.random(nx), 0.1 * rng.random(nx),
+                            0.1 * rng.random(nx), scale * (1 + 0.3 * rng.random(nx)))
+    q = q[None, None].copy()
+    h = (1.0 / (nx - 1), 1.0, 1.0)
+    bc = (int(recipe.startswith("teno5")), 0, 0)
+    case = cases.Case("f", 1, (nx, 1, 1), h, bc, bc, q, 1.4, 1.0, 0.5, recipe, "SSPRK3")
+    spec = oracle_spec(case, recipe=recipe)
+    want = from_oracle(spec, oracle.rhs(spec, SCHEME_OF[recipe[:5]], FLUX_OF["Rusanov"], to_oracle(spec, q)))
+    rho, u, v, w, p = cases.primitive(q)
+    fmax = (np.abs(q).max() + p.max()) * (np.abs(u) + np.sqrt(1.4 * p / rho)).max()
+    s = case.solver()
+    for variant in (0, 1):
+        s.variant = variant
+        err = np.abs(s.residual().reshape(q.shape) - want)[..., 1:-1, :]
+        assert err.max() <= 2 * 1000 * EPS * fmax / h[0]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dim,n", [(2, (40, 9, 1)), (2, (150, 37, 1)), (3, (33, 18, 40)), (3, (20, 70, 6)), (3, (70, 9, 33))])
 @pytest.mark.parametrize("bc", [0, 1])
 @pytest.mark.parametrize("recipe", ["weno3Roe", "weno5Rusanov", "weno7Rusanov"])
