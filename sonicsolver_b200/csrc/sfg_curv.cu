@@ -671,7 +671,7 @@ __device__ __forceinline__ void curv_face_dev32x2(const float (&d)[SchemeInfo<SC
     float dbar[5], qa[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        dbar[v] = 0.5f * (d[CL][v] + d[CL + 1][v]);
+        dbar[v] = fmaf(0.5f, d[CL + 1][v], 0.5f * d[CL][v]);  // as 0.5 (..): the halves are exact
         qa[v] = ref.q[v] + dbar[v];
     }
     const float pa = (gamma - 1.f) * (qa[4] - 0.5f * (qa[1] * qa[1] + qa[2] * qa[2] + qa[3] * qa[3]) * rcp_approx(qa[0]));
@@ -686,17 +686,17 @@ __device__ __forceinline__ void curv_face_dev32x2(const float (&d)[SchemeInfo<SC
         for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[2 * CL - k][v]), f2(d[k][v], d[2 * CL + 1 - k][v]));
         curv_project(e, x, E[k]);
     }
-    float mid[5], M[5];
+    float mid[5], M[5];  // half the middle difference
 #pragma unroll
-    for (int v = 0; v < 5; ++v) mid[v] = d[CL + 1][v] - d[CL][v];
+    for (int v = 0; v < 5; ++v) mid[v] = fmaf(0.5f, d[CL + 1][v], -0.5f * d[CL][v]);
     curv_project(e, mid, M);
     float2 w[5], dq[5], kept = f2(0.f), bad = f2(0.f);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        const float2 em = f2(M[v], -M[v]);
-        if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], em, bad, count, kept);
-        else if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], em, bad);
-        else w[v] = weno5_delta2(E[0][v], E[1][v], em, bad);
+        const float2 H = f2(M[v], -M[v]);
+        if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], H, bad, count, kept);
+        else if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, f2(0.f), bad);
+        else w[v] = weno5_delta2(E[0][v], E[1][v], H, f2(0.f), bad);
     }
     flag_bad(bad, flags);
     if constexpr (SCHEME == TENO5) {

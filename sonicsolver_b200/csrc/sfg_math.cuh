@@ -1040,22 +1040,27 @@ __device__ __forceinline__ float2 teno5_core2(float2 v0, float2 v1, float2 v2, f
 // FP32 WENO5 / TENO5 (WENO7 below) on a face's points in differences, the left and right
 // sides as the two lanes of a pair; the mathematics of indicators64.  With the
 // mirror-signed difference pairs E0 = (c1 - c0, c4 - c5), E1 = (c2 - c1,
-// c3 - c4), E2 = (c3 - c2, c2 - c3):
+// c3 - c4), E2 = (c3 - c2, c2 - c3) = 2 H:
 //   T1 = E1 - E0 = (t1, t4),  T2 = E2 - E1 = (t2, t3),  T2' = its swap
 //   4 b_k = 13/3 t^2 + r^2:  (T1, T1 + 2 E1), (T2, E1 + E2), (T2', T2' - 2 E2)
 //   p_k - mid = T1/3 - T2/2, -T2/6, -T2'/6
-// and the face states are d-bar + R (deltas).  Kept with N2 = -T2.
+// Kept with N2 = -T2.  Deltas from the midpoint of c2 and c3 make the face states
+// d-bar + R (deltas); with H added they are deltas from the side's nearer point,
+// and the states d2 + R (..), d3 + R (..).  The Cartesian faces take the second
+// form: there the rounding of d-bar, the same in both states, made residuals
+// 1.05 to 1.2 x less accurate than the form on points was (0.86 to 1.01 x now, at 2 % of a
+// Taylor-Green step).
 struct Diff2 {
     float2 T1, N2, N2s;  // (t1, t4), -(t2, t3), -(t3, t2)
     float2 e[3];         // eps + 4 b_k
 };
 
-__device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 E2, float eps) {
+__device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 H, float eps) {
     Diff2 d;
     d.T1 = sub2(E1, E0);
-    d.N2 = sub2(E1, E2);
+    d.N2 = fma2(f2(-2.f), H, E1);
     d.N2s = swap2(d.N2);
-    const float2 r0 = fma2(f2(2.f), E1, d.T1), r1 = add2(E1, E2), r2 = fma2(f2(2.f), E2, d.N2s);
+    const float2 r0 = fma2(f2(2.f), E1, d.T1), r1 = fma2(f2(2.f), H, E1), r2 = fma2(f2(4.f), H, d.N2s);
     const float2 c = f2(13.f / 3.f);
     const float2 b0 = fma2(mul2(c, d.T1), d.T1, f2(eps)), b1 = fma2(mul2(c, d.N2), d.N2, f2(eps));
     d.e[0] = fma2(r0, r0, b0);
@@ -1064,16 +1069,16 @@ __device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 E2, fl
     return d;
 }
 
-// WENO5-JS deltas of both sides.
-__device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 E2, float2& bad) {
-    const Diff2 d = indicators2(E0, E1, E2, 4.f * 1e-6f);
+// WENO5-JS deltas of both sides, `base` added: H or 0.
+__device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, float2 base, float2& bad) {
+    const Diff2 d = indicators2(E0, E1, H, 4.f * 1e-6f);
     const float2 s0 = mul2(d.e[0], d.e[0]), s1 = mul2(d.e[1], d.e[1]), s2 = mul2(d.e[2], d.e[2]);
     const float2 wa = mul2(s1, s2), wb = mul2(s0, s2), wc = mul2(s0, s1);  // weights 1 : 6 : 3
     const float2 den = fma2(f2(3.f), fma2(f2(2.f), wb, wc), wa);
     const float2 h = mul2(f2(0.5f), d.N2);
     const float2 num = fma2(wa, fma2(f2(1.f / 3.f), d.T1, h), fma2(wb, d.N2, mul2(wc, swap2(h))));
     bad = watch2(bad, den);  // den >= 10 eps^4 > 0 unless an input was not finite
-    return mul2(num, rcp2(den));
+    return fma2(num, rcp2(den), base);
 }
 
 // WENO7-JS deltas of both sides: weno7_pair64's form with E_k = (W_k, -W_{6-k}),
@@ -1082,7 +1087,8 @@ __device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 E2, 
 // leave FP32 range.  Against the scalar form, us a step: 700 x 520 267 -> 123,
 // 128 x 100 x 90 3314 -> 862 (with the 3-D tile's chunks), curved 500 x 400
 // 248 -> 88 (with the curved faces' other changes).
-__device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, float2 E3, float2& bad) {
+__device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, float2 H, float2 base, float2& bad) {
+    const float2 E3 = add2(H, H);
     const float2 T1 = sub2(E1, E0), T2 = sub2(E2, E1), T3 = sub2(E3, E2), T4 = swap2(T3), T5 = swap2(T2);
     const float2 G[4] = {sub2(T2, T1), sub2(T3, T2), sub2(T4, T3), sub2(T5, T4)};
     const float2 mid = mul2(f2(0.5f), add2(E2, E3));
@@ -1104,7 +1110,7 @@ __device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, 
         num = fma2(w, P[k], num);
     }
     bad = watch2(bad, den);
-    return mul2(num, rcp2(mul2(f2(12.f), den)));
+    return fma2(num, rcp2(mul2(f2(12.f), den)), base);
 }
 
 // TENO5 deltas of both sides.  With `count` (a launch-uniform switch: the
@@ -1112,9 +1118,9 @@ __device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, 
 // sub-stencils of each lane.  A lane that keeps all three sub-stencils takes
 // the linear weights' sum on the cut-off path too, so its bits do not depend
 // on the vote.
-__device__ __forceinline__ float2 teno5_delta2(float2 E0, float2 E1, float2 E2, float2& bad, bool count,
+__device__ __forceinline__ float2 teno5_delta2(float2 E0, float2 E1, float2 H, float2& bad, bool count,
                                                float2& kept) {
-    const Diff2 d = indicators2(E0, E1, E2, 0.f);
+    const Diff2 d = indicators2(E0, E1, H, 0.f);
     const float2 all = fma2(f2(1.f / 30.f), d.T1, fma2(f2(0.15f), d.N2, mul2(f2(0.05f), d.N2s)));
     if (warp_all(teno_smooth2(d.e))) {
         if (count) kept = add2(kept, f2(3.f));
@@ -1349,7 +1355,10 @@ __device__ __forceinline__ void phys_flux_dev2(const Ref32& r, const float2 d[5]
     c = f2(x.x * rsqrtf(x.x), x.y * rsqrtf(x.y));
 }
 
-template <int AX>
+// JUMP: the dissipation from d_R - d_L, as rusanov_dev has it, at one operation a
+// variable more (WENO7: without it 1-D residuals are 1.1 x less accurate than
+// that scheme's were).
+template <int AX, bool JUMP>
 __device__ __forceinline__ void rusanov_dev2(const Ref32& r, const float2 d[5], float gamma, float F[5],
                                              unsigned& flags, float scale = 1.f) {
     float2 f[5], un, c;
@@ -1359,6 +1368,10 @@ __device__ __forceinline__ void rusanov_dev2(const Ref32& r, const float2 d[5], 
     const float2 lr = f2(lam, -lam);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
+        if (JUMP) {
+            F[v] = fmaf(-lam, d[v].y - d[v].x, f[v].x + f[v].y) * (0.5f * scale);
+            continue;
+        }
         const float2 g = fma2(lr, d[v], f[v]);
         F[v] = (g.x + g.y) * (0.5f * scale);
     }
@@ -1373,7 +1386,7 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
     float dbar[5], qbar[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        dbar[v] = 0.5f * (d[CL][v] + d[CL + 1][v]);
+        dbar[v] = fmaf(0.5f, d[CL + 1][v], 0.5f * d[CL][v]);  // as 0.5 (..): the halves are exact
         qbar[v] = ref.q[v] + dbar[v];
     }
     Eigen<float> es;
@@ -1401,7 +1414,7 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
             w[v] = teno5_core2(P[0][v], P[1][v], P[2][v], bad, count, kept, all);
         }
     } else {
-        // WENO5, WENO7: mirror-signed difference pairs (d_{k+1} - d_k, d_{2CL-k} - d_{2CL+1-k}), projected
+        // WENO5, WENO7: mirror-signed difference pairs (d_{k+1} - d_k, d_{2CL-k} - d_{2CL+1-k}), projected.
         float2 E[CL][5];
 #pragma unroll
         for (int k = 0; k < CL; ++k) {
@@ -1410,15 +1423,15 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
             for (int v = 0; v < 5; ++v) x[v] = sub2(f2(d[k + 1][v], d[2 * CL - k][v]), f2(d[k][v], d[2 * CL + 1 - k][v]));
             to_characteristic2<AX>(e, x, E[k]);
         }
-        float m[5], M[5];  // the middle difference, the same on both sides up to its sign
+        float m[5], M[5];  // half the middle difference, the same on both sides up to its sign
 #pragma unroll
-        for (int v = 0; v < 5; ++v) m[v] = d[CL + 1][v] - d[CL][v];
+        for (int v = 0; v < 5; ++v) m[v] = fmaf(0.5f, d[CL + 1][v], -0.5f * d[CL][v]);
         project32<AX>(es, m, M);
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-            const float2 em = f2(M[v], -M[v]);
-            if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], em, bad);
-            else w[v] = weno5_delta2(E[0][v], E[1][v], em, bad);
+            const float2 H = f2(M[v], -M[v]);
+            if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, H, bad);
+            else w[v] = weno5_delta2(E[0][v], E[1][v], H, H, bad);
         }
     }
     flag_bad(bad, flags);
@@ -1428,9 +1441,10 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
     float2 dq[5], x2[5];
     from_characteristic2<AX>(e, w, dq);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) x2[v] = add2(f2(dbar[v]), dq[v]);  // (left, right) deviations from q_ref
+    for (int v = 0; v < 5; ++v)  // (left, right) deviations from q_ref
+        x2[v] = add2(SCHEME == TENO5 ? f2(dbar[v]) : f2(d[CL][v], d[CL + 1][v]), dq[v]);
     if constexpr (FLUX == RUSANOV) {
-        rusanov_dev2<AX>(ref, x2, gamma, F, flags, scale);
+        rusanov_dev2<AX, SCHEME == WENO7>(ref, x2, gamma, F, flags, scale);
     } else {
         float xl[5], xr[5];
 #pragma unroll

@@ -135,3 +135,29 @@ def test_fp32_taylor_green_tracks_fp64():
     assert rel_linf(q32, q64).max() <= 20 * STEP_TOL
     ke64, ke32 = cases.kinetic_energy(q64), cases.kinetic_energy(q32)
     assert abs(ke32 - ke64) <= 1e-6 * ke64
+
+
+@pytest.mark.parametrize("dim,n", [(1, (1500, 1, 1)), (2, (96, 80, 1))])
+@pytest.mark.parametrize("recipe", ["weno5Rusanov", "weno7Rusanov"])
+def test_difference_form_is_as_accurate_as_points(recipe, dim, n):
+    """FP32-flux residuals of WENO5 and WENO7, whose faces work on differences,
+    against FP64 ones: their error is that of rounding the same face states as
+    TENO5, whose face works on points.  Over eight smooth fields the ratio is
+    0.95 to 1.03; a face mean rounded once for both states makes it 1.09 to
+    1.13."""
+    h = tuple(1.0 / x if x > 1 else 1.0 for x in n)
+    bc = tuple(1 if d < dim else 0 for d in range(3))
+
+    def error(rec):
+        total = 0.0
+        for seed in range(8):
+            q = np.ascontiguousarray(smooth_state(dim, n, seed=seed, noise=0.0))
+            r = []
+            for prec in (capi.PREC_FP64, capi.PREC_FP32_FLUX):
+                s = capi.Solver(dim, n, h, bc, bc, recipe=rec, precision=prec)
+                s.upload(q)
+                r.append(s.residual())
+            total += np.linalg.norm(r[1] - r[0]) / np.linalg.norm(r[0])
+        return total
+
+    assert error(recipe) <= 1.06 * error("teno5Rusanov")
