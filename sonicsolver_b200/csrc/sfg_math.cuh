@@ -1052,31 +1052,37 @@ __device__ __forceinline__ float2 teno5_core2(float2 v0, float2 v1, float2 v2, f
 // Taylor-Green step).
 struct Diff2 {
     float2 T1, N2, N2s;  // (t1, t4), -(t2, t3), -(t3, t2)
-    float2 e[3];         // eps + 4 b_k
+    float2 e[3];         // 4 b_k
 };
 
-__device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 H, float eps) {
+__device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 H) {
     Diff2 d;
     d.T1 = sub2(E1, E0);
     d.N2 = fma2(f2(-2.f), H, E1);
     d.N2s = swap2(d.N2);
     const float2 r0 = fma2(f2(2.f), E1, d.T1), r1 = fma2(f2(2.f), H, E1), r2 = fma2(f2(4.f), H, d.N2s);
     const float2 c = f2(13.f / 3.f);
-    const float2 b0 = fma2(mul2(c, d.T1), d.T1, f2(eps)), b1 = fma2(mul2(c, d.N2), d.N2, f2(eps));
+    const float2 b0 = mul2(mul2(c, d.T1), d.T1), b1 = mul2(mul2(c, d.N2), d.N2);
     d.e[0] = fma2(r0, r0, b0);
     d.e[1] = fma2(r1, r1, b1);
     d.e[2] = fma2(r2, r2, swap2(b1));
     return d;
 }
 
-// WENO5-JS deltas of both sides, `base` added: H or 0.
+// WENO5-JS deltas of both sides, `base` added: H or 0.  Its indicators are b_k
+// themselves (r / 2 from H and h at no cost), not 4 b_k: the denominator, 10 b^4,
+// then leaves FP32 range at density jumps of 1.5e4 (6 (4 b)^4 of the form on
+// points did at 1.2e4, 10 (4 b)^4 at 8e3).
 __device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, float2 base, float2& bad) {
-    const Diff2 d = indicators2(E0, E1, H, 4.f * 1e-6f);
-    const float2 s0 = mul2(d.e[0], d.e[0]), s1 = mul2(d.e[1], d.e[1]), s2 = mul2(d.e[2], d.e[2]);
+    const float2 T1 = sub2(E1, E0), N2 = fma2(f2(-2.f), H, E1), h = mul2(f2(0.5f), N2), hs = swap2(h);
+    const float2 r0 = fma2(f2(0.5f), T1, E1), r1 = fma2(f2(0.5f), E1, H), r2 = fma2(f2(2.f), H, hs);
+    const float2 c = f2(13.f / 12.f);
+    const float2 b0 = fma2(mul2(c, T1), T1, f2(1e-6f)), b1 = fma2(mul2(c, N2), N2, f2(1e-6f));
+    const float2 e0 = fma2(r0, r0, b0), e1 = fma2(r1, r1, b1), e2 = fma2(r2, r2, swap2(b1));
+    const float2 s0 = mul2(e0, e0), s1 = mul2(e1, e1), s2 = mul2(e2, e2);
     const float2 wa = mul2(s1, s2), wb = mul2(s0, s2), wc = mul2(s0, s1);  // weights 1 : 6 : 3
     const float2 den = fma2(f2(3.f), fma2(f2(2.f), wb, wc), wa);
-    const float2 h = mul2(f2(0.5f), d.N2);
-    const float2 num = fma2(wa, fma2(f2(1.f / 3.f), d.T1, h), fma2(wb, d.N2, mul2(wc, swap2(h))));
+    const float2 num = fma2(wa, fma2(f2(1.f / 3.f), T1, h), fma2(wb, N2, mul2(wc, hs)));
     bad = watch2(bad, den);  // den >= 10 eps^4 > 0 unless an input was not finite
     return fma2(num, rcp2(den), base);
 }
@@ -1120,7 +1126,7 @@ __device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, 
 // on the vote.
 __device__ __forceinline__ float2 teno5_delta2(float2 E0, float2 E1, float2 H, float2& bad, bool count,
                                                float2& kept) {
-    const Diff2 d = indicators2(E0, E1, H, 0.f);
+    const Diff2 d = indicators2(E0, E1, H);
     const float2 all = fma2(f2(1.f / 30.f), d.T1, fma2(f2(0.15f), d.N2, mul2(f2(0.05f), d.N2s)));
     if (warp_all(teno_smooth2(d.e))) {
         if (count) kept = add2(kept, f2(3.f));

@@ -161,3 +161,20 @@ def test_difference_form_is_as_accurate_as_points(recipe, dim, n):
         return total
 
     assert error(recipe) <= 1.06 * error("teno5Rusanov")
+
+
+@pytest.mark.parametrize("scale", [1.0, 4000.0, 5000.0, 6000.0, 8000.0])
+def test_weno5_takes_density_jumps_of_dense_media(scale):
+    """Density jumps of 1.8 x scale: the folded FP32 weights (fourth powers of the
+    indicators) stay in range up to 1.4e4, so dense media run in SI units; the
+    residual is the FP64 path's to FP32 round-off, a few 1e-6 of its largest."""
+    n = 200
+    x = np.arange(n) / n
+    q = np.ascontiguousarray(cases.conserved(scale * (1 + 0.9 * np.sign(np.sin(10 * np.pi * x))), 0.1 + 0 * x, 0 * x,
+                                             0 * x, scale * (2 + 0.5 * np.cos(2 * np.pi * x))))
+    r = []
+    for prec in (capi.PREC_FP64, capi.PREC_FP32_FLUX):
+        s = capi.Solver(1, (n, 1, 1), (1 / n, 1.0, 1.0), (1, 0, 0), (1, 0, 0), recipe="weno5Rusanov", precision=prec)
+        s.upload(q)
+        r.append(s.residual())
+    assert np.abs(r[1] - r[0]).max() <= 5e-6 * np.abs(r[0]).max()
