@@ -1092,6 +1092,7 @@ static int capture_steps(sfg_solver_s* s, int n, cudaGraphExec_t* out) {
     int crc = SFG_OK;
     for (int i = 0; i < n && !crc; ++i) crc = enqueue_cfl_step(s, true, true);
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    if (crc && e == cudaSuccess) cudaGraphDestroy(g);
     if (crc) return crc;
     if (e != cudaSuccess) return fail(SFG_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     e = cudaGraphInstantiate(out, g, 0);
@@ -1103,13 +1104,18 @@ static int capture_steps(sfg_solver_s* s, int n, cudaGraphExec_t* out) {
     return SFG_OK;
 }
 
-// Captures `n` steps into (*graph, *steps) unless the slot holds them.
-static int keep_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* steps) {
-    if (*graph && *steps == n) return SFG_OK;
+// Captures `n` steps into (*graph, *steps) unless the slot holds them.  Whether
+// it holds them now: a graph saves launches and nothing else, so a run whose
+// graph cannot be had (the stream cannot be captured, no memory) goes on launch
+// by launch.
+static bool keep_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* steps) {
+    if (*graph && *steps == n) return true;
     if (*graph) cudaGraphExecDestroy(*graph);
     *graph = nullptr;
     *steps = n;
-    return capture_steps(s, n, graph);
+    if (capture_steps(s, n, graph) == SFG_OK) return true;
+    (void)cudaGetLastError();  // ours: the next launch must not report it
+    return false;
 }
 
 // sfg_advance outside the cluster kernel: graphs of `graph_steps` CFL steps,
@@ -1129,6 +1135,7 @@ static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms
     CUDA_TRY(cudaEventCreate(&e1));
     cudaEventRecord(e0, s->stream);
     int rc = enqueue_open_run(s);
+    bool graphs = true;
     for (bool first = true; !rc; first = false) {
         // steps left at most; after the first launches also by time, with two
         // to spare for a shrinking dt
@@ -1138,22 +1145,26 @@ static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms
         const int n = full ? graph_steps : std::max(1, int(left));
         cudaGraphExec_t ready = full ? (s->graph_steps == n ? s->graph : nullptr)
                                      : (s->rest_steps == n ? s->rest_graph : nullptr);
+        bool keep_rest = false;
         if (ready) {
             if (cudaGraphLaunch(ready, s->stream) != cudaSuccess)
                 rc = fail(SFG_ERR_CUDA, "graph launch: %s", cudaGetErrorString(cudaGetLastError()));
         } else {
             for (int i = 0; i < n && !rc; ++i) rc = enqueue_cfl_step(s, true, true);
             if (!rc && !full) {
-                if (s->rest_steps == n) {
-                    rc = keep_graph(s, n, &s->rest_graph, &s->rest_steps);
-                } else {
+                keep_rest = s->rest_steps == n;
+                if (!keep_rest) {
                     if (s->rest_graph) cudaGraphExecDestroy(s->rest_graph);
                     s->rest_graph = nullptr;
                     s->rest_steps = n;
                 }
             }
         }
-        if (!rc && (asked || full)) rc = keep_graph(s, graph_steps, &s->graph, &s->graph_steps);
+        const bool keep = (asked || full) && !(s->graph && s->graph_steps == graph_steps);
+        if (!rc && graphs) {
+            if (keep_rest) graphs = keep_graph(s, n, &s->rest_graph, &s->rest_steps);
+            if (keep && graphs) graphs = keep_graph(s, graph_steps, &s->graph, &s->graph_steps);
+        }
         unsigned bits = 0;
         if (!rc && (cudaMemcpyAsync(hc, s->clock, sizeof(Clock), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
                     cudaStreamSynchronize(s->stream) != cudaSuccess ||

@@ -218,7 +218,7 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t) {
     return cudaSuccess;
 }
 
-cudaError_t cudaGetLastError() {
+__attribute__((visibility("default"))) cudaError_t cudaGetLastError() {
     const cudaError_t e = g_last;
     g_last = cudaSuccess;
     return e;

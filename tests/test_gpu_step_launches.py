@@ -115,3 +115,17 @@ def test_cfl_step_is_one_step_of_a_run(name, time_recipe):
         b.step()
     assert e.value.code == capi.ERR_STATE and b.time() == (0.0, 0)
     np.testing.assert_array_equal(b.download(), before)
+
+
+@pytest.mark.gpu
+def test_stream_that_cannot_be_captured():
+    """The legacy default stream: runs of any length go launch by launch, with the
+    bits of a captured one, and leave no error behind."""
+    case, _ = _grid("tiles2d")
+    a, b = case.solver(), case.solver(stream=1)  # 1: cudaStreamLegacy
+    for kw in (dict(max_steps=9, graph_steps=4), dict(max_steps=70), dict(max_steps=2), dict(max_steps=2)):
+        (sa, da), (sb, db) = (s.advance(1e30, dt_capacity=70, **kw) for s in (a, b))
+        assert sa.steps == sb.steps == kw["max_steps"] and a.time() == b.time()
+        np.testing.assert_array_equal(da, db)
+        np.testing.assert_array_equal(a.download(), b.download())
+    case.solver().advance(1e30, max_steps=2)

@@ -124,3 +124,14 @@ def test_noalloc_residual_goes_only_where_kernels_can_write(fake, dim, precision
             call(q, missing)
         assert e.value.code == capi.ERR_CUDA and fake.fake_residual() != missing
     assert host.all()
+
+
+@pytest.mark.parametrize("call", [b"cudaStreamBeginCapture", b"cudaStreamEndCapture", b"cudaGraphInstantiate"])
+def test_run_without_a_graph(fake, call):
+    """A run whose graph cannot be had is a run all the same, and its failed
+    capture is not the next call's error."""
+    s = _grid(40).solver()
+    fake.fake_fail(call, 0, 1000)
+    for _ in range(2):
+        s.advance(1e30, max_steps=9, graph_steps=4)
+    assert fake.cudaGetLastError() == 0
