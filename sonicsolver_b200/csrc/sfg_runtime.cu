@@ -1127,13 +1127,18 @@ static bool keep_graph(sfg_solver_s* s, int n, cudaGraphExec_t* graph, int* step
 // Steps whose graph is not there yet are launched one by one too, and the graph
 // is captured behind them, while they run: at the first call of a caller that
 // names its graph length (`asked`), else when a run has that many steps to go.
-// `ms`: device time of the launches.
+// `ms`: device time of the launches, without the captures between them.
 static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms) {
     Clock* hc = s->host_clock;
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     cudaEventRecord(e0, s->stream);
+    *ms = 0.f;
+    auto lap = [&] {
+        float t = 0.f;
+        if (cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) *ms += t;
+    };
     int rc = enqueue_open_run(s);
     bool graphs = true;
     for (bool first = true; !rc; first = false) {
@@ -1161,7 +1166,9 @@ static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms
             }
         }
         const bool keep = (asked || full) && !(s->graph && s->graph_steps == graph_steps);
-        if (!rc && graphs) {
+        const bool capture = !rc && graphs && (keep || keep_rest);
+        if (capture) {
+            cudaEventRecord(e1, s->stream);  // the launches so far; the GPU may idle until the next ones
             if (keep_rest) graphs = keep_graph(s, n, &s->rest_graph, &s->rest_steps);
             if (keep && graphs) graphs = keep_graph(s, graph_steps, &s->graph, &s->graph_steps);
         }
@@ -1170,12 +1177,15 @@ static int advance_graph(sfg_solver_s* s, int graph_steps, bool asked, float* ms
                     cudaStreamSynchronize(s->stream) != cudaSuccess ||
                     cudaMemcpy(&bits, s->flags, sizeof bits, cudaMemcpyDeviceToHost) != cudaSuccess))
             rc = fail(SFG_ERR_CUDA, "advance: %s", cudaGetErrorString(cudaGetLastError()));
+        if (capture && !rc) {
+            lap();
+            cudaEventRecord(e0, s->stream);
+        }
         if (bits || !hc->active || hc->steps >= hc->max_steps) break;
     }
     if (!rc) {
         cudaEventRecord(e1, s->stream);
-        cudaEventSynchronize(e1);
-        cudaEventElapsedTime(ms, e0, e1);
+        lap();
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

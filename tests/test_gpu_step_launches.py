@@ -129,3 +129,15 @@ def test_stream_that_cannot_be_captured():
         np.testing.assert_array_equal(da, db)
         np.testing.assert_array_equal(a.download(), b.download())
     case.solver().advance(1e30, max_steps=2)
+
+
+@pytest.mark.gpu
+def test_device_time_leaves_the_capture_out():
+    """stats.device_ms of the run that captures its graph behind its first steps:
+    the steps' time, not that of capturing and instantiating 512 steps (7 ms,
+    against 0.2 for the two steps)."""
+    case, _ = _grid("tiles2d")
+    case.solver().advance(1e30, max_steps=2, graph_steps=512)  # kernels loaded
+    s = case.solver()
+    first, again = (s.advance(1e30, max_steps=2, graph_steps=512)[0].device_ms for _ in range(2))
+    assert 0.0 < first < 1.0 and 0.0 < again < 1.0
