@@ -388,8 +388,8 @@ double sfg_server_now(sfg_server s);
  * tiles, 3-D: 16 x 15 columns marching up 32-plane chunks), 2 = fused 2-D
  * tile kernel with 22 x 22 tiles; for 1-D grids variant 2 runs sfg_advance
  * in one thread-block cluster that steps the whole run on device (FP64, up to
- * 3968 nodes, no boundary laws, not Lax-Wendroff; other 1-D grids and single
- * stages use the 1-D tiles).  sfg_create picks 2 for 1-D, 1 for 2-D and 0
+ * 3968 nodes, forward Euler 7936, no boundary laws, not Lax-Wendroff; other 1-D
+ * grids and single stages use the 1-D tiles).  sfg_create picks 2 for 1-D, 1 for 2-D and 0
  * for 3-D grids; results agree across variants to round-off (FP32-flux: every
  * face takes the stage's one reference state; the sweeps scale face fluxes
  * by the area in FP64, the tiles in FP32), and the tile variants give the

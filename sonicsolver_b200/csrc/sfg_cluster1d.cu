@@ -16,18 +16,18 @@
 //     next lane by a warp shuffle, so a warp of 32 faces finishes up to 31
 //     nodes (the face at a warp boundary is computed by both warps);
 //   * one hardware cluster barrier (barrier.cluster: release / acquire at
-//     cluster scope) closes each stage; the last stage of a step also
-//     publishes each CTA's CFL maximum and status bits into CTA 0's shared
-//     memory, so every CTA reads the same dt and stop decision after that
-//     barrier (slots double-buffered by step parity: a slot is rewritten two
-//     steps later, after a barrier that every reader has passed).
+//     cluster scope) closes each stage; in the last stage of a step every warp
+//     also writes its CFL maximum and status bits into its slot of every CTA's
+//     shared memory, so every CTA finds the same dt and stop decision in its
+//     own after that barrier (slots double-buffered by step parity: a slot is
+//     rewritten two steps later, after a barrier that every reader has passed).
 // The clock arithmetic is that of finalize_dt_kernel and commit_kernel
 // (Time::Driver, SF_time.cpp:42-93), replayed in every thread; the face flux
 // and the stage update are the functions the other kernels use (face_flux,
 // finish_node).
 //
 // FP64 (the plain path), transmissive / periodic / frozen ends, all fluxes
-// but Lax-Wendroff, up to CL_MAX_NODES nodes.
+// but Lax-Wendroff, up to CL_MAX_NODES nodes (forward Euler: twice as many).
 #include <cooperative_groups.h>
 
 #include "sfg_internal.h"
@@ -41,9 +41,12 @@ namespace sfg {
 constexpr int CL_CTAS_MAX = 16;     // a cluster of 16 (opt-in size), or of 8 where 16 cannot be placed
 constexpr int CL_WARPS_MAX = 8;
 // One pass of eight warps (248 nodes) in each of 16 CTAs.  Beyond it a stage
-// takes two passes and the graph path is faster (us a step, cluster / graph:
-// WENO5 3000 nodes 12.2 / 19.8, 4000 19.9 / 20.1, 6000 20.9 / 20.3; WENO7 3000
-// 17.0 / 24.5, 4000 29.3 / 24.7; TENO5 3000 16.7 / 23.4, 4000 24.8 / 23.4).
+// takes two passes and the graph path is as fast or faster for one scheme or
+// another (us a step at 4100 nodes, cluster / graph: WENO5 17.9 / 20.2, WENO7 27.6 /
+// 24.7, TENO5 25.0 / 23.9; at 3968 10.8 / 19.7, 15.5 / 23.8, 14.3 / 23.2).  An Euler
+// step is one stage here and a stage, a copy and the launches' latency there:
+// two passes win for every scheme (4100: WENO5 7.0 / 12.1, WENO7 10.2 / 13.5;
+// 7900: 7.5 / 11.8, 10.5 / 13.1), three do not (8500: WENO7 14.3 / 13.5).
 constexpr int CL_MAX_NODES = CL_CTAS_MAX * 31 * CL_WARPS_MAX;
 
 namespace {
@@ -314,9 +317,9 @@ static cudaError_t launch_cluster_f(int flux, const GridView& g, const ClusterRu
 }
 
 // Whether a 1-D grid can run in the cluster kernel.
-bool cluster1d_eligible(const GridView& g, int flux, int prec64) {
+bool cluster1d_eligible(const GridView& g, int flux, int prec64, int time_id) {
     return g.dim == 1 && prec64 && flux != LAXW && !g.curv && g.hi[0] - g.lo[0] >= 8 &&
-           g.n[0] <= CL_MAX_NODES;
+           g.n[0] <= (time_id == T_EULER ? 2 : 1) * CL_MAX_NODES;
 }
 
 cudaError_t launch_cluster1d(int scheme, int flux, const GridView& g, const ClusterRun& run, cudaStream_t st) {

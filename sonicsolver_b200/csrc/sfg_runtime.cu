@@ -47,7 +47,7 @@ cudaError_t launch_curv_geometry(const GridView& g, const double* nm, double* co
 cudaError_t launch_curv_stage(int scheme, int flux, int prec64, int tiles, const GridView& g, const StageView& sv,
                               double* fl, cudaStream_t st);
 cudaError_t launch_teno_flips(const GridView& g, const double* q, unsigned long long* out, cudaStream_t st);
-bool cluster1d_eligible(const GridView& g, int flux, int prec64);
+bool cluster1d_eligible(const GridView& g, int flux, int prec64, int time_id);
 cudaError_t launch_cluster1d(int scheme, int flux, const GridView& g, const ClusterRun& run, cudaStream_t st);
 }  // namespace sfg
 
@@ -1272,7 +1272,7 @@ int sfg_advance(sfg_solver s, double t_end, int64_t max_steps, double write_inte
     float ms = 0.f;
     bool ran = false;
     if (s->grid.dim == 1 && s->variant == 2 && !s->has_laws &&
-        cluster1d_eligible(s->gv, s->recipe->flux, s->num.precision == SFG_PREC_FP64)) {
+        cluster1d_eligible(s->gv, s->recipe->flux, s->num.precision == SFG_PREC_FP64, s->num.time_recipe)) {
         rc = advance_cluster(s, &ms, &ran);
         if (rc) return rc;
     }

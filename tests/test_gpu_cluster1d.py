@@ -97,17 +97,24 @@ def test_cluster_run_matches_oracle_and_graph_path(recipe, time_recipe, ends):
     assert rel_linf(q2[:, :, sl], ref.reshape(q.shape)[:, :, sl]).max() <= 1e-10
 
 
-@pytest.mark.parametrize("n,ends", [(10, "transmissive"), (11, "periodic"), (12, "frozen-low"), (17, "transmissive"),
-                                    (65, "periodic"), (2049, "transmissive"), (8192, "periodic")])
-def test_grid_sizes_split_over_the_cluster(n, ends):
+@pytest.mark.parametrize("n,ends,time_recipe", [
+    (10, "transmissive", "SSPRK3"), (11, "periodic", "SSPRK3"), (12, "frozen-low", "SSPRK3"), (17, "transmissive", "SSPRK3"),
+    (65, "periodic", "SSPRK3"), (129, "transmissive", "SSPRK3"), (130, "transmissive", "classicalRK4"),
+    (1984, "periodic", "SSPRK3"), (1985, "periodic", "classicalRK4"), (2049, "transmissive", "SSPRK3"),
+    (3967, "frozen-low", "SSPRK3"), (3968, "periodic", "classicalRK4"), (3969, "periodic", "forwardEuler"),
+    (7936, "transmissive", "forwardEuler")])
+def test_grid_sizes_split_over_the_cluster(n, ends, time_recipe):
     """From the smallest eligible grid (8 solved nodes: one per CTA, trailing
-    CTAs idle for the shorter chunks) to the largest (8192 nodes)."""
-    q = _state(n, seed=3, shock=True)
-    steps = 20
-    (st2, dts2, q2), (st1, dts1, q1) = _cluster_and_graph(n, ends, "weno5Rusanov", "SSPRK3", q, steps)
+    CTAs idle for the shorter chunks) over 8 and 16 CTAs (127 and 128 solved
+    nodes), four and eight warps (124 and 125 nodes a CTA) and one and two
+    passes (248 and 249) to the largest (3968 nodes, Euler 7936)."""
+    euler = time_recipe == "forwardEuler"
+    q = _state(n, seed=3, shock=not euler)
+    steps = 12 if euler else 20
+    (st2, dts2, q2), (st1, dts1, q1) = _cluster_and_graph(n, ends, "weno5Rusanov", time_recipe, q, steps)
     _same(dts2, dts1, 1e-11)
     _same(q2, q1, 1e-10)
-    dts_ref, _, ref = _oracle_run(n, ends, "weno5Rusanov", "SSPRK3", q, steps)
+    dts_ref, _, ref = _oracle_run(n, ends, "weno5Rusanov", time_recipe, q, steps)
     np.testing.assert_allclose(dts2, dts_ref, rtol=1e-11, atol=0)
     sl = slice(1, -1) if ends == "transmissive" else slice(None)
     assert rel_linf(q2[:, :, sl], ref.reshape(q.shape)[:, :, sl]).max() <= 1e-10
