@@ -38,7 +38,7 @@ namespace cg = cooperative_groups;
 
 namespace sfg {
 
-constexpr int CL_CTAS_MAX = 16;     // a cluster of 16 (opt-in size), or of 8 where 16 cannot be placed
+constexpr int CL_CTAS_MAX = 16;     // the opt-in cluster size
 constexpr int CL_WARPS_MAX = 8;
 // One pass of eight warps (248 nodes) in each of 16 CTAs.  Beyond it a stage
 // takes two passes and the graph path is as fast or faster for one scheme or
@@ -297,11 +297,7 @@ static cudaError_t launch_cluster_n(const GridView& g, const ClusterRun& run, cu
 template <int SCHEME, int FLUX>
 static cudaError_t launch_cluster(const GridView& g, const ClusterRun& run, cudaStream_t st) {
     // 16 CTAs from 8 nodes each on: below that there is nothing to spread
-    if (g.hi[0] - g.lo[0] >= CL_CTAS_MAX * 8) {
-        const cudaError_t e = launch_cluster_n<CL_CTAS_MAX, SCHEME, FLUX>(g, run, st);
-        if (e == cudaSuccess) return e;
-        (void)cudaGetLastError();  // not placed: nothing ran
-    }
+    if (g.hi[0] - g.lo[0] >= CL_CTAS_MAX * 8) return launch_cluster_n<CL_CTAS_MAX, SCHEME, FLUX>(g, run, st);
     return launch_cluster_n<8, SCHEME, FLUX>(g, run, st);
 }
 
