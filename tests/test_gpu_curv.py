@@ -20,8 +20,11 @@ GRIDS = {1: ((61, 1, 1), (1.0 / 60, 1.0, 1.0)), 2: ((40, 33, 1), (0.025, 0.03, 1
          3: ((14, 12, 11), (0.07, 0.08, 0.09))}
 
 
-def _pair(dim, bc, recipe, time_recipe="SSPRK3", seed=0, shock=False, cfl=0.45, precision=capi.PREC_FP64):
-    n, h = GRIDS[dim]
+LARGE = ((251, 203, 1), (0.004, 0.005, 1.0))  # 464 blocks of 16 x 7: 22 x 22 tiles in both precisions
+
+
+def _pair(dim, bc, recipe, time_recipe="SSPRK3", seed=0, shock=False, cfl=0.45, precision=capi.PREC_FP64, grid=None):
+    n, h = grid or GRIDS[dim]
     scheme, _ = split_recipe(recipe)
     ng = NG_OF[scheme]
     bcs = (bc,) * 3
@@ -249,3 +252,50 @@ def test_curvilinear_2d_face_launches_and_fused_tiles(variant, precision, bc):
         s.step(dt)
     got = s.download().reshape(spec.interior(Q).shape)
     assert rel_linf(got, from_oracle(spec, Q)).max() <= (TOL if fp64 else 2e-6)
+
+
+@pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_FP32_FLUX])
+@pytest.mark.parametrize("bc", [capi.BC_TRANSMISSIVE, capi.BC_PERIODIC])
+@pytest.mark.parametrize("recipe", ["weno3Rusanov", "weno5Rusanov", "weno5Roe", "teno5Rusanov", "weno7Rusanov", "weno7Roe"])
+def test_large_curved_grids_match_oracle(recipe, bc, precision):
+    """A curved 2-D grid of more 16 x 7 blocks than are resident at once (22 x 22
+    tiles, ragged at both ends): residual and one step.  The FP32 residual's
+    error is the rounding of a flux over h, its size a flux's gradient: on 251
+    nodes instead of 40 the same field changes 6.3 times less per node, so the
+    5e-6 of the 40 x 33 grid are 3.2e-5 here."""
+    s, spec, q = _pair(2, bc, recipe, seed=51, precision=precision, grid=LARGE)
+    scheme, flux = split_recipe(recipe)
+    fp64 = precision == capi.PREC_FP64
+    Q = to_oracle(spec, q)
+    sl = _solved(spec, bc)
+    if fp64 or scheme != "teno5":
+        R_ref = from_oracle(spec, po.rhs(spec, SCHEME_OF[scheme], FLUX_OF[flux], Q))
+        assert rel_linf(s.residual().reshape(R_ref.shape)[sl], R_ref[sl]).max() <= (TOL if fp64 else 3.2e-5)
+    dt = po.dt(spec, Q, 0.45)
+    po.Stepper(spec, SCHEME_OF[scheme], FLUX_OF[flux], po.SSPRK3).step(Q, dt)
+    s.step(dt)
+    want = from_oracle(spec, Q)
+    err = rel_linf(s.download().reshape(want.shape)[sl], want[sl]).max()
+    assert err <= (TOL if fp64 else 1e-4 if scheme == "teno5" else 2e-6)
+
+
+@pytest.mark.parametrize("precision", [capi.PREC_FP64, capi.PREC_FP32_FLUX])
+@pytest.mark.parametrize("recipe", ["weno3Roe", "weno5Rusanov", "teno5Rusanov", "teno5Roe", "weno7Rusanov"])
+def test_curved_tile_shapes_give_the_same_bits(recipe, precision):
+    """A periodic curved grid (16 x 7 tiles) against itself repeated 6 x 5 times
+    (22 x 22 tiles): every node sees the same values, so three steps agree to
+    the bit."""
+    n, h = (48, 42, 1), (0.02, 0.025, 1.0)
+    bcs = (capi.BC_PERIODIC,) * 3
+    M = curvilinear_metrics(2, n, h, 0, seed=6)
+    q = smooth_state(2, n, seed=6, shock=not recipe.startswith("teno5"))
+    out = []
+    for rep in ((1, 1, 1, 1), (1, 5, 6, 1)):
+        big = (n[0] * rep[2], n[1] * rep[1], 1)
+        s = capi.Solver(2, big, h, bcs, bcs, recipe=recipe, cfl=0.45, precision=precision)
+        s.set_metrics(np.ascontiguousarray(np.tile(M, rep)))
+        s.upload(np.ascontiguousarray(np.tile(q, rep)))
+        _, dts = s.advance(1e30, max_steps=3, dt_capacity=3)
+        out.append((dts, s.download().reshape(1, big[1], big[0], 5)))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(np.tile(out[0][1], (1, 5, 6, 1)), out[1][1])
