@@ -225,7 +225,7 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(CL_WARPS_MAX * 32
                         for (int v = 0; v < 5; ++v) st[k][v] = src[v * per];
                     }
                     double F[5];
-                    face_flux<0, SCHEME, FLUX, double>(st, g.gamma, F, flags, cut, 0.0);
+                    face_flux<0, SCHEME, FLUX>(st, g.gamma, F, flags, cut, 0.0);
 #pragma unroll
                     for (int v = 0; v < 5; ++v) Fa[v] = F[v] * g.area[0];
                     if (SCHEME == TENO5 && (lane < share || f == s1)) cores += 10;

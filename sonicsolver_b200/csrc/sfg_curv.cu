@@ -176,30 +176,23 @@ __device__ __forceinline__ void right_col(const CharBasisT<T>& e, T (&r)[5]) {
     }
 }
 
-// Field K of the characteristic reconstruction: project the stencil on row
-// K, reconstruct both sides, add column K times the results to qL / qR.
-template <int K, int SCHEME, int NST, int W, typename T>
-__device__ __forceinline__ void recon_field(const CharBasisT<T>& e, const T (&st)[NST][5], T (&qL)[5], T (&qR)[5],
-                                            unsigned& flags, unsigned& cut) {
+// Field K of a WENO3 face: project the stencil on row K, reconstruct both sides,
+// add column K times the results to qL / qR.
+template <int K, typename T>
+__device__ __forceinline__ void recon_field(const CharBasisT<T>& e, const T (&st)[4][5], T (&qL)[5], T (&qR)[5],
+                                            unsigned& flags) {
     T row[5];
     left_row<K, T>(e, row);
-    T ch[NST];
+    T ch[4];
 #pragma unroll
-    for (int s = 0; s < NST; ++s) {
+    for (int s = 0; s < 4; ++s) {
         T acc = T(0);
 #pragma unroll
         for (int k = 0; k < 5; ++k) acc += row[k] * st[s][k];
         ch[s] = acc;
     }
-    T wl, wr;
-    T sl[8], sr[8];
-#pragma unroll
-    for (int s = 0; s < W; ++s) {
-        sl[s] = ch[s];
-        sr[s] = ch[NST - 1 - s];
-    }
-    wl = recon_core<SCHEME, T>(sl, flags, cut);
-    wr = recon_core<SCHEME, T>(sr, flags, cut);
+    const T sl[4] = {ch[0], ch[1], ch[2], ch[3]}, sr[4] = {ch[3], ch[2], ch[1], ch[0]};
+    const T wl = weno3_core<T>(sl, flags), wr = weno3_core<T>(sr, flags);
     T col[5];
     right_col<K, T>(e, col);
 #pragma unroll
@@ -207,6 +200,16 @@ __device__ __forceinline__ void recon_field(const CharBasisT<T>& e, const T (&st
         qL[r] += col[r] * wl;
         qR[r] += col[r] * wr;
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void recon_fields(const CharBasisT<T>& e, const T (&st)[4][5], T (&qL)[5], T (&qR)[5],
+                                             unsigned& flags) {
+    recon_field<0, T>(e, st, qL, qR, flags);
+    recon_field<1, T>(e, st, qL, qR, flags);
+    recon_field<2, T>(e, st, qL, qR, flags);
+    recon_field<3, T>(e, st, qL, qR, flags);
+    recon_field<4, T>(e, st, qL, qR, flags);
 }
 
 __device__ __forceinline__ void gemv5(const double (&M)[5][5], const double (&x)[5], double (&y)[5]) {
@@ -581,7 +584,7 @@ __device__ __forceinline__ void curv_back(const CurvEig<S>& e, const T (&w)[5], 
 template <int SCHEME, int FLUX>
 __device__ __forceinline__ void curv_face64(const double (&st)[SchemeInfo<SCHEME>::NST][5], const double (&n)[3],
                                             double gamma, double (&F)[5], unsigned& flags, unsigned& cut) {
-    constexpr int NST = SchemeInfo<SCHEME>::NST, W = SchemeInfo<SCHEME>::W;
+    constexpr int NST = SchemeInfo<SCHEME>::NST;
     double qavg[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) qavg[v] = 0.5 * (st[NST / 2 - 1][v] + st[NST / 2][v]);
@@ -618,11 +621,7 @@ __device__ __forceinline__ void curv_face64(const double (&st)[SchemeInfo<SCHEME
     } else {
         CharBasis e;
         char_basis_n(qavg, n, gamma, e, flags);
-        recon_field<0, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<1, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<2, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<3, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
-        recon_field<4, SCHEME, NST, W, double>(e, st, qL, qR, flags, cut);
+        recon_fields<double>(e, st, qL, qR, flags);
     }
     flux_n<FLUX>(qL, qR, n, gamma, F, flags);
 }
@@ -727,23 +726,18 @@ __device__ __forceinline__ void curv_face_dev32(const float (&d)[SchemeInfo<SCHE
                                                 unsigned& cut, bool count) {
     if constexpr (SCHEME != WENO3) {
         curv_face_dev32x2<SCHEME, FLUX>(d, ref, n, gamma, F, flags, cut, count);
-        return;
-    }
-    constexpr int NST = SchemeInfo<SCHEME>::NST, W = SchemeInfo<SCHEME>::W, CL = NST / 2 - 1;
-    float qa[5];
+    } else {
+        float qa[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) qa[v] = ref.q[v] + 0.5f * (d[CL][v] + d[CL + 1][v]);
-    const float pa = (gamma - 1.f) * (qa[4] - 0.5f * (qa[1] * qa[1] + qa[2] * qa[2] + qa[3] * qa[3]) / qa[0]);
-    if (!(qa[0] > 0.f) || !(pa > 0.f)) flags |= FLAG_PRESSURE;
-    CharBasisT<float> e;
-    char_basis_p<float>(qa, pa, n, gamma, e);
-    float dL[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, dR[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    recon_field<0, SCHEME, NST, W, float>(e, d, dL, dR, flags, cut);
-    recon_field<1, SCHEME, NST, W, float>(e, d, dL, dR, flags, cut);
-    recon_field<2, SCHEME, NST, W, float>(e, d, dL, dR, flags, cut);
-    recon_field<3, SCHEME, NST, W, float>(e, d, dL, dR, flags, cut);
-    recon_field<4, SCHEME, NST, W, float>(e, d, dL, dR, flags, cut);
-    flux_dev_n<FLUX>(ref, dL, dR, n, gamma, F, flags);
+        for (int v = 0; v < 5; ++v) qa[v] = ref.q[v] + 0.5f * (d[1][v] + d[2][v]);
+        const float pa = (gamma - 1.f) * (qa[4] - 0.5f * (qa[1] * qa[1] + qa[2] * qa[2] + qa[3] * qa[3]) / qa[0]);
+        if (!(qa[0] > 0.f) || !(pa > 0.f)) flags |= FLAG_PRESSURE;
+        CharBasisT<float> e;
+        char_basis_p<float>(qa, pa, n, gamma, e);
+        float dL[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, dR[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        recon_fields<float>(e, d, dL, dR, flags);
+        flux_dev_n<FLUX>(ref, dL, dR, n, gamma, F, flags);
+    }
 }
 
 }  // namespace

@@ -60,7 +60,7 @@ __device__ __forceinline__ void teno_flips_face(const GridView& g, const double*
             for (int s = 0; s < 5; ++s) a[s] = side ? c64[NST - 1 - s][v] : c64[s][v];
             double a0, a1, a2;
             teno_betas<double>(a, a0, a1, a2);
-            const int m64 = Teno<double>::keep_mask(a0, a1, a2, fl);
+            const int m64 = teno_keep64(a0, a1, a2, fl);
             int m32 = 0;
             for (int k = 0; k < 3; ++k) m32 |= int((side ? keep[k].y : keep[k].x) != 0.f) << k;
             dec += 3;

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128, SCHEME == WENO7 && sizeof(T) == sizeof(do
                 for (int v = 0; v < 5; ++v) d[s][v] = float(st[s][v] - qref[v]);
             face_flux_dev32<0, SCHEME, FLUX>(d, ref, float(g.gamma), Ft, flags, cut, sv.counters != nullptr);
         } else {
-            face_flux<0, SCHEME, FLUX, T>(st, T(g.gamma), Ft, flags, cut, T(FLUX == LAXW ? sv.clock->dt / g.h[0] : 0.0));
+            face_flux<0, SCHEME, FLUX>(st, g.gamma, Ft, flags, cut, FLUX == LAXW ? sv.clock->dt / g.h[0] : 0.0);
         }
 #pragma unroll
         for (int v = 0; v < 5; ++v) F[v] = double(Ft[v]) * g.area[0];
@@ -229,8 +229,7 @@ __global__ void __launch_bounds__(128, 4) sweep_yz(GridView g, StageView sv, int
                 for (int v = 0; v < 5; ++v) next[v] = __ldg(at + v * vs);
             }
             T Ft[5];
-            face_flux<AX, SCHEME, FLUX, T>(st, T(g.gamma), Ft, flags, cut,
-                                           T(FLUX == LAXW ? sv.clock->dt / g.h[AX] : 0.0));
+            face_flux<AX, SCHEME, FLUX>(st, g.gamma, Ft, flags, cut, FLUX == LAXW ? sv.clock->dt / g.h[AX] : 0.0);
             if (SCHEME == TENO5) cores += 10;
             double F[5];
 #pragma unroll

@@ -21,10 +21,10 @@
 namespace sfg {
 
 template <int SCHEME> struct SchemeInfo;
-template <> struct SchemeInfo<WENO3> { static constexpr int NST = 4, W = 4; };
-template <> struct SchemeInfo<WENO5> { static constexpr int NST = 6, W = 5; };
-template <> struct SchemeInfo<TENO5> { static constexpr int NST = 6, W = 5; };
-template <> struct SchemeInfo<WENO7> { static constexpr int NST = 8, W = 7; };
+template <> struct SchemeInfo<WENO3> { static constexpr int NST = 4; };
+template <> struct SchemeInfo<WENO5> { static constexpr int NST = 6; };
+template <> struct SchemeInfo<TENO5> { static constexpr int NST = 6; };
+template <> struct SchemeInfo<WENO7> { static constexpr int NST = 8; };
 
 // Momentum slots (1 + x/y/z) of the normal n and tangents l, m per axis, with
 // the sign of the tangent along that slot.
@@ -162,37 +162,13 @@ __device__ __forceinline__ void from_characteristic(const Eigen<T>& e, const T w
 }
 
 // ---------------------------------------------------------------------------
-// Scalar reconstruction cores.  v[0..W-1] is the upwind-ordered stencil.
+// Scalar reconstruction cores on points: WENO3, and WENO7 where its form in
+// differences is out of range.  v[0..W-1] is the upwind-ordered stencil.
 // ---------------------------------------------------------------------------
 
-// WENO5-JS (SF_WENO5.cpp:42-62): weights d_k/(eps+b_k)^2 normalised.  The
-// three alpha divisions and the normalisation are folded into one division:
-// with s_k = (eps+b_k)^2, w_k = d_k * prod_{j!=k} s_j, result = sum w_k p_k / sum w_k.
-template <typename T>
-__device__ __forceinline__ T weno5_core(const T* v, unsigned& flags) {
-    const T p0 = T(2) * v[0] - T(7) * v[1] + T(11) * v[2];
-    const T p1 = -v[1] + T(5) * v[2] + T(2) * v[3];
-    const T p2 = T(2) * v[2] + T(5) * v[3] - v[4];
-    const T t0 = v[0] - T(2) * v[1] + v[2], r0 = v[0] - T(4) * v[1] + T(3) * v[2];
-    const T t1 = v[1] - T(2) * v[2] + v[3], r1 = v[1] - v[3];
-    const T t2 = v[2] - T(2) * v[3] + v[4], r2 = T(3) * v[2] - T(4) * v[3] + v[4];
-    const T c13 = T(13.0 / 12.0);
-    const T b0 = c13 * (t0 * t0) + T(0.25) * (r0 * r0);
-    const T b1 = c13 * (t1 * t1) + T(0.25) * (r1 * r1);
-    const T b2 = c13 * (t2 * t2) + T(0.25) * (r2 * r2);
-    const T eps = T(1e-6);
-    const T s0 = (eps + b0) * (eps + b0);
-    const T s1 = (eps + b1) * (eps + b1);
-    const T s2 = (eps + b2) * (eps + b2);
-    const T w0 = T(0.1) * (s1 * s2);
-    const T w1 = T(0.6) * (s0 * s2);
-    const T w2 = T(0.3) * (s0 * s1);
-    const T den = w0 + w1 + w2;
-    if (!(den > T(0)) || !finite_(den)) flags |= FLAG_NONFINITE;
-    return div_<T>(w0 * p0 + w1 * p1 + w2 * p2, T(6) * den);
-}
-
-// WENO3-JS (SF_WENO3.cpp:42-57), same folding.
+// WENO3-JS (SF_WENO3.cpp:42-57): weights d_k/(eps+b_k)^2 normalised, the alpha
+// divisions and the normalisation folded into one: with s_k = (eps+b_k)^2, w_k =
+// d_k * prod_{j!=k} s_j, result = sum w_k p_k / sum w_k.
 template <typename T>
 __device__ __forceinline__ T weno3_core(const T* v, unsigned& flags) {
     const T p0 = -v[0] + T(5) * v[1] + T(2) * v[2];
@@ -254,29 +230,19 @@ __device__ __forceinline__ T weno7_core(const T* v, unsigned& flags) {
     return div_<T>(a0 * p0 + a1 * p1 + a2 * p2 + a3 * p3, T(12) * sum);
 }
 
-// TENO5 (SF_TENO5.cpp:44-92): C = 1, q = 6, eps = 1e-40, CT = 1e-5.
-// keep_mask() is the cut-off decision alone (bit k set = sub-stencil k kept);
-// core() is the reconstruction built on it.  `cut` accumulates the number of
-// cut sub-stencils.
+// TENO5 (SF_TENO5.cpp:44-92): C = 1, q = 6, eps = 1e-40, CT = 1e-5.  `cut`
+// accumulates the number of cut sub-stencils.
 //
-// The sub-stencil polynomials and smoothness indicators are written with
-// every rounding fixed (fma where two operations fuse, the _rn intrinsics
-// where they must not): left to the compiler, products shared between them
-// (2 v2, 3 v2, ...) fuse or not depending on the code around them, so the
-// same inputs could round differently in two call sites.
+// Everything below is written with every rounding fixed (fma where two
+// operations fuse, the _rn intrinsics where they must not): left to the
+// compiler, products shared between terms fuse or not depending on the code
+// around them, so the same inputs could round differently in two call sites.
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 
-// 6 x the three sub-stencil reconstructions (p_k of the reference).
-template <typename T>
-__device__ __forceinline__ void teno_polys(const T* v, T& p0, T& p1, T& p2) {
-    p0 = fma(T(11), v[2], fma(T(-7), v[1], mul_rn(T(2), v[0])));
-    p1 = fma(T(2), v[3], fma(T(5), v[2], -v[1]));
-    p2 = add_rn(fma(T(5), v[3], mul_rn(T(2), v[2])), -v[4]);
-}
-
+// Smoothness indicators of the three sub-stencils of v[0..4].
 template <typename T>
 __device__ __forceinline__ void teno_betas(const T* v, T& b0, T& b1, T& b2) {
     const T t0 = add_rn(fma(T(-2), v[1], v[0]), v[2]), r0 = fma(T(3), v[2], fma(T(-4), v[1], v[0]));
@@ -288,72 +254,32 @@ __device__ __forceinline__ void teno_betas(const T* v, T& b0, T& b1, T& b2) {
     b2 = fma(c13, mul_rn(t2, t2), mul_rn(T(0.25), mul_rn(r2, r2)));
 }
 
-template <typename T> struct Teno;
-
 // The smooth-stencil shortcuts below are taken per warp, when every active
 // lane's stencils pass: a uniform branch, with no divergent paths to
 // reconverge.  A lane whose stencils are smooth but whose warp is not takes
 // the cut-off path, which gives it the same bits.
 __device__ __forceinline__ bool warp_all(bool p) { return __all_sync(__activemask(), p); }
 
-// d0 p0 + d1 p1 + d2 p2 with its roundings fixed (one product, two fused
-// multiply-adds), so a weight set given as constants and the same set chosen
-// at run time round alike.
-__device__ __forceinline__ double teno_sum64(double d0, double d1, double d2, double p0, double p1, double p2) {
-    return fma(d2, p2, fma(d1, p1, d0 * p0));
-}
-
-// A smooth sub-stencil triple keeps all three sub-stencils, which the FP64
-// cut-off finds only after its division: with tau <= 4 e_min (e_k = b_k +
-// 1e-40) every g_k = 1 + tau/e_k lies in [1, 5] up to a few ulps, so G_k >=
-// 1 > lim = 1e-5 sum G <= 0.47 and the mask is 7.  b_max <= 1e30 keeps the
-// products e0 e1 e2 and the shared reciprocal of two of them finite and
-// normal, so the cut-off path raises no non-finite flag either; NaN or
-// infinite indicators fail the test.  The weights for mask 7 are then the
-// cut-off path's to the bit.
-__device__ __forceinline__ bool teno_smooth64(const double (&b)[3], double tau) {
-    const double em = fmin(b[0], fmin(b[1], b[2])) + 1e-40;
-    return tau <= 4.0 * em && fmax(b[0], fmax(b[1], b[2])) <= 1e30;
-}
-
 // FP64 keeps the reference's gamma_k = (1 + tau5/(b_k+eps))^6 and tests
 // gamma_k < CT * sum(gamma) (the reference divides; the comparison is the same
-// up to rounding at the threshold).
-template <> struct Teno<double> {
-    static __device__ __forceinline__ int keep_mask(double b0, double b1, double b2, unsigned& flags) {
-        const double tau = fabs(b0 - b2);
-        // tau/e_k for the three sub-stencils from one reciprocal of the
-        // product e0 e1 e2 (>= 1e-120, no underflow in FP64)
-        const double e0 = b0 + 1e-40, e1 = b1 + 1e-40, e2 = b2 + 1e-40;
-        const double e12 = e1 * e2;
-        const double ti = tau / (e0 * e12);
-        const double g0 = 1.0 + ti * e12;
-        const double g1 = 1.0 + ti * (e0 * e2);
-        const double g2 = 1.0 + ti * (e0 * e1);
-        const double q0 = g0 * g0 * g0, q1 = g1 * g1 * g1, q2 = g2 * g2 * g2;
-        const double G0 = q0 * q0, G1 = q1 * q1, G2 = q2 * q2;
-        const double lim = 1e-5 * (G0 + G1 + G2);
-        if (!finite_(lim)) flags |= FLAG_NONFINITE;
-        return int(!(G0 < lim)) | (int(!(G1 < lim)) << 1) | (int(!(G2 < lim)) << 2);
-    }
-    static __device__ __forceinline__ double core(const double* v, unsigned& flags, unsigned& cut) {
-        double p0, p1, p2, b0, b1, b2;
-        teno_polys<double>(v, p0, p1, p2);
-        teno_betas<double>(v, b0, b1, b2);
-        const double bb[3] = {b0, b1, b2};
-        if (warp_all(teno_smooth64(bb, fabs(b0 - b2))))
-            return teno_sum64(0.1, 0.6, 0.3, p0, p1, p2) * (1.0 / 6.0);  // mask 7
-        const int m = keep_mask(b0, b1, b2, flags);
-        cut += 3 - __popc(m);
-        if (m == 0) { flags |= FLAG_TENO_CUTOFF; return 0.0; }
-        // 1 / (6 * sum of the kept linear weights), by kept set (selects, no
-        // indexed local array)
-        const double inv6act = m == 7 ? 1.0 / 6.0 : m == 6 ? 1.0 / 5.4 : m == 5 ? 1.0 / 2.4 : m == 4 ? 1.0 / 1.8
-                             : m == 3 ? 1.0 / 4.2 : m == 2 ? 1.0 / 3.6 : 1.0 / 0.6;
-        const double d0 = (m & 1) ? 0.1 : 0.0, d1 = (m & 2) ? 0.6 : 0.0, d2 = (m & 4) ? 0.3 : 0.0;
-        return teno_sum64(d0, d1, d2, p0, p1, p2) * inv6act;
-    }
-};
+// up to rounding at the threshold).  The decision alone: bit k set = sub-stencil
+// k kept.
+__device__ __forceinline__ int teno_keep64(double b0, double b1, double b2, unsigned& flags) {
+    const double tau = fabs(b0 - b2);
+    // tau/e_k for the three sub-stencils from one reciprocal of the
+    // product e0 e1 e2 (>= 1e-120, no underflow in FP64)
+    const double e0 = b0 + 1e-40, e1 = b1 + 1e-40, e2 = b2 + 1e-40;
+    const double e12 = e1 * e2;
+    const double ti = tau / (e0 * e12);
+    const double g0 = 1.0 + ti * e12;
+    const double g1 = 1.0 + ti * (e0 * e2);
+    const double g2 = 1.0 + ti * (e0 * e1);
+    const double q0 = g0 * g0 * g0, q1 = g1 * g1 * g1, q2 = g2 * g2 * g2;
+    const double G0 = q0 * q0, G1 = q1 * q1, G2 = q2 * q2;
+    const double lim = 1e-5 * (G0 + G1 + G2);
+    if (!finite_(lim)) flags |= FLAG_NONFINITE;
+    return int(!(G0 < lim)) | (int(!(G1 < lim)) << 1) | (int(!(G2 < lim)) << 2);
+}
 
 // FP32 cut-off, for two independent sub-stencil triples at once (the two
 // lanes).  gamma_k = g_k^6 with g_k = 1 + tau/e_k leaves single-precision
@@ -404,30 +330,6 @@ __device__ __forceinline__ bool teno_smooth2(const float2 (&B)[3]) {
     return fabsf(0.25f * d02.x) <= em.x && fabsf(0.25f * d02.y) <= em.y;
 }
 
-template <> struct Teno<float> {
-    static __device__ __forceinline__ int keep_mask(float b0, float b1, float b2, unsigned& flags) {
-        float2 k[3];
-        float2 bad = f2(0.f);
-        teno_keep32x2(f2(b0), f2(b1), f2(b2), k, bad);
-        flag_bad(bad, flags);
-        return int(k[0].x != 0.f) | (int(k[1].x != 0.f) << 1) | (int(k[2].x != 0.f) << 2);
-    }
-    static __device__ __forceinline__ float core(const float* v, unsigned& flags, unsigned& cut) {
-        float p0, p1, p2, b0, b1, b2;
-        teno_polys<float>(v, p0, p1, p2);
-        teno_betas<float>(v, b0, b1, b2);
-        const float2 bb[3] = {f2(b0), f2(b1), f2(b2)};
-        if (warp_all(teno_smooth2(bb)))  // mask 7 (teno_smooth2 on both lanes of the broadcast)
-            return __fdividef(fmaf(0.3f, p2, fmaf(0.6f, p1, 0.1f * p0)), 6.f * ((0.1f + 0.6f) + 0.3f));
-        const int m = keep_mask(b0, b1, b2, flags);
-        cut += 3 - __popc(m);
-        const float d0 = (m & 1) ? 0.1f : 0.f, d1 = (m & 2) ? 0.6f : 0.f, d2 = (m & 4) ? 0.3f : 0.f;
-        const float act = (d0 + d1) + d2;
-        if (!(act > 0.f)) { flags |= FLAG_TENO_CUTOFF; return 0.f; }
-        return __fdividef(fmaf(d2, p2, fmaf(d1, p1, d0 * p0)), 6.f * act);
-    }
-};
-
 // ---------------------------------------------------------------------------
 // FP64 WENO5 / TENO5 on a face's six points (WENO7: eight) in differences.  With the
 // characteristic first differences W_i = c_{i+1} - c_i (i = 0..4) and second
@@ -469,7 +371,7 @@ __device__ __forceinline__ void indicators64(const double (&W)[5], double eps, d
     er[2] = fma(r2, r2, b[1]);
 }
 
-// WENO5-JS: the folding of weno5_core on both sides, one division for the
+// WENO5-JS (SF_WENO5.cpp:42-62): weno3_core's folding on both sides, one division for the
 // two: with x/a and y/b needed, r = 1/(a b) gives x (b r) and y (a r): in that
 // order only a b has to stay in range (x b is larger by a difference), which it
 // does for differences up to 1e19; the denominators are at least 2.6e-21
@@ -564,9 +466,12 @@ __device__ __forceinline__ void weno7_pair64(const double (&W)[7], double& dl, d
 
 // The smooth-stencil test on the indicators e_k = 4 b_k + eps of one side:
 // tau <= 4 e_min and e_max < 1e30, taken on the high words (order and factor
-// 4 of positive doubles to 2^-20), which keeps it off the FP64 pipe.  The
-// proof at teno_smooth64 leaves far more room than 2^-20.  Unsigned: a NaN of
-// either sign is above 1e30.
+// 4 of positive doubles to 2^-20), which keeps it off the FP64 pipe.  A triple
+// that passes keeps all three sub-stencils, which the cut-off finds only after
+// its division: every g_k = 1 + tau/e_k lies in [1, 5] up to that 2^-20, so G_k >=
+// 1 > lim = 1e-5 sum G <= 0.47; and e_max keeps the products e0 e1 e2 and the
+// shared reciprocal of two of them finite and normal, so the cut-off path would
+// raise no flag either.  Unsigned: a NaN of either sign is above 1e30.
 __device__ __forceinline__ bool teno_smooth_hi(const double (&e)[3], double tau) {
     const unsigned h0 = (unsigned)__double2hiint(e[0]), h1 = (unsigned)__double2hiint(e[1]),
                    h2 = (unsigned)__double2hiint(e[2]);
@@ -617,14 +522,6 @@ __device__ __forceinline__ void teno5_pair64(const double (&W)[5], double& dl, d
             else dl = x;
         }
     }
-}
-
-template <int SCHEME, typename T>
-__device__ __forceinline__ T recon_core(const T* v, unsigned& flags, unsigned& cut) {
-    if constexpr (SCHEME == WENO5) return weno5_core<T>(v, flags);
-    else if constexpr (SCHEME == TENO5) return Teno<T>::core(v, flags, cut);
-    else if constexpr (SCHEME == WENO3) return weno3_core<T>(v, flags);
-    else return weno7_core<T>(v, flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -912,58 +809,36 @@ __device__ __forceinline__ void face_flux64(const double (&st)[SchemeInfo<SCHEME
     if (top >= 0x7ff00000) flags |= FLAG_NONFINITE;
 }
 
-// `lam` = dt / h along AX, used by the Lax-Wendroff flux only.
-template <int AX, int SCHEME, int FLUX, typename T>
-__device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>::NST][5], T gamma, T F[5],
-                                          unsigned& flags, unsigned& cut, T lam = T(0)) {
-    if constexpr (sizeof(T) == sizeof(double) && SCHEME != WENO3) {
+// FP64 face flux.  `lam` = dt / h along AX, used by the Lax-Wendroff flux only.
+// WENO3 works on the projected points.
+template <int AX, int SCHEME, int FLUX>
+__device__ __forceinline__ void face_flux(const double (&st)[SchemeInfo<SCHEME>::NST][5], double gamma, double F[5],
+                                          unsigned& flags, unsigned& cut, double lam) {
+    if constexpr (SCHEME != WENO3) {
         face_flux64<AX, SCHEME, FLUX>(st, gamma, F, flags, cut, lam);
-        return;
-    }
-    constexpr int NST = SchemeInfo<SCHEME>::NST;
-    constexpr int W = SchemeInfo<SCHEME>::W;
-    constexpr int CL = NST / 2 - 1;
-    constexpr bool DEV = sizeof(T) < sizeof(double);
-    double qbar64[5];
+    } else {
+        double qbar[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) qbar64[v] = 0.5 * (st[CL][v] + st[CL + 1][v]);
-    T qbar[5];
+        for (int v = 0; v < 5; ++v) qbar[v] = 0.5 * (st[1][v] + st[2][v]);
+        Eigen<double> e;
+        if (!eigen_at<AX, double>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
+        double ch[4][5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) qbar[v] = T(qbar64[v]);
-    Eigen<T> e;
-    if (!eigen_at<AX, T>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
-    T ch[NST][5];
+        for (int s = 0; s < 4; ++s) to_characteristic<AX, double>(e, st[s], ch[s]);
+        double wl[5], wr[5], ql[5], qr[5];
 #pragma unroll
-    for (int s = 0; s < NST; ++s) {
-        T d[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) d[v] = DEV ? T(st[s][v] - qbar64[v]) : T(st[s][v]);
-        to_characteristic<AX, T>(e, d, ch[s]);
-    }
-    T wl[5], wr[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        T sl[W], sr[W];
-#pragma unroll
-        for (int s = 0; s < W; ++s) {
-            sl[s] = ch[s][v];
-            sr[s] = ch[NST - 1 - s][v];
+        for (int v = 0; v < 5; ++v) {
+            const double sl[4] = {ch[0][v], ch[1][v], ch[2][v], ch[3][v]}, sr[4] = {ch[3][v], ch[2][v], ch[1][v], ch[0][v]};
+            wl[v] = weno3_core<double>(sl, flags);
+            wr[v] = weno3_core<double>(sr, flags);
         }
-        wl[v] = recon_core<SCHEME, T>(sl, flags, cut);
-        wr[v] = recon_core<SCHEME, T>(sr, flags, cut);
-    }
-    T dl[5], dr[5], ql[5], qr[5];
-    from_characteristic<AX, T>(e, wl, dl);
-    from_characteristic<AX, T>(e, wr, dr);
+        from_characteristic<AX, double>(e, wl, ql);
+        from_characteristic<AX, double>(e, wr, qr);
+        flux_of<AX, FLUX, double>(ql, qr, gamma, lam, F, flags);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        ql[v] = DEV ? T(qbar64[v] + double(dl[v])) : dl[v];
-        qr[v] = DEV ? T(qbar64[v] + double(dr[v])) : dr[v];
+        for (int v = 0; v < 5; ++v)
+            if (!finite_(F[v])) flags |= FLAG_NONFINITE;
     }
-    flux_of<AX, FLUX, T>(ql, qr, gamma, lam, F, flags);
-#pragma unroll
-    for (int v = 0; v < 5; ++v)
-        if (!finite_(F[v])) flags |= FLAG_NONFINITE;
 }
 
 // ---------------------------------------------------------------------------
@@ -1480,50 +1355,41 @@ __device__ __forceinline__ void face_flux_dev32(const float (&d)[SchemeInfo<SCHE
                                                 bool count = true, float scale = 1.f) {
     if constexpr (SCHEME != WENO3) {
         face_flux_dev32x2<AX, SCHEME, FLUX>(d, ref, gamma, F, flags, cut, count, scale);
-        return;
-    }
-    const float (&qref)[5] = ref.q;
-    constexpr int NST = SchemeInfo<SCHEME>::NST;
-    constexpr int W = SchemeInfo<SCHEME>::W;
-    constexpr int CL = NST / 2 - 1;
-    float dbar[5], qbar[5];
+    } else {
+        float dbar[5], qbar[5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        dbar[v] = 0.5f * (d[CL][v] + d[CL + 1][v]);
-        qbar[v] = qref[v] + dbar[v];
-    }
-    Eigen<float> e;
-    if (!eigen_at<AX, float>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
-    float ch[NST][5];
-#pragma unroll
-    for (int s = 0; s < NST; ++s) {
-        float dd[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) dd[v] = d[s][v] - dbar[v];
-        to_characteristic<AX, float>(e, dd, ch[s]);
-    }
-    float wl[5], wr[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        float sl[W], sr[W];
-#pragma unroll
-        for (int s = 0; s < W; ++s) {
-            sl[s] = ch[s][v];
-            sr[s] = ch[NST - 1 - s][v];
+        for (int v = 0; v < 5; ++v) {
+            dbar[v] = 0.5f * (d[1][v] + d[2][v]);
+            qbar[v] = ref.q[v] + dbar[v];
         }
-        wl[v] = recon_core<SCHEME, float>(sl, flags, cut);
-        wr[v] = recon_core<SCHEME, float>(sr, flags, cut);
-    }
-    float dl[5], dr[5], xl[5], xr[5];
-    from_characteristic<AX, float>(e, wl, dl);
-    from_characteristic<AX, float>(e, wr, dr);
+        Eigen<float> e;
+        if (!eigen_at<AX, float>(qbar, gamma, e)) flags |= FLAG_PRESSURE;
+        float ch[4][5];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {  // face states as deviations from q_ref
-        xl[v] = dbar[v] + dl[v];
-        xr[v] = dbar[v] + dr[v];
+        for (int s = 0; s < 4; ++s) {
+            float dd[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) dd[v] = d[s][v] - dbar[v];
+            to_characteristic<AX, float>(e, dd, ch[s]);
+        }
+        float wl[5], wr[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            const float sl[4] = {ch[0][v], ch[1][v], ch[2][v], ch[3][v]}, sr[4] = {ch[3][v], ch[2][v], ch[1][v], ch[0][v]};
+            wl[v] = weno3_core<float>(sl, flags);
+            wr[v] = weno3_core<float>(sr, flags);
+        }
+        float dl[5], dr[5], xl[5], xr[5];
+        from_characteristic<AX, float>(e, wl, dl);
+        from_characteristic<AX, float>(e, wr, dr);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {  // face states as deviations from q_ref
+            xl[v] = dbar[v] + dl[v];
+            xr[v] = dbar[v] + dr[v];
+        }
+        if constexpr (FLUX == RUSANOV) rusanov_dev<AX>(ref, xl, xr, gamma, F, flags, scale);
+        else roe_dev<AX>(ref, xl, xr, gamma, F, flags, scale);
     }
-    if constexpr (FLUX == RUSANOV) rusanov_dev<AX>(ref, xl, xr, gamma, F, flags, scale);
-    else roe_dev<AX>(ref, xl, xr, gamma, F, flags, scale);
 }
 
 }  // namespace sfg

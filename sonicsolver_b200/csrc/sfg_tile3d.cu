@@ -103,8 +103,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
 #pragma unroll
                 for (int v = 0; v < 5; ++v) st[s][v] = ring[(v * R + slot) * COL + t];
             }
-            face_flux<2, SCHEME, FLUX, double>(st, g.gamma, Fz, flags, cut,
-                                               FLUX == LAXW ? sv.clock->dt / g.h[2] : 0.0);
+            face_flux<2, SCHEME, FLUX>(st, g.gamma, Fz, flags, cut, FLUX == LAXW ? sv.clock->dt / g.h[2] : 0.0);
         }
     };
 
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
                     for (int s = 0; s < NST; ++s)
 #pragma unroll
                         for (int v = 0; v < 5; ++v) sd[s][v] = st[s][v];
-                    face_flux<0, SCHEME, FLUX, double>(sd, g.gamma, Ft, flags, cut, lamx);
+                    face_flux<0, SCHEME, FLUX>(sd, g.gamma, Ft, flags, cut, lamx);
 #pragma unroll
                     for (int v = 0; v < 5; ++v) fx[v * NFX + f] = Ft[v] * T(g.area[0]);
                 }
@@ -189,7 +188,7 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
                     for (int s = 0; s < NST; ++s)
 #pragma unroll
                         for (int v = 0; v < 5; ++v) sd[s][v] = st[s][v];
-                    face_flux<1, SCHEME, FLUX, double>(sd, g.gamma, Ft, flags, cut, lamy);
+                    face_flux<1, SCHEME, FLUX>(sd, g.gamma, Ft, flags, cut, lamy);
 #pragma unroll
                     for (int v = 0; v < 5; ++v) fy[v * NFY + kf] = Ft[v] * T(g.area[1]);
                 }

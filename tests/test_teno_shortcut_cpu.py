@@ -10,7 +10,7 @@ every triple the test passes keeps all three sub-stencils:
   s = tau t, keep iff x_k^6 >= 1e-5 sum x_j^6, eps = FLT_MIN.  The kernel's
   reciprocal is the SFU approximation; here it is the correctly rounded
   one, perturbed by +-2 ulp to cover the approximation's error.
-* FP64 (Teno<double>::keep_mask, teno5_pair64): g_k = 1 + tau e_i e_j /
+* FP64 (teno_keep64, teno5_pair64): g_k = 1 + tau e_i e_j /
   (e0 e1 e2), keep iff not G_k < 1e-5 sum G, eps = 1e-40.
 
 NaN and infinite indicators must fail the test (they take the cut-off path
