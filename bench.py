@@ -38,17 +38,19 @@ sys.path.insert(0, ROOT)
 #   first axis of 2-D/3-D: read q_s, write R                         -> 80
 #   last axis (stage update): read q_s, R, q0, write q_out (+K RK4)   -> 160
 STATE_BYTES = 40
-# algorithmic FLOPs per face (reconstruction + flux), counted from the kernel
-# source: projection 12/pt, WENO5 core ~58 + 1 div, TENO5 core ~70 + 3 div
-# (the full cut-off; a smooth stencil skips it and does fewer),
-# back-projection 24, Rusanov ~60 + 2 div + 2 sqrt, eigen ~30 + rsqrt.
+# FLOPs of a TENO5 + Rusanov face (FMA = 2; a division or root 1), counted from
+# the kernel source with every stencil smooth (the cut-off path does more).  FP64,
+# in differences: face mean and basis 44, five differences 25 and their
+# projection 105, five fields x 50, back-projection 48, flux 72.  FP32, on points:
+# mean and basis 51, six points 30 and their projection 126, five fields x 75,
+# back-projection 50, flux 131.
 # DRAM bytes (read + write) of one stage-1 launch of the fused 2-D tile kernel
 # on the 1024^2 vortex (variant 1: 32 x 15 tiles, variant 2: 22 x 22), from
 # one ncu --set full capture per kernel of the same command line with --quick.
 PROFILED_DRAM_BYTES = {("tile2d", 1, 1024, "fp32flux"): 42.300e6 + 7.356e6,
                        ("tile2d", 2, 1024, "fp32flux"): 42.036e6 + 4.637e6,
                        ("tile2d", 2, 1024, "fp64"): 42.113e6 + 5.318e6}
-FLOPS_PER_FACE = {"weno5": 6 * 12 + 10 * 59 + 24 + 64 + 34, "teno5": 6 * 12 + 10 * 73 + 24 + 64 + 34}
+FLOPS_PER_FACE = {"fp64": 44 + 25 + 105 + 5 * 50 + 48 + 72, "fp32": 51 + 30 + 126 + 5 * 75 + 50 + 131}
 
 
 def parse():
@@ -264,8 +266,10 @@ def run_ours(args, rank, world):
                       "l2": "inputs larger than L2 (4 x 42 MB state arrays touched per stage)"},
            "clocks": clk.summary(), "gpu_launches": None}
     dim = case.dim
-    launches_per_step = 2 + 3 * (1 if (dim == 2 and s.variant > 0) else dim) + 1  # dt, finalize, stages, commit
-    out["gpu_launches"] = launches_per_step * (K + 0)
+    # a run opens with dt and finalize; a step is its stages, the last of which
+    # ends it (tiles) or is followed by a commit (axis sweeps)
+    tiles = dim == 2 and s.variant > 0
+    out["gpu_launches"] = 2 + K * (3 if tiles else 3 * dim + 1)
     if args.quick:
         s.close()
         return out
@@ -300,7 +304,8 @@ def run_ours(args, rank, world):
     out["e2e"] = {"value": round(whole_job_rate(cells * E, e2e_ms, world) / 1e6, 2), "unit": "Mcell-steps/s",
                   "h2d_bytes_per_step": int(host.nbytes), "d2h_bytes_per_step": int(host.nbytes),
                   "steps": E, "path": "sfg_upload(pinned) + sfg_step + sfg_download per step"}
-    out["gpu_launches"] += E * (launches_per_step + 2)
+    # per step: the transposes in and out, dt, finalize, the stages, commit
+    out["gpu_launches"] += E * (2 + 2 + 3 * (1 if tiles else dim) + 1)
     s.close()
     if s2 is not None:
         # the other precision's e2e on the same path (rank 0): the FP64 e2e
@@ -391,7 +396,8 @@ def rank0_comparisons(args, out, s, case, prec, stream, K, W):
     achieved = bytes_node * nodes / (ms_axes[dom] * 1e-3) / 1e9
     fp_peak = capi.fma_peak_tflops(fp64=(prec == capi.PREC_FP64), seconds=0.5)
     faces = nodes * (dim if fused else 1)  # faces evaluated by one launch
-    fl = FLOPS_PER_FACE["teno5"] * faces / (ms_axes[dom] * 1e-3) / 1e12
+    flops = FLOPS_PER_FACE["fp32" if prec else "fp64"]
+    fl = flops * faces / (ms_axes[dom] * 1e-3) / 1e12
     traffic = PROFILED_DRAM_BYTES.get(("tile2d", s.variant, args.size, args.precision)) if fused else None
     ms_step = out["ms_per_step"]
     step_gbs = 320 * cells / (ms_step * 1e-3) / 1e9   # SSPRK3, FP64 state: 80 + 120 + 120 B per cell-step
@@ -413,7 +419,7 @@ def rank0_comparisons(args, out, s, case, prec, stream, K, W):
                        "issue_roof": {"unit": "TFLOP/s", "achieved": round(fl, 2), "fma_peak": round(fp_peak, 2),
                                       "frac": round(fl / fp_peak, 4) if fp_peak else None,
                                       "arith": "fp32" if prec else "fp64",
-                                      "flops_per_face": FLOPS_PER_FACE["teno5"],
+                                      "flops_per_face": flops,
                                       "peak_source": "measured (sfg_measure_fma_peak: dependent-FMA loop, "
                                                      "this GPU, this run)"},
                        "note": "bound = the binding roof: arithmetic issue (issue_roof), not HBM; achieved / "

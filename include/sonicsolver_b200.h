@@ -173,7 +173,8 @@ typedef struct {
     int64_t steps;            /* steps taken                                 */
     double time;              /* physical time reached                       */
     double last_dt;           /* last step size                              */
-    double device_ms;         /* device time of the advance (CUDA events)     */
+    double device_ms;         /* device time of the advance (CUDA events), a    */
+                              /* run's own graph capture left out              */
     uint32_t status_bits;     /* SFG_FLAG_* seen                             */
     uint64_t teno_cut;        /* TENO5 sub-stencils cut (when counted)        */
     uint64_t teno_cores;      /* TENO5 cores evaluated (when counted)         */
@@ -384,13 +385,16 @@ int sfg_server_drain(sfg_server s, double timeout_s);
 double sfg_server_now(sfg_server s);
 
 /* Kernel variant of the stage operator: 0 = one sweep launch per axis
- * (any dimension), 1 = fused tile kernel (2-D: 32 x 15 tiles, 1-D: 511-node
- * tiles, 3-D: 16 x 15 columns marching up 32-plane chunks), 2 = fused 2-D
- * tile kernel with 22 x 22 tiles; for 1-D grids variant 2 runs sfg_advance
+ * (any dimension), 1 = fused tile kernel, its tile by the grid's size (2-D: 32 x
+ * 15, smaller ones for grids that leave SMs without, 32 x 23 for large ones;
+ * 1-D: 511 or 255 nodes; 3-D: 16 x 15 columns marching up chunks of 2 to 32
+ * planes), 2 = the same with 22 x 22 tiles where variant 1 would take 32 x 15 or
+ * 32 x 23 (2-D; small grids run the same launch in both; curved grids take 22 x
+ * 22 or 16 x 7 tiles in either); for 1-D grids variant 2 runs sfg_advance
  * in one thread-block cluster that steps the whole run on device (FP64, up to
  * 3968 nodes, forward Euler 7936, no boundary laws, not Lax-Wendroff; other 1-D
- * grids and single stages use the 1-D tiles).  sfg_create picks 2 for 1-D, 1 for 2-D and 0
- * for 3-D grids; results agree across variants to round-off (FP32-flux: every
+ * grids and single stages use the 1-D tiles).  sfg_create picks 2 for 1-D, 1 for
+ * 2-D and 0 for 3-D grids; results agree across variants to round-off (FP32-flux: every
  * face takes the stage's one reference state; the sweeps scale face fluxes
  * by the area in FP64, the tiles in FP32), and the tile variants give the
  * same bits as a batch. */

@@ -3,9 +3,11 @@
 Picks the stage-operator kernel variant by timing the candidates on the
 device, per (GPU model, dimension, size class, recipe, precision):
 
-  * single grids: variant 0 (one sweep launch per axis), 1 (32 x 15 tiles,
-    511-node 1-D tiles, or 3-D 16 x 15 columns marching in z), 2 (22 x 22
-    tiles, 2-D only), each timed with
+  * single grids: variant 0 (one sweep launch per axis), 1 (tiles whose shape
+    follows the grid's size: 2-D, 1-D, or 3-D columns marching in z), 2 (2-D
+    only: 22 x 22 where variant 1 takes 32 x 15 or 32 x 23 tiles; on small grids
+    the launch of variant 1, which then wins or loses by noise and nothing
+    else), each timed with
     sfg_time_sweeps (CUDA events on the solver's stream, stage 0 repeated);
     a 1-D tile win selects 1-D variant 2, which runs the same tiles for
     single stages and adds the whole-run cluster kernel to sfg_advance;
@@ -15,8 +17,8 @@ device, per (GPU model, dimension, size class, recipe, precision):
 Results are cached in a JSON table (default ``~/.cache/sonicsolver_b200/
 tuning.json``, or $SFG_TUNING_FILE) so the search runs once per shape class.
 Every variant computes the same result (FP64: identical to round-off; FP32:
-the per-tile reference changes the rounding), so tuning never changes the
-numerics beyond that.
+the sweeps scale face fluxes by the area in FP64, the tiles in FP32), so tuning
+never changes the numerics beyond that.
 """
 from __future__ import annotations
 

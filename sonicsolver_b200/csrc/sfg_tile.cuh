@@ -9,7 +9,8 @@
 //   2. evaluates every face of the tile once from shared memory into
 //      shared-memory flux arrays.  The face list is warp aligned per axis, so
 //      no warp mixes the x and y template paths, and sized to whole rounds of
-//      256 threads (32 x 15 and 22 x 22 tiles: 4 rounds; 1-D 511 nodes: 2);
+//      256 threads (16 x 7 tiles: 1 round, 32 x 7: 2, 32 x 15 and 22 x 22: 4,
+//      32 x 23: 6; 1-D 255 nodes: 1, 511: 2);
 //   3. forms div = dFx (+ dFy) per node and finishes it: stage combination
 //      with state validation, or R = Jac * div.
 // Faces on a tile edge are evaluated by both neighbouring tiles from the same
@@ -35,7 +36,7 @@ namespace sfg {
 
 constexpr int TILE_THREADS = 256;
 constexpr int TILE1D = 511;        // 1-D tile: 512 faces = 2 rounds of 256
-constexpr int TILE1D_SHORT = 255;  // 1-D tile of one round (a batch's drained tail)
+constexpr int TILE1D_SHORT = 255;  // 1-D tile of one round (few blocks: a small grid, a batch's drained tail)
 
 template <int SCHEME, int TX, int TY>
 struct TileShape {
