@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(128, SCHEME == WENO7 && sizeof(T) == sizeof(do
             for (int s = 0; s < NST; ++s)
 #pragma unroll
                 for (int v = 0; v < 5; ++v) d[s][v] = float(st[s][v] - qref[v]);
-            face_flux_dev32<0, SCHEME, FLUX>(d, ref, float(g.gamma), Ft, flags, cut, sv.counters != nullptr);
+            face_flux_dev32<0, SCHEME, FLUX>(d, ref, float(g.gamma), Ft, flags, cut, sv.counters != nullptr, 1.f,
+                                             [&](int k, int v) { return d[NST / 2 - 1 + k][v]; });
         } else {
             face_flux<0, SCHEME, FLUX>(st, g.gamma, Ft, flags, cut, FLUX == LAXW ? sv.clock->dt / g.h[0] : 0.0);
         }
@@ -140,7 +141,8 @@ __device__ __forceinline__ void sweep_yz_f32_segment(const GridView& g, const St
     double Fp[5];
     for (int f = s0; f <= s1; ++f) {
         float Ft[5];
-        face_flux_dev32<AX, SCHEME, FLUX>(d, ref, gamma, Ft, flags, cut, sv.counters != nullptr);
+        face_flux_dev32<AX, SCHEME, FLUX>(d, ref, gamma, Ft, flags, cut, sv.counters != nullptr, 1.f,
+                                          [&](int k, int v) { return d[NST / 2 - 1 + k][v]; });
         if (SCHEME == TENO5) cores += 10;
         double F[5];
 #pragma unroll

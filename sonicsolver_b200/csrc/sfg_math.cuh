@@ -1258,11 +1258,19 @@ __device__ __forceinline__ void rusanov_dev2(const Ref32& r, const float2 d[5], 
     }
 }
 
+// A load of its own, not the register an earlier one left.
+__device__ __forceinline__ float again(const float* p) { return *const_cast<const volatile float*>(p); }
+
 // face_flux_dev32 with the left / right work paired in float2 (WENO5, TENO5, WENO7).
-template <int AX, int SCHEME, int FLUX>
+// near(0, v) and near(1, v): d of the points beside the face once more.  The
+// tiles read them from shared memory again where the states are formed: kept from
+// the start they are ten registers through the whole face, which spilled at 64
+// registers a thread (us a step: WENO5 1500 x 1400 400 -> 386, WENO7 + Roe 160 x 120
+// x 100 1805 -> 1530).
+template <int AX, int SCHEME, int FLUX, typename Near>
 __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
                                                   float gamma, float F[5], unsigned& flags, unsigned& cut, bool count,
-                                                  float scale) {
+                                                  float scale, Near near) {
     constexpr int CL = SchemeInfo<SCHEME>::NST / 2 - 1;  // the face lies between points CL and CL + 1
     float dbar[5], qbar[5];
 #pragma unroll
@@ -1323,7 +1331,7 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
     from_characteristic2<AX>(e, w, dq);
 #pragma unroll
     for (int v = 0; v < 5; ++v)  // (left, right) deviations from q_ref
-        x2[v] = add2(SCHEME == TENO5 ? f2(dbar[v]) : f2(d[CL][v], d[CL + 1][v]), dq[v]);
+        x2[v] = add2(SCHEME == TENO5 ? f2(dbar[v]) : f2(near(0, v), near(1, v)), dq[v]);
     if constexpr (FLUX == RUSANOV) {
         rusanov_dev2<AX, SCHEME == WENO7>(ref, x2, gamma, F, flags, scale);
     } else {
@@ -1348,13 +1356,14 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
 // `count`: the launch's TENO5 cut-off accounting is on (sfg_set_counting);
 // `cut` then receives the cut sub-stencils of the face.  `scale` multiplies
 // the flux (a face area): folded into the flux's closing factor 1/2, which
-// is exact, so F * scale rounds as one multiply after the flux would.
-template <int AX, int SCHEME, int FLUX>
+// is exact, so F * scale rounds as one multiply after the flux would.  `near`: see
+// face_flux_dev32x2.
+template <int AX, int SCHEME, int FLUX, typename Near>
 __device__ __forceinline__ void face_flux_dev32(const float (&d)[SchemeInfo<SCHEME>::NST][5], const Ref32& ref,
-                                                float gamma, float F[5], unsigned& flags, unsigned& cut,
-                                                bool count = true, float scale = 1.f) {
+                                                float gamma, float F[5], unsigned& flags, unsigned& cut, bool count,
+                                                float scale, Near near) {
     if constexpr (SCHEME != WENO3) {
-        face_flux_dev32x2<AX, SCHEME, FLUX>(d, ref, gamma, F, flags, cut, count, scale);
+        face_flux_dev32x2<AX, SCHEME, FLUX>(d, ref, gamma, F, flags, cut, count, scale, near);
     } else {
         float dbar[5], qbar[5];
 #pragma unroll

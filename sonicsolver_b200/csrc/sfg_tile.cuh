@@ -214,8 +214,8 @@ __device__ __forceinline__ void tile2d_f32_body(const GridView& g, const StageVi
             for (int s = 0; s < NST; ++s)
 #pragma unroll
                 for (int v = 0; v < 5; ++v) st[s][v] = base[v * SX * SY + s];
-            face_flux_dev32<0, SCHEME, FLUX>(st, ref, gamma, Ft, flags, cut, sv.counters != nullptr,
-                                             float(g.area[0]));
+            face_flux_dev32<0, SCHEME, FLUX>(st, ref, gamma, Ft, flags, cut, sv.counters != nullptr, float(g.area[0]),
+                                             [&](int k, int v) { return again(base + v * SX * SY + H - 1 + k); });
 #pragma unroll
             for (int v = 0; v < 5; ++v) fx[v * NFX + f] = Ft[v];
         } else {
@@ -227,8 +227,8 @@ __device__ __forceinline__ void tile2d_f32_body(const GridView& g, const StageVi
             for (int s = 0; s < NST; ++s)
 #pragma unroll
                 for (int v = 0; v < 5; ++v) st[s][v] = base[v * SX * SY + s * SX];
-            face_flux_dev32<1, SCHEME, FLUX>(st, ref, gamma, Ft, flags, cut, sv.counters != nullptr,
-                                             float(g.area[1]));
+            face_flux_dev32<1, SCHEME, FLUX>(st, ref, gamma, Ft, flags, cut, sv.counters != nullptr, float(g.area[1]),
+                                             [&](int k, int v) { return again(base + v * SX * SY + (H - 1 + k) * SX); });
 #pragma unroll
             for (int v = 0; v < 5; ++v) fy[v * NFY + k] = Ft[v];
         }
@@ -289,8 +289,8 @@ __device__ __forceinline__ void tile1d_body(const GridView& g, const StageView& 
 #pragma unroll
             for (int v = 0; v < 5; ++v) st[s][v] = sq[v * SX + f + s];
         if constexpr (F32) {
-            face_flux_dev32<0, SCHEME, FLUX>(st, ref, T(g.gamma), Ft, flags, cut, sv.counters != nullptr,
-                                             T(g.area[0]));
+            face_flux_dev32<0, SCHEME, FLUX>(st, ref, T(g.gamma), Ft, flags, cut, sv.counters != nullptr, T(g.area[0]),
+                                             [&](int k, int v) { return again(sq + v * SX + f + NST / 2 - 1 + k); });
 #pragma unroll
             for (int v = 0; v < 5; ++v) fx[v * NF + f] = Ft[v];
         } else {

@@ -94,7 +94,9 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
 #pragma unroll
                 for (int v = 0; v < 5; ++v) d[s][v] = ring[(v * R + slot) * COL + t];
             }
-            face_flux_dev32<2, SCHEME, FLUX>(d, ref, float(g.gamma), Fz, flags, cut, sv.counters != nullptr);
+            const int below = ((p % R) + R) % R, above = (((p + 1) % R) + R) % R;
+            face_flux_dev32<2, SCHEME, FLUX>(d, ref, float(g.gamma), Fz, flags, cut, sv.counters != nullptr, 1.f,
+                                             [&](int s, int v) { return again(ring + (v * R + (s ? above : below)) * COL + t); });
         } else {
             double st[NST][5];
 #pragma unroll
@@ -155,7 +157,8 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
                 if constexpr (F32) {
                     // the area rides in the flux's exact factor 1/2
                     face_flux_dev32<0, SCHEME, FLUX>(st, ref, float(g.gamma), Ft, flags, cut, sv.counters != nullptr,
-                                                     float(g.area[0]));
+                                                     float(g.area[0]),
+                                                     [&](int s, int v) { return again(base + v * SX * SY + H - 1 + s); });
 #pragma unroll
                     for (int v = 0; v < 5; ++v) fx[v * NFX + f] = Ft[v];
                 } else {
@@ -179,7 +182,8 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == sizeof(float) ? T3_
                 if constexpr (F32) {
                     // the area rides in the flux's exact factor 1/2
                     face_flux_dev32<1, SCHEME, FLUX>(st, ref, float(g.gamma), Ft, flags, cut, sv.counters != nullptr,
-                                                     float(g.area[1]));
+                                                     float(g.area[1]),
+                                                     [&](int s, int v) { return again(base + v * SX * SY + (H - 1 + s) * SX); });
 #pragma unroll
                     for (int v = 0; v < 5; ++v) fy[v * NFY + kf] = Ft[v];
                 } else {
