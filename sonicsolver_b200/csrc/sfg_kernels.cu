@@ -316,17 +316,6 @@ __global__ void commit_kernel(Clock* c, const unsigned* flags, double* dt_log, l
     if (open_next) clock_open_step(c, *flags);
 }
 
-// End of a forward Euler step: the stage's output becomes the state, unless
-// the step did not run (the output is then an older one).  It reads the clock
-// before it commits the step itself (MODE_STEP), so the stage has no tail.
-__global__ void __launch_bounds__(256) euler_copy_kernel(StageView sv, double2* q, long long n2) {
-    if (sv.require_active && !sv.clock->active) return;
-    const double2* out = reinterpret_cast<const double2*>(sv.qout);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += (long long)gridDim.x * blockDim.x)
-        q[i] = out[i];
-    if (sv.mode & MODE_STEP) step_tail(sv);
-}
-
 __global__ void set_dt_kernel(Clock* c, double dt) {
     c->dt = dt;
     c->active = 1;
@@ -526,14 +515,6 @@ cudaError_t launch_finalize_dt(Clock* c, const unsigned* flags, cudaStream_t st)
 cudaError_t launch_commit(Clock* c, const unsigned* flags, double* dt_log, long long dt_cap, int cfl_next,
                           int open_next, cudaStream_t st) {
     commit_kernel<<<1, 1, 0, st>>>(c, flags, dt_log, dt_cap, cfl_next, open_next);
-    return cudaGetLastError();
-}
-
-// `sv`: the Euler stage; `q`: the state, 5 x vs doubles (vs a multiple of 32).
-cudaError_t launch_euler_copy(const StageView& sv, double* q, long long vs, cudaStream_t st) {
-    const long long n2 = 5 * vs / 2;
-    const unsigned blocks = (unsigned)std::min<long long>((n2 + 255) / 256, 148LL * 8);
-    euler_copy_kernel<<<blocks, 256, 0, st>>>(sv, reinterpret_cast<double2*>(q), n2);
     return cudaGetLastError();
 }
 
