@@ -694,8 +694,8 @@ __device__ __forceinline__ void curv_face_dev32x2(const float (&d)[SchemeInfo<SC
     for (int v = 0; v < 5; ++v) {
         const float2 H = f2(M[v], -M[v]);
         if constexpr (SCHEME == TENO5) w[v] = teno5_delta2(E[0][v], E[1][v], H, bad, count, kept);
-        else if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, f2(0.f), bad);
-        else w[v] = weno5_delta2(E[0][v], E[1][v], H, f2(0.f), bad);
+        else if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, bad);
+        else w[v] = weno5_delta2(E[0][v], E[1][v], H, bad);
     }
     flag_bad(bad, flags);
     if constexpr (SCHEME == TENO5) {

@@ -919,12 +919,12 @@ __device__ __forceinline__ float2 teno5_core2(float2 v0, float2 v1, float2 v2, f
 //   T1 = E1 - E0 = (t1, t4),  T2 = E2 - E1 = (t2, t3),  T2' = its swap
 //   4 b_k = 13/3 t^2 + r^2:  (T1, T1 + 2 E1), (T2, E1 + E2), (T2', T2' - 2 E2)
 //   p_k - mid = T1/3 - T2/2, -T2/6, -T2'/6
-// Kept with N2 = -T2.  Deltas from the midpoint of c2 and c3 make the face states
-// d-bar + R (deltas); with H added they are deltas from the side's nearer point,
-// and the states d2 + R (..), d3 + R (..).  The Cartesian faces take the second
-// form: there the rounding of d-bar, the same in both states, made residuals
-// 1.05 to 1.2 x less accurate than the form on points was (0.86 to 1.01 x now, at 2 % of a
-// Taylor-Green step).
+// Kept with N2 = -T2.  The face states are d-bar + R (deltas).  The Cartesian faces
+// form them as d2 + (m / 2 + R (..)) and d3 + (-m / 2 + R (..)), m = d3 - d2: with
+// d-bar itself its rounding, the same in both states, made residuals 1.05 to 1.2 x
+// less accurate than the form on points was.  The half difference goes in as it
+// is and not through R L, which is the identity only to 1e-7 and would act on the
+// jump of the two states as a (signed) dissipation.
 struct Diff2 {
     float2 T1, N2, N2s;  // (t1, t4), -(t2, t3), -(t3, t2)
     float2 e[3];         // 4 b_k
@@ -944,11 +944,11 @@ __device__ __forceinline__ Diff2 indicators2(float2 E0, float2 E1, float2 H) {
     return d;
 }
 
-// WENO5-JS deltas of both sides, `base` added: H or 0.  Its indicators are b_k
+// WENO5-JS deltas of both sides.  Its indicators are b_k
 // themselves (r / 2 from H and h at no cost), not 4 b_k: the denominator, 10 b^4,
 // then leaves FP32 range at density jumps of 1.5e4 (6 (4 b)^4 of the form on
 // points did at 1.2e4, 10 (4 b)^4 at 8e3).
-__device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, float2 base, float2& bad) {
+__device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, float2& bad) {
     const float2 T1 = sub2(E1, E0), N2 = fma2(f2(-2.f), H, E1), h = mul2(f2(0.5f), N2), hs = swap2(h);
     const float2 r0 = fma2(f2(0.5f), T1, E1), r1 = fma2(f2(0.5f), E1, H), r2 = fma2(f2(2.f), H, hs);
     const float2 c = f2(13.f / 12.f);
@@ -959,7 +959,7 @@ __device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, f
     const float2 den = fma2(f2(3.f), fma2(f2(2.f), wb, wc), wa);
     const float2 num = fma2(wa, fma2(f2(1.f / 3.f), T1, h), fma2(wb, N2, mul2(wc, hs)));
     bad = watch2(bad, den);  // den >= 10 eps^4 > 0 unless an input was not finite
-    return fma2(num, rcp2(den), base);
+    return mul2(num, rcp2(den));
 }
 
 // WENO7-JS deltas of both sides: weno7_pair64's form with E_k = (W_k, -W_{6-k}),
@@ -968,7 +968,7 @@ __device__ __forceinline__ float2 weno5_delta2(float2 E0, float2 E1, float2 H, f
 // leave FP32 range.  Against the scalar form, us a step: 700 x 520 267 -> 123,
 // 128 x 100 x 90 3314 -> 862 (with the 3-D tile's chunks), curved 500 x 400
 // 248 -> 88 (with the curved faces' other changes).
-__device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, float2 H, float2 base, float2& bad) {
+__device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, float2 H, float2& bad) {
     const float2 E3 = add2(H, H);
     const float2 T1 = sub2(E1, E0), T2 = sub2(E2, E1), T3 = sub2(E3, E2), T4 = swap2(T3), T5 = swap2(T2);
     const float2 G[4] = {sub2(T2, T1), sub2(T3, T2), sub2(T4, T3), sub2(T5, T4)};
@@ -991,7 +991,7 @@ __device__ __forceinline__ float2 weno7_delta2(float2 E0, float2 E1, float2 E2, 
         num = fma2(w, P[k], num);
     }
     bad = watch2(bad, den);
-    return fma2(num, rcp2(mul2(f2(12.f), den)), base);
+    return mul2(num, rcp2(mul2(f2(12.f), den)));
 }
 
 // TENO5 deltas of both sides.  With `count` (a launch-uniform switch: the
@@ -1319,8 +1319,8 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
             const float2 H = f2(M[v], -M[v]);
-            if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, H, bad);
-            else w[v] = weno5_delta2(E[0][v], E[1][v], H, H, bad);
+            if constexpr (SCHEME == WENO7) w[v] = weno7_delta2(E[0][v], E[1][v], E[2][v], H, bad);
+            else w[v] = weno5_delta2(E[0][v], E[1][v], H, bad);
         }
     }
     flag_bad(bad, flags);
@@ -1330,8 +1330,14 @@ __device__ __forceinline__ void face_flux_dev32x2(const float (&d)[SchemeInfo<SC
     float2 dq[5], x2[5];
     from_characteristic2<AX>(e, w, dq);
 #pragma unroll
-    for (int v = 0; v < 5; ++v)  // (left, right) deviations from q_ref
-        x2[v] = add2(SCHEME == TENO5 ? f2(dbar[v]) : f2(near(0, v), near(1, v)), dq[v]);
+    for (int v = 0; v < 5; ++v) {  // (left, right) deviations from q_ref
+        if constexpr (SCHEME == TENO5) {
+            x2[v] = add2(f2(dbar[v]), dq[v]);
+        } else {
+            const float a = near(0, v), b = near(1, v), h = fmaf(0.5f, b, -0.5f * a);
+            x2[v] = add2(f2(a, b), add2(f2(h, -h), dq[v]));
+        }
+    }
     if constexpr (FLUX == RUSANOV) {
         rusanov_dev2<AX, SCHEME == WENO7>(ref, x2, gamma, F, flags, scale);
     } else {
